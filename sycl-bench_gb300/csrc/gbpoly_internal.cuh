@@ -187,12 +187,14 @@ inline bool symmetric_operand(const GemmF32Args& a) {
   return !a.dual && a.A == a.B && a.lda == a.ldb && a.M == a.N && a.op_a != a.op_b;
 }
 gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a);
-// Workspace of the K split the FP32 kernel uses for grids too small to fill a
-// device of `sm_count` SMs (0 when it does not split).
+// What gbpoly_workspace_query reports for an FP32 contraction: the partial
+// products of a K split in global memory.  The kernel keeps them in the
+// shared memory of its clusters and needs none of it; the figure stays for
+// callers that reserve by it.
 size_t fp32_split_k_bytes(int sm_count, int64_t M, int64_t N, int64_t K);
-// The K split count gbpoly_gemm_f32 uses for an FP32 contraction of this
-// shape on operands the TMA kernel can read (1: no split).
-int fp32_split_k_count(int sm_count, int64_t M, int64_t N, int64_t K);
+// The K split count gbpoly_gemm_f32 uses for a non-symmetric FP32 contraction
+// of this shape (1: no split).
+gbpoly_status fp32_split_k_count(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, int& splits);
 // Tensor-core forms (split_gemm.cu): tf32, bf16x3, tf32x3, bf16x6, fp16x3,
 // fp8.  The split term panels live in the context workspace.
 gbpoly_status launch_gemm_tensor(gbpoly_ctx* ctx, gbpoly_precision prec, const GemmF32Args& a);
@@ -348,11 +350,22 @@ __device__ __forceinline__ uint32_t cluster_count_x() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // Address of the same shared-memory object in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t cluster_map(const void* p, uint32_t rank) {
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
   return r;
+}
+// 16 bytes of a cluster CTA's shared memory (an address of cluster_map).
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
 }
 // Arrive on an mbarrier given by its cluster address (this CTA's or a
 // peer's), with the default (CTA-scope) release: the arrival only counts,

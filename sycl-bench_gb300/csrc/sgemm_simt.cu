@@ -4,96 +4,169 @@
 //
 // The reference launches one work-item per C element that walks the whole k
 // range through global memory.  Here one CTA owns a 128x128 tile of C:
-//   * one producer warp streams BK=32 slices of the A and B panels into a
-//     ring of shared-memory stages with 2-D TMA (cp.async.bulk.tensor),
-//     each stage guarded by a full/empty mbarrier pair;
+//   * a producer warpgroup streams BK=32 slices of the A and B panels into a
+//     ring of shared-memory stages, each guarded by a full/empty mbarrier
+//     pair.  Both tiles lie [k][row or column] there, whatever the operand's
+//     layout (Fetch, below);
 //   * eight consumer warps (256 threads) each keep an 8x8 block of C in
-//     registers and run FFMA over 128-bit shared-memory loads;
+//     registers and run packed FFMA over 128-bit shared-memory loads;
 //   * the epilogue applies C = alpha*acc + beta*C with bounds checks.
+// Grids that would not fill the device split K over the CTAs of a cluster.
 // syr2k's two products (A_i.B_j + B_i.A_j) stream four tiles per stage into
 // the same accumulator.  Symmetric updates (syrk, syr2k, X^T.X) compute only
 // the tiles on and below the diagonal; a tile below it also stores its
-// transpose (with its own beta * C term), so the full square is written.  Operands whose base or leading dimension is not
-// 16-byte aligned (TMA's rule) take a simple tiled kernel without TMA.
+// transpose (with its own beta * C term), so the full square is written.
+//
+// Bound: the FP32 pipe, 152 SMs x 128 x 2 x 2070 MHz = 80.5 TFLOP/s; whole
+// tiles (M = 2432, N = 4096, K = 2048; op N/N, N/T, T/N, T/T) run at 63.4,
+// 62.3, 68.3 and 64.4 TFLOP/s, against 55.7, 52.9, 57.2 and 53.7 with scalar
+// FFMA on tiles in their stored layout.  The packed FFMA (two products per
+// instruction) takes its operands from register pairs: with both tiles
+// [k][...] a pair of B values is half a 16-byte load and only A's 8 values
+// per k are duplicated; K-major tiles, whose loads hold 4 k of one row, had
+// to be paired by moves (N/N 54, N/T 36 TFLOP/s), and pairs along k need
+// twice the accumulators (N/N 26).
+#include <algorithm>
+
 #include "gbpoly_internal.cuh"
 #include "tiled_gemm.cuh"
+#include "umma.cuh"
 
 namespace gbpoly {
 namespace {
 
 constexpr int kBM = 128, kBN = 128, kBK = 32;
-constexpr int kConsumers = 256;            // 8 consumer warps
-constexpr int kThreads = kConsumers + 32;  // + 1 producer warp
+constexpr int kProducers = 128;  // warpgroup 0
+constexpr int kConsumers = 256;  // warpgroups 1 and 2: 8 consumer warps
+constexpr int kThreads = kProducers + kConsumers;
+// Registers per thread after the split: 128 x 40 + 256 x 232 = 64,512, what
+// the 384 threads are launched with (168 each).
+constexpr uint32_t kRegsProducer = 40, kRegsConsumer = 232;
 constexpr int kTileBytes = kBM * kBK * 4;  // 16 KB, same for every tile shape used
+constexpr int kMaxSplit = 8;               // CTAs of a cluster (portable cluster size)
+// Costs of a CTA besides its k tiles, in k tiles' time (2.4 us; best_split):
+// a 64 x 64 x 64 call takes 10.4 us for two k tiles; a split one about 2 us more
+constexpr double kFixedTiles = 1.5, kSplitTiles = 0.8;
 
-// Byte offset of float4 chunk `chunk` (0..7) of row `row` in a [rows][32]
-// fp32 tile written by TMA with 128-byte swizzle (chunk index XOR row%8).
-__device__ __forceinline__ uint32_t swz128(int row, int chunk) {
-  return static_cast<uint32_t>(row * 128 + ((chunk ^ (row & 7)) << 4));
+using umma::regs_decrease;
+using umma::regs_increase;
+
+// How a 128-wide, 32-deep operand tile gets into shared memory as
+// [32 k][128 rows or columns]:
+//   Tma   MN-major operand (rows or columns contiguous) with a 16-byte-aligned
+//         base and leading dimension: one 2-D tiled copy;
+//   Rows  the same at any alignment: 4-byte cp.async by the 128 producer threads;
+//   Turn  K-major operand (k contiguous), any alignment: 4-byte cp.async, the
+//         tile turned on the way.  A warp copies 4 rows x 8 k per instruction
+//         (four 32-byte sectors) and the 16-byte chunks of k row k are permuted
+//         by k % 8, so its 32 words fall in 32 banks.
+// The words cost 128 instructions per tile over four warps, against 4096
+// cycles of products per tile pair.
+enum class Fetch { Tma, Rows, Turn };
+
+// One operand as stored: X[r * ld + c], R x Cn elements.
+struct Operand {
+  const float* X;
+  int64_t ld;
+  int R, Cn;
+};
+
+__device__ __forceinline__ void cp_async_word(uint32_t dst, const float* src, bool ok) {
+  const uint32_t n = ok ? 4u : 0u;  // 0 source bytes: the word is filled with zero
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 
-// Operand tile layouts in shared memory:
-//  K-major (k innermost, e.g. A as stored, or B^T as stored):
-//     [128 rows][32 k], 128-byte swizzled.
-//  MN-major (row/col innermost, e.g. B as stored for C = A.B):
-//     [32 k][128], unswizzled 512-byte rows.
-//
-// Register fragment: v[i][kk] for the 8 rows (or columns) this thread owns
-// and the 4 k values of one k-step.
-//  MN-major: owned indices 4t..4t+3 and 64+4t..64+4t+3 (vector loads along the row).
-//  K-major:  owned indices t+16i (rows t, t+16, ...), so that the 8 lanes of a
-//            quarter warp hit 8 distinct swizzle phases (conflict-free).
-template <bool KMAJ>
-__device__ __forceinline__ int owned_index(int t, int i) {
-  if constexpr(KMAJ)
-    return t + 16 * i;
-  else
-    return (i < 4) ? (4 * t + i) : (64 + 4 * t + (i - 4));
-}
-
-template <bool KMAJ>
-__device__ __forceinline__ void load_frag(const char* tile, int t, int kstep, float (&v)[8][4]) {
-  if constexpr(KMAJ) {
+// One producer thread's words of the tile whose first row or column is x0, zero beyond the matrix.
+template <Fetch F>
+__device__ __forceinline__ void fetch_words(uint32_t dst, const Operand& o, int x0, int k0) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if constexpr(F == Fetch::Turn) {
+    const int kl = lane & 7, rl = lane >> 3;
+    const float* p = o.X + int64_t(x0 + 4 * warp + rl) * o.ld + k0 + kl;
+#pragma unroll 2
+    for(int i = 0; i < 8; ++i) {  // chunks of four rows warp, warp + 4, ...
+      const int c = warp + 4 * i;
+      const bool row = x0 + 4 * c + rl < o.R;
+      const uint32_t d = dst + kl * 512 + ((c ^ kl) << 4) + 4 * rl;
 #pragma unroll
-    for(int i = 0; i < 8; ++i) {
-      const int row = t + 16 * i;
-      const float4 x = *reinterpret_cast<const float4*>(tile + swz128(row, kstep));
-      v[i][0] = x.x;
-      v[i][1] = x.y;
-      v[i][2] = x.z;
-      v[i][3] = x.w;
+      for(int g = 0; g < 4; ++g) {
+        const bool ok = row && k0 + 8 * g + kl < o.Cn;
+        cp_async_word(d + 8 * 512 * g, ok ? p + 8 * g : o.X, ok);
+      }
+      p += 16 * o.ld;
     }
   } else {
+#pragma unroll 2
+    for(int i = 0; i < 8; ++i) {  // k rows warp, warp + 4, ...
+      const int k = warp + 4 * i;
+      const bool kin = k0 + k < o.R;
+      const float* p = o.X + int64_t(k0 + (kin ? k : 0)) * o.ld + x0;
 #pragma unroll
-    for(int kk = 0; kk < 4; ++kk) {
-      const char* rowp = tile + (kstep * 4 + kk) * 512;
-      const float4 lo = *reinterpret_cast<const float4*>(rowp + 16 * t);
-      const float4 hi = *reinterpret_cast<const float4*>(rowp + 256 + 16 * t);
-      v[0][kk] = lo.x;
-      v[1][kk] = lo.y;
-      v[2][kk] = lo.z;
-      v[3][kk] = lo.w;
-      v[4][kk] = hi.x;
-      v[5][kk] = hi.y;
-      v[6][kk] = hi.z;
-      v[7][kk] = hi.w;
+      for(int e = 0; e < 4; ++e) {
+        const int c = lane + 32 * e;
+        const bool ok = kin && x0 + c < o.Cn;
+        cp_async_word(dst + 512 * k + 4 * c, ok ? p + c : o.X, ok);
+      }
     }
   }
 }
 
-template <bool A_KMAJ, bool B_KMAJ>
-__device__ __forceinline__ void mma_tile(const char* ta, const char* tb, int tm, int tn, float (&acc)[8][8]) {
-#pragma unroll 1
-  for(int ks = 0; ks < kBK / 4; ++ks) {
-    float a[8][4], b[8][4];
-    load_frag<A_KMAJ>(ta, tm, ks, a);
-    load_frag<B_KMAJ>(tb, tn, ks, b);
+// A thread's 8 x 8 block: rows  4 li + 16 (i / 4) + i % 4 of its warp's 32,
+// columns 4 lj + 32 (j / 4) + j % 4 of its warp's 64 (lanes 4 x 8, warps 4 x
+// 2): per k two 16-byte loads of A (4 distinct in a warp) and two of B (8
+// distinct: one shared-memory wavefront each).
+__device__ __forceinline__ int owned_row(int li, int i) { return 4 * li + 16 * (i >> 2) + (i & 3); }
+__device__ __forceinline__ int owned_col(int lj, int j) { return 4 * lj + 32 * (j >> 2) + (j & 3); }
+
+// Two FP32 fused multiply-adds in one instruction (each rounded as fmaf).
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void fma2(uint64_t& d, uint64_t a, uint64_t b) {
+  asm volatile("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));  // volatile: keeps the order below
+}
+
+// One k tile.  oa, ob: the thread's first 16 bytes of a k row (unpermuted).
+// acc[i][h] holds columns 2h and 2h + 1 of row i; a pair of B values is used
+// by all eight rows before the next, so that it is read once.
+template <bool TURN_A, bool TURN_B>
+__device__ __forceinline__ void mma_tile(const char* ta, const char* tb, uint32_t oa, uint32_t ob,
+    uint64_t (&acc)[8][4]) {
 #pragma unroll
-    for(int kk = 0; kk < 4; ++kk)
+  for(int k8 = 0; k8 < kBK; k8 += 8) {
 #pragma unroll
-      for(int i = 0; i < 8; ++i)
+    for(int kk = 0; kk < 8; kk += 4) {
+      float a[4][8], b[4][8];
 #pragma unroll
-        for(int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i][kk], b[j][kk], acc[i][j]);
+      for(int e = 0; e < 4; ++e) {
+        const int x = kk + e;  // k % 8
+        // a turned tile's chunk c lies at c ^ x; the thread's chunks are its first one plus 4 (A) or 8 (B)
+        const char* ra = ta + (TURN_A ? oa ^ (x << 4) : oa) + x * 512;
+        const char* rb = tb + (TURN_B ? ob ^ (x << 4) : ob) + x * 512;
+        const float4 a0 = *reinterpret_cast<const float4*>(ra);
+        const float4 a1 = *reinterpret_cast<const float4*>(ra + (TURN_A && (x & 4) ? -64 : 64));
+        const float4 b0 = *reinterpret_cast<const float4*>(rb);
+        const float4 b1 = *reinterpret_cast<const float4*>(rb + 128);
+        a[e][0] = a0.x, a[e][1] = a0.y, a[e][2] = a0.z, a[e][3] = a0.w;
+        a[e][4] = a1.x, a[e][5] = a1.y, a[e][6] = a1.z, a[e][7] = a1.w;
+        b[e][0] = b0.x, b[e][1] = b0.y, b[e][2] = b0.z, b[e][3] = b0.w;
+        b[e][4] = b1.x, b[e][5] = b1.y, b[e][6] = b1.z, b[e][7] = b1.w;
+      }
+#pragma unroll
+      for(int e = 0; e < 4; ++e)
+#pragma unroll
+        for(int h = 0; h < 4; ++h) {
+          const uint64_t bp = pack2(b[e][2 * h], b[e][2 * h + 1]);
+#pragma unroll
+          for(int i = 0; i < 8; ++i) fma2(acc[i][h], pack2(a[e][i], a[e][i]), bp);
+        }
+    }
+    ta += 8 * 512, tb += 8 * 512;
   }
 }
 
@@ -119,14 +192,24 @@ __device__ __forceinline__ void lower_coords(int t, int& tile_m, int& tile_n) {
   tile_n = t - tm * (tm + 1) / 2;
 }
 
-// A_KMAJ: op(A) rows are contiguous in k (op_a == N).  B_KMAJ: op(B) columns
-// are contiguous in k (op_b == T).  DUAL: syr2k, tiles A_i, B_j, B_i, A_j.
-template <bool A_KMAJ, bool B_KMAJ, bool DUAL, int STAGES>
-__global__ void __launch_bounds__(kThreads, 1) sgemm_tma_kernel(const __grid_constant__ CUtensorMap tmA,
-    const __grid_constant__ CUtensorMap tmB, int M, int N, int K, float alpha, float beta, float* __restrict__ C,
-    int64_t ldc, int lower, int kt_per_split, float* __restrict__ part, int* err) {
+// FA, FB: how op(A)'s and op(B)'s tiles are fetched.  DUAL: syr2k (both
+// operands K-major), tiles A_i, B_j, B_i, A_j.
+//
+// K split: the gridDim.y CTAs of a cluster take consecutive K ranges of one
+// tile.  Each writes its sums to its own shared memory (the drained ring);
+// CTA r then adds the cluster's sums of its share of the rows, in rank order
+// (every run gives the same bits), and writes them.  No global scratch, no
+// second launch: a launch stays independent of every other one, on any
+// stream or in any graph.
+template <Fetch FA, Fetch FB, bool DUAL, int STAGES>
+__global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constant__ CUtensorMap tmA,
+    const __grid_constant__ CUtensorMap tmB, const Operand oa, const Operand ob, int M, int N, int K,
+    float alpha, float beta, float* __restrict__ C, int64_t ldc, int lower, int kt_per_split, int* err) {
   constexpr int kTilesPerStage = DUAL ? 4 : 2;
   constexpr int kStageBytes = kTilesPerStage * kTileBytes;
+  constexpr int kTmaTiles = DUAL ? 0 : int(FA == Fetch::Tma) + int(FB == Fetch::Tma);
+  constexpr bool kWords = kTmaTiles < 2;
+  static_assert(!DUAL || (FA == Fetch::Turn && FB == Fetch::Turn), "syr2k: K-major operands");
   extern __shared__ __align__(1024) char smem_raw[];
   // 1024-byte aligned (128-byte swizzle atoms); offset arithmetic keeps the pointer in the shared window
   char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -143,73 +226,78 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_tma_kernel(const __grid_con
     tile_coords(blockIdx.x, tiles_m, tiles_n, tile_m, tile_n);
   const int m0 = tile_m * kBM, n0 = tile_n * kBN;
   const bool mirror = lower && tile_m != tile_n;
-  // split K (gridDim.y > 1): this CTA covers k tiles [kt0, kt0 + nkt) and
-  // writes alpha * its partial product to its slice of `part` (M x N, ld N);
-  // a reduction kernel adds the slices and beta * C
+  const int splits = int(gridDim.y), split = int(blockIdx.y);  // the cluster is 1 x splits: split == rank
   const int ktiles = (K + kBK - 1) / kBK;
-  const int kt0 = int(blockIdx.y) * kt_per_split;
+  const int kt0 = split * kt_per_split;
   const int nkt = max(0, min(ktiles, kt0 + kt_per_split) - kt0);
-  if(gridDim.y > 1) {
-    C = part + int64_t(blockIdx.y) * int64_t(M) * N;
-    ldc = N;
-    beta = 0.f;
-  }
 
   if(tid == 0) {
 #pragma unroll
     for(int s = 0; s < STAGES; ++s) {
-      mbar_init(&full[s], 1);
+      mbar_init(&full[s], (kTmaTiles > 0 ? 1 : 0) + (kWords ? kProducers : 0));
       mbar_init(&empty[s], kConsumers / 32);
     }
     fence_mbar_init();
   }
   __syncthreads();
 
-  if(warp == kConsumers / 32) {
+  if(warp < kProducers / 32) {
     // ------------------------------------------------------------ producer
-    if(lane == 0) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
+    regs_decrease<kRegsProducer>();
+    if(kWords || tid == 0) {
+      if constexpr(FA == Fetch::Tma) if(tid == 0) tma_prefetch_desc(&tmA);
+      if constexpr(FB == Fetch::Tma) if(tid == 0) tma_prefetch_desc(&tmB);
       int issued = 0;
       for(int i = 0; i < nkt; ++i) {
         const int s = i % STAGES;
         if(i >= STAGES && !mbar_wait(&empty[s], ((i / STAGES) - 1) & 1, err, kDevErrEmptyWait)) break;
         char* st = smem + s * kStageBytes;
-        mbar_arrive_expect_tx(&full[s], kStageBytes);
         const int k0 = (kt0 + i) * kBK;
-        if constexpr(DUAL) {
-          tma_load_2d(st + 0 * kTileBytes, &tmA, &full[s], k0, m0);  // A rows of the C tile
-          tma_load_2d(st + 1 * kTileBytes, &tmB, &full[s], k0, n0);  // B rows of the C tile columns
-          tma_load_2d(st + 2 * kTileBytes, &tmB, &full[s], k0, m0);
-          tma_load_2d(st + 3 * kTileBytes, &tmA, &full[s], k0, n0);
-        } else {
-          if constexpr(A_KMAJ)
-            tma_load_2d(st, &tmA, &full[s], k0, m0);
-          else
-            tma_load_2d(st, &tmA, &full[s], m0, k0);
-          if constexpr(B_KMAJ)
-            tma_load_2d(st + kTileBytes, &tmB, &full[s], k0, n0);
-          else
-            tma_load_2d(st + kTileBytes, &tmB, &full[s], n0, k0);
+        if constexpr(kTmaTiles > 0) {
+          if(tid == 0) {
+            mbar_arrive_expect_tx(&full[s], kTmaTiles * kTileBytes);
+            if constexpr(FA == Fetch::Tma) tma_load_2d(st, &tmA, &full[s], m0, k0);
+            if constexpr(FB == Fetch::Tma) tma_load_2d(st + kTileBytes, &tmB, &full[s], n0, k0);
+          }
+        }
+        if constexpr(kWords) {
+          const uint32_t d = smem_u32(st);
+          if constexpr(FA != Fetch::Tma) fetch_words<FA>(d, oa, m0, k0);
+          if constexpr(FB != Fetch::Tma) fetch_words<FB>(d + kTileBytes, ob, n0, k0);
+          if constexpr(DUAL) {
+            fetch_words<FB>(d + 2 * kTileBytes, ob, m0, k0);
+            fetch_words<FA>(d + 3 * kTileBytes, oa, n0, k0);
+          }
+          // one arrival per producer thread, when its copies so far have landed
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(smem_u32(&full[s])) : "memory");
         }
         ++issued;
       }
       // Drain: do not leave the CTA while copies into its shared memory are in flight.
-      for(int kt = max(0, issued - STAGES); kt < issued; ++kt) {
-        if(!mbar_wait(&full[kt % STAGES], (kt / STAGES) & 1, err, kDevErrDrainWait)) break;
-      }
+      if constexpr(kWords) asm volatile("cp.async.wait_all;" ::: "memory");
+      if(kTmaTiles > 0 && tid == 0)
+        for(int kt = max(0, issued - STAGES); kt < issued; ++kt)
+          if(!mbar_wait(&full[kt % STAGES], (kt / STAGES) & 1, err, kDevErrDrainWait)) break;
+    }
+    __syncwarp();
+    if(splits > 1) {
+      cluster_sync();  // the cluster's sums are written
+      cluster_arrive();
+      cluster_wait();  // and read
     }
     return;
   }
 
   // -------------------------------------------------------------- consumers
-  const int tm = warp * 2 + (lane >> 4);  // 0..15
-  const int tn = lane & 15;               // 0..15
-  float acc[8][8];
+  regs_increase<kRegsConsumer>();
+  const int ctid = tid - kProducers, cwarp = ctid >> 5;
+  const int li = lane >> 3, lj = lane & 7;
+  const int wr = 32 * (cwarp >> 1), wc = 64 * (cwarp & 1);  // the warp's rows and columns of the tile
+  uint64_t acc2[8][4];
 #pragma unroll
-  for(int i = 0; i < 8; ++i)
+  for(auto& row : acc2)
 #pragma unroll
-    for(int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for(auto& v : row) v = 0;
 
   bool ok = true;
   for(int kt = 0; kt < nkt; ++kt) {
@@ -218,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_tma_kernel(const __grid_con
       // epilogue reads it: 512 lines of 128 bytes, two per consumer thread
 #pragma unroll
       for(int e = 0; e < 2; ++e) {
-        const int line = tid + kConsumers * e, r = line >> 2, c = 32 * (line & 3);
+        const int line = ctid + kConsumers * e, r = line >> 2, c = 32 * (line & 3);
         if(m0 + r < M && n0 + c < N) prefetch_l2(C + int64_t(m0 + r) * ldc + n0 + c);
         if(mirror && n0 + r < N && m0 + c < M) prefetch_l2(C + int64_t(n0 + r) * ldc + m0 + c);
       }
@@ -229,193 +317,292 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_tma_kernel(const __grid_con
       break;
     }
     const char* st = smem + s * kStageBytes;
-    if constexpr(DUAL) {
-      mma_tile<true, true>(st + 0 * kTileBytes, st + 1 * kTileBytes, tm, tn, acc);
-      mma_tile<true, true>(st + 2 * kTileBytes, st + 3 * kTileBytes, tm, tn, acc);
-    } else {
-      mma_tile<A_KMAJ, B_KMAJ>(st, st + kTileBytes, tm, tn, acc);
-    }
+    mma_tile<FA == Fetch::Turn, FB == Fetch::Turn>(st, st + kTileBytes, 4 * wr + 16 * li, 4 * wc + 16 * lj, acc2);
+    if constexpr(DUAL)
+      mma_tile<true, true>(st + 2 * kTileBytes, st + 3 * kTileBytes, 4 * wr + 16 * li, 4 * wc + 16 * lj, acc2);
     __syncwarp();
     if(lane == 0) mbar_arrive(&empty[s]);
+  }
+
+  // The thread's block as 16 quads: quad f is row f / 2, columns 4 (f % 2) .. + 3.
+  float4 acc[16];
+#pragma unroll
+  for(int f = 0; f < 16; ++f) {
+    unpack2(acc2[f / 2][2 * (f & 1)], acc[f].x, acc[f].y);
+    unpack2(acc2[f / 2][2 * (f & 1) + 1], acc[f].z, acc[f].w);
+  }
+  const bool read_c = beta != 0.f;
+  const bool vec = (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;  // 16-byte-aligned rows
+  auto row_of = [&](int f) { return m0 + wr + owned_row(li, f >> 1); };
+  auto col_of = [&](int f) { return n0 + wc + owned_col(lj, 4 * (f & 1)); };
+  auto load_c = [&](int f) {
+    const int r = row_of(f), c = col_of(f);
+    const float* p = C + static_cast<int64_t>(r) * ldc + c;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if(!read_c || r >= M) return v;
+    if(vec && c + 3 < N) return *reinterpret_cast<const float4*>(p);
+    if(c < N) v.x = p[0];
+    if(c + 1 < N) v.y = p[1];
+    if(c + 2 < N) v.z = p[2];
+    if(c + 3 < N) v.w = p[3];
+    return v;
+  };
+  auto store_c = [&](int f, float4 s, float4 old) {
+    const int r = row_of(f), c = col_of(f);
+    float* p = C + static_cast<int64_t>(r) * ldc + c;
+    if(r >= M) return;
+    const float4 o = make_float4(fmaf(beta, old.x, alpha * s.x), fmaf(beta, old.y, alpha * s.y),
+        fmaf(beta, old.z, alpha * s.z), fmaf(beta, old.w, alpha * s.w));
+    if(vec && c + 3 < N) {
+      *reinterpret_cast<float4*>(p) = o;
+      return;
+    }
+    if(c < N) p[0] = o.x;
+    if(c + 1 < N) p[1] = o.y;
+    if(c + 2 < N) p[2] = o.z;
+    if(c + 3 < N) p[3] = o.w;
+  };
+  // a mirrored tile's transpose, strictly above the diagonal: C[n][m] from the product element (m, n)
+  auto load_t = [&](int f) {
+    const int r = row_of(f), c = col_of(f);
+    const float* p = C + static_cast<int64_t>(c) * ldc + r;
+    const bool ok = read_c && r < M;
+    return make_float4(ok && c < N ? p[0] : 0.f, ok && c + 1 < N ? p[ldc] : 0.f, ok && c + 2 < N ? p[2 * ldc] : 0.f,
+        ok && c + 3 < N ? p[3 * ldc] : 0.f);
+  };
+  auto store_t = [&](int f, float4 s, float4 old) {
+    const int r = row_of(f), c = col_of(f);
+    float* p = C + static_cast<int64_t>(c) * ldc + r;
+    if(r >= M) return;
+    if(c < N) p[0] = fmaf(beta, old.x, alpha * s.x);
+    if(c + 1 < N) p[ldc] = fmaf(beta, old.y, alpha * s.y);
+    if(c + 2 < N) p[2 * ldc] = fmaf(beta, old.z, alpha * s.z);
+    if(c + 3 < N) p[3 * ldc] = fmaf(beta, old.w, alpha * s.w);
+  };
+
+  if(splits > 1) {
+    // every consumer warp has read its last stage, every copy has landed (each was waited for)
+    asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");
+    float4* mine = reinterpret_cast<float4*>(smem) + ctid;
+#pragma unroll
+    for(int f = 0; f < 16; ++f) mine[f * kConsumers] = acc[f];
+    cluster_sync();
+    // this CTA's quads: f0 .. f1 - 1 (two to eight), all their loads in flight together
+    const int f0 = 16 * split / splits, f1 = 16 * (split + 1) / splits;
+    float4 sum[8];
+#pragma unroll
+    for(int e = 0; e < 8; ++e) sum[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for(int c = 0; c < kMaxSplit; ++c) {
+      if(c >= splits) break;
+      const uint32_t theirs = cluster_map(mine, c) + f0 * kConsumers * 16;
+      float4 v[8];
+#pragma unroll
+      for(int e = 0; e < 8; ++e)
+        if(f0 + e < f1) v[e] = ld_cluster_f4(theirs + e * kConsumers * 16);
+#pragma unroll
+      for(int e = 0; e < 8; ++e)
+        if(f0 + e < f1) sum[e].x += v[e].x, sum[e].y += v[e].y, sum[e].z += v[e].z, sum[e].w += v[e].w;
+    }
+    cluster_arrive();
+#pragma unroll
+    for(int t = 0; t < 2; ++t) {
+      if(!ok || (t == 1 && !mirror)) continue;
+      float4 old[8];
+#pragma unroll
+      for(int e = 0; e < 8; ++e)
+        if(f0 + e < f1) old[e] = t ? load_t(f0 + e) : load_c(f0 + e);
+#pragma unroll
+      for(int e = 0; e < 8; ++e)
+        if(f0 + e < f1) t ? store_t(f0 + e, sum[e], old[e]) : store_c(f0 + e, sum[e], old[e]);
+    }
+    __syncwarp();
+    cluster_wait();  // no CTA leaves (or is left) while its sums are being read
+    return;
   }
   if(!ok) return;
 
   // --------------------------------------------------------------- epilogue
-  // C = alpha * acc + beta * C, four rows (then, below the diagonal of a
-  // symmetric product, four transposed rows) at a time: the 32 C values of a
-  // group are loaded before the group's first store.  A load cannot move above
-  // a store that may alias it, so interleaving them per element would
-  // serialise one memory round trip per element.
-  constexpr bool kVecCols = !B_KMAJ && !DUAL;
-  const bool vec_ok = kVecCols && ((ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(C) & 15) == 0);
-  int rm[8], cn[8];  // owned rows (m) and columns (n)
+  // C = alpha * acc + beta * C, four rows at a time: the C values of a group
+  // are loaded before the group's first store.  A load cannot move above a
+  // store that may alias it, so interleaving them per element would serialise
+  // one memory round trip per element.
 #pragma unroll
-  for(int i = 0; i < 8; ++i) rm[i] = m0 + owned_index<A_KMAJ || DUAL>(tm, i);
+  for(int t = 0; t < 2; ++t) {
+    if(t == 1 && !mirror) break;
 #pragma unroll
-  for(int j = 0; j < 8; ++j) cn[j] = n0 + owned_index<B_KMAJ || DUAL>(tn, j);
-  const bool read_c = beta != 0.f;
+    for(int g = 0; g < 16; g += 8) {
+      float4 old[8];
 #pragma unroll
-  for(int g = 0; g < 8; g += 4) {
-    float cv[4][8];
+      for(int e = 0; e < 8; ++e) old[e] = t ? load_t(g + e) : load_c(g + e);
 #pragma unroll
-    for(int r = 0; r < 4; ++r) {
-      const int i = g + r;
-      const float* crow = C + static_cast<int64_t>(rm[i]) * ldc;
-#pragma unroll
-      for(int h = 0; h < 2; ++h) {
-        if(read_c && vec_ok && rm[i] < M && cn[4 * h] + 3 < N) {
-          const float4 c = *reinterpret_cast<const float4*>(crow + cn[4 * h]);
-          cv[r][4 * h + 0] = c.x, cv[r][4 * h + 1] = c.y, cv[r][4 * h + 2] = c.z, cv[r][4 * h + 3] = c.w;
-        } else {
-#pragma unroll
-          for(int q = 0; q < 4; ++q)
-            cv[r][4 * h + q] = (read_c && rm[i] < M && cn[4 * h + q] < N) ? crow[cn[4 * h + q]] : 0.f;
-        }
-      }
-    }
-#pragma unroll
-    for(int r = 0; r < 4; ++r) {
-      const int i = g + r;
-      if(rm[i] >= M) continue;
-      float* crow = C + static_cast<int64_t>(rm[i]) * ldc;
-#pragma unroll
-      for(int h = 0; h < 2; ++h) {
-        float o[4];
-#pragma unroll
-        for(int q = 0; q < 4; ++q) o[q] = fmaf(beta, cv[r][4 * h + q], alpha * acc[i][4 * h + q]);
-        if(vec_ok && cn[4 * h] + 3 < N) {
-          *reinterpret_cast<float4*>(crow + cn[4 * h]) = make_float4(o[0], o[1], o[2], o[3]);
-        } else {
-#pragma unroll
-          for(int q = 0; q < 4; ++q)
-            if(cn[4 * h + q] < N) crow[cn[4 * h + q]] = o[q];
-        }
-      }
-    }
-  }
-  if(mirror) {  // C[n][m] from the product element (m, n): the tile's transpose, strictly above the diagonal
-#pragma unroll
-    for(int g = 0; g < 8; g += 4) {
-      float mv[4][8];
-#pragma unroll
-      for(int r = 0; r < 4; ++r)
-#pragma unroll
-        for(int i = 0; i < 8; ++i)
-          mv[r][i] = (read_c && cn[g + r] < N && rm[i] < M) ? C[static_cast<int64_t>(cn[g + r]) * ldc + rm[i]] : 0.f;
-#pragma unroll
-      for(int r = 0; r < 4; ++r) {
-        const int j = g + r;
-        if(cn[j] >= N) continue;
-        float* crow = C + static_cast<int64_t>(cn[j]) * ldc;
-#pragma unroll
-        for(int i = 0; i < 8; ++i)
-          if(rm[i] < M) crow[rm[i]] = fmaf(beta, mv[r][i], alpha * acc[i][j]);
-      }
+      for(int e = 0; e < 8; ++e) t ? store_t(g + e, acc[g + e], old[e]) : store_c(g + e, acc[g + e], old[e]);
     }
   }
 }
 
-// C = sum over the splits of part[s] (already scaled by alpha) + beta C, the
-// splits added in index order.
-__global__ void split_k_reduce_kernel(const float* __restrict__ part, int splits, int M, int N, float beta, float* C,
-    int64_t ldc) {
-  const int64_t total = int64_t(M) * N;
-  const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-  for(int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < total; e += stride) {
-    const int64_t m = e / N, n = e - m * N;
-    float s = 0.f;
-    for(int k = 0; k < splits; ++k) s += part[int64_t(k) * total + e];
-    float* c = C + m * ldc + n;
-    *c = beta != 0.f ? fmaf(beta, *c, s) : s;
-  }
-}
+template <Fetch FA, Fetch FB, bool DUAL>
+struct Kernel {
+  static constexpr int kStages = DUAL ? 3 : 4;
+  static constexpr int kSmem = kStages * (DUAL ? 4 : 2) * kTileBytes + 1024 + 2 * kStages * 8;
+  static constexpr auto fn = sgemm_kernel<FA, FB, DUAL, kStages>;
 
-// K split for grids too small to fill the device: about one CTA per SM, at
-// least 4 k tiles (128 of K) per split, at most 8 splits.
-int split_k_count(int sm_count, int64_t tiles, int64_t ktiles) {
-  if(tiles <= 0 || tiles * 2 > sm_count || ktiles < 8) return 1;
-  int64_t s = std::min<int64_t>(std::min<int64_t>(sm_count / tiles, ktiles / 4), 8);
-  if(s <= 1) return 1;
-  const int64_t per = (ktiles + s - 1) / s;
-  return int((ktiles + per - 1) / per);  // every split non-empty
-}
+  // Once per device context: shared-memory opt-in and the register check of
+  // the warp split (setmaxnreg draws on the registers of the launch).
+  static gbpoly_status prepare(gbpoly_ctx* ctx) {
+    static ContextMark prepared;
+    if(prepared.valid(ctx->device)) return GBPOLY_OK;
+    GBPOLY_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    cudaFuncAttributes fa;
+    GBPOLY_CUDA_TRY(cudaFuncGetAttributes(&fa, fn));
+    if(long(fa.numRegs) * kThreads < long(kProducers) * kRegsProducer + long(kConsumers) * kRegsConsumer)
+      return fail(GBPOLY_ERR_UNSUPPORTED, "FP32 kernel built with too few registers for its warp split");
+    prepared.set(ctx->device);
+    return GBPOLY_OK;
+  }
 
-template <bool A_KMAJ, bool B_KMAJ, bool DUAL, int STAGES>
-gbpoly_status launch_tma(gbpoly_ctx* ctx, const GemmF32Args& a, const CUtensorMap& ta, const CUtensorMap& tb,
-    bool lower) {
-  constexpr int kStageBytes = (DUAL ? 4 : 2) * kTileBytes;
-  constexpr int kSmem = STAGES * kStageBytes + 1024 + 2 * STAGES * 8;
-  auto kern = sgemm_tma_kernel<A_KMAJ, B_KMAJ, DUAL, STAGES>;
-  static ContextMark attr_set;  // the attribute is set once per device context
-  if(!attr_set.valid(ctx->device)) {
-    GBPOLY_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-    attr_set.set(ctx->device);
+  struct Launch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    Launch(gbpoly_ctx* ctx, unsigned tiles, unsigned splits) {
+      cfg.gridDim = dim3(tiles, splits);
+      cfg.blockDim = dim3(kThreads);
+      cfg.dynamicSmemBytes = kSmem;
+      cfg.stream = ctx->stream;
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = splits, attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = splits > 1 ? 1 : 0;
+    }
+  };
+};
+
+// Clusters of 1 x s CTAs resident at once on the context's device (one CTA
+// per SM in every variant of the kernel, so one query serves them all).
+gbpoly_status cluster_capacity(gbpoly_ctx* ctx, int (&cap)[kMaxSplit + 1]) {
+  using K = Kernel<Fetch::Tma, Fetch::Tma, false>;
+  static std::atomic<int> known_cap[32][kMaxSplit + 1];
+  static ContextMark known;
+  if(known.valid(ctx->device)) {
+    for(int s = 1; s <= kMaxSplit; ++s) cap[s] = known_cap[ctx->device][s];
+    return GBPOLY_OK;
   }
-  int64_t tiles = ((a.M + kBM - 1) / kBM) * ((a.N + kBN - 1) / kBN);
-  if(lower) {
-    const int64_t t = (a.M + kBM - 1) / kBM;
-    tiles = t * (t + 1) / 2;
+  gbpoly_status st = K::prepare(ctx);
+  if(st != GBPOLY_OK) return st;
+  cap[1] = std::max(1, ctx->sm_count);
+  for(int s = 2; s <= kMaxSplit; ++s) {
+    typename K::Launch l(ctx, unsigned(ctx->sm_count), unsigned(s));
+    int n = 0;
+    GBPOLY_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, K::fn, &l.cfg));
+    cap[s] = n;  // 0: no cluster of this size
   }
-  // the split depends on the full square's tile count, so a symmetric product
-  // splits K exactly like the same product computed in full (same bits)
-  const int64_t ktiles = (a.K + kBK - 1) / kBK;
-  int splits = a.ksplit > 0 ? int(std::min<int64_t>(a.ksplit, std::max<int64_t>(ktiles, 1)))
-                            : split_k_count(ctx->sm_count, ((a.M + kBM - 1) / kBM) * ((a.N + kBN - 1) / kBN), ktiles);
-  const int kt_per_split = int((ktiles + splits - 1) / splits);
-  splits = int((ktiles + kt_per_split - 1) / kt_per_split);  // every split non-empty
-  if(splits < 1) splits = 1;
-  float* part = nullptr;
-  if(splits > 1) {
-    gbpoly_status st = ensure_workspace(ctx, size_t(splits) * size_t(a.M) * size_t(a.N) * sizeof(float));
-    if(st != GBPOLY_OK) return st;
-    part = static_cast<float*>(ctx->ws.ptr);
-  }
-  {
-    ProfileScope prof(ctx, DUAL ? "sgemm_simt_dual" : "sgemm_simt");
-    kern<<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(splits)), kThreads, kSmem, ctx->stream>>>(ta, tb,
-        static_cast<int>(a.M), static_cast<int>(a.N), static_cast<int>(a.K), a.alpha, a.beta, a.C, a.ldc,
-        lower ? 1 : 0, kt_per_split, part, ctx->err_dev);
-    GBPOLY_CUDA_TRY(cudaGetLastError());
-  }
-  if(splits > 1) {
-    ProfileScope prof(ctx, "split_k_reduce");
-    const int64_t total = a.M * a.N;
-    const unsigned blocks = unsigned(std::min<int64_t>((total + 255) / 256, 8ll * ctx->sm_count));
-    split_k_reduce_kernel<<<blocks, 256, 0, ctx->stream>>>(part, splits, int(a.M), int(a.N), a.beta, a.C, a.ldc);
-    GBPOLY_CUDA_TRY(cudaGetLastError());
+  if(ctx->device >= 0 && ctx->device < 32) {
+    for(int s = 1; s <= kMaxSplit; ++s) known_cap[ctx->device][s] = cap[s];
+    known.set(ctx->device);
   }
   return GBPOLY_OK;
 }
 
+// K split of a launch of `tiles` tiles (measured on GB300, all splits 1 to 8 of
+// eighteen shapes: within 4 % of the fastest but for syr2k at 512, 27 against
+// 23 us; gemm 1024 47 us with 2 against 59 with a workspace split and its
+// reduction launch, syr2k 1536 178 with 3 against 299 unsplit, 2048 and up unsplit) of `ktiles` k tiles each: the count
+// whose rounds of clusters take the least time, in units of one k tile's
+// products: each CTA spends its share of the k tiles, a fixed part (launch,
+// first copies, C) and, when split, the exchange of sums.
+int best_split(const int (&cap)[kMaxSplit + 1], int64_t tiles, int64_t ktiles, bool dual) {
+  const double unit = dual ? 2.0 : 1.0;  // syr2k: a k tile is two products
+  int best = 1;
+  double best_t = 0;
+  for(int s = 1; s <= kMaxSplit && s <= std::max<int64_t>(ktiles, 1); ++s) {
+    if(cap[s] <= 0) continue;
+    const int64_t per = (ktiles + s - 1) / s;
+    if(s > 1 && (ktiles + per - 1) / per != s) continue;  // an empty split
+    const double t = double((tiles + cap[s] - 1) / cap[s]) * (unit * double(per) + kFixedTiles + (s > 1 ? kSplitTiles : 0));
+    if(s == 1 || t < 0.97 * best_t) best = s, best_t = t;
+  }
+  return best;
+}
+
+// The K split of an FP32 contraction.  A symmetric product launches the lower
+// triangle of tiles; small ones take the full square's split all the same, so
+// that they give the bits of the same product computed in full (with at most
+// 25 tiles the full square's split is 6 to 8, near the limit of 8 in any case).
+gbpoly_status split_count(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, bool lower, bool dual, int& splits) {
+  int cap[kMaxSplit + 1] = {};
+  gbpoly_status st = cluster_capacity(ctx, cap);
+  if(st != GBPOLY_OK) return st;
+  const int64_t tm = (M + kBM - 1) / kBM, tn = (N + kBN - 1) / kBN;
+  const int64_t tiles = lower && tm * tn > 25 ? tm * (tm + 1) / 2 : tm * tn;
+  splits = best_split(cap, tiles, (K + kBK - 1) / kBK, dual);
+  return GBPOLY_OK;
+}
+
+template <Fetch FA, Fetch FB, bool DUAL>
+gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob) {
+  using Kn = Kernel<FA, FB, DUAL>;
+  // Symmetric product (op(A) == op(B)^T as stored, or syr2k): lower triangle of tiles only.
+  const bool lower = a.M == a.N && (DUAL || symmetric_operand(a));
+  gbpoly_status st = Kn::prepare(ctx);
+  if(st != GBPOLY_OK) return st;
+  const int64_t tm = (a.M + kBM - 1) / kBM, tn = (a.N + kBN - 1) / kBN, ktiles = (a.K + kBK - 1) / kBK;
+  const int64_t tiles = lower ? tm * (tm + 1) / 2 : tm * tn;
+  if(tiles >= (1ll << 31)) return fail(GBPOLY_ERR_UNSUPPORTED, "too many output tiles");
+  int splits = a.ksplit;
+  if(splits <= 0 && (st = split_count(ctx, a.M, a.N, a.K, lower, DUAL, splits)) != GBPOLY_OK) return st;
+  splits = int(std::min<int64_t>(splits, std::max<int64_t>(ktiles, 1)));
+  const int kt_per_split = int((ktiles + splits - 1) / splits);
+  CUtensorMap ta = {}, tb = {};
+  auto map = [&](CUtensorMap* t, const Operand& o) {
+    return make_tmap_2d(ctx, t, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, o.X, o.R, o.Cn, o.ld, kBK, 128,
+        CU_TENSOR_MAP_SWIZZLE_NONE);
+  };
+  if(FA == Fetch::Tma && (st = map(&ta, oa)) != GBPOLY_OK) return st;
+  if(FB == Fetch::Tma && (st = map(&tb, ob)) != GBPOLY_OK) return st;
+  ProfileScope prof(ctx, DUAL ? "sgemm_simt_dual" : "sgemm_simt");
+  typename Kn::Launch l(ctx, unsigned(tiles), unsigned(splits));
+  GBPOLY_CUDA_TRY(cudaLaunchKernelEx(&l.cfg, Kn::fn, ta, tb, oa, ob, int(a.M), int(a.N), int(a.K), a.alpha, a.beta, a.C,
+      a.ldc, lower ? 1 : 0, kt_per_split, ctx->err_dev));
+  return GBPOLY_OK;
+}
+
+template <Fetch FA>
+gbpoly_status launch_left(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob, Fetch fb) {
+  switch(fb) {
+  case Fetch::Tma: return launch_sgemm<FA, Fetch::Tma, false>(ctx, a, oa, ob);
+  case Fetch::Rows: return launch_sgemm<FA, Fetch::Rows, false>(ctx, a, oa, ob);
+  default: return launch_sgemm<FA, Fetch::Turn, false>(ctx, a, oa, ob);
+  }
+}
+
+// A K-major operand is turned on its way; an MN-major one goes by TMA where
+// its base and rows are 16-byte aligned (and it is not empty).
+Fetch fetch_of(const Operand& o, bool k_major) {
+  if(k_major) return Fetch::Turn;
+  return (reinterpret_cast<uintptr_t>(o.X) & 15) == 0 && (o.ld & 3) == 0 && o.R > 0 ? Fetch::Tma : Fetch::Rows;
+}
+
 }  // namespace
 
-// Workspace bytes of the K split of an FP32 contraction, for a device of at
-// most `sm_count` SMs (more SMs never need less).
-int fp32_split_k_count(int sm_count, int64_t M, int64_t N, int64_t K) {
-  return split_k_count(sm_count, ((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN), (K + kBK - 1) / kBK);
+gbpoly_status fp32_split_k_count(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, int& splits) {
+  return split_count(ctx, M, N, K, false, false, splits);
 }
 
 size_t fp32_split_k_bytes(int sm_count, int64_t M, int64_t N, int64_t K) {
-  const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN);
-  const int s = split_k_count(sm_count, tiles, (K + kBK - 1) / kBK);
-  return s > 1 ? size_t(s) * size_t(M) * size_t(N) * sizeof(float) : 0;
+  const int64_t tiles = ((M + kBM - 1) / kBM) * ((N + kBN - 1) / kBN), ktiles = (K + kBK - 1) / kBK;
+  if(tiles <= 0 || tiles * 2 > sm_count || ktiles < 8) return 0;
+  const int64_t s = std::min<int64_t>(std::min<int64_t>(sm_count / tiles, ktiles / 4), 8);
+  if(s <= 1) return 0;
+  const int64_t per = (ktiles + s - 1) / s;
+  return size_t((ktiles + per - 1) / per) * size_t(M) * size_t(N) * sizeof(float);
 }
-
-namespace {
-
-bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
-}  // namespace
 
 gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a) {
   if(a.M == 0 || a.N == 0) return GBPOLY_OK;
   const bool a_kmaj = a.op_a == GBPOLY_OP_N;
   const bool b_kmaj = a.op_b == GBPOLY_OP_T;
-  bool tma_ok = aligned16(a.A) && aligned16(a.B) && (a.lda % 4 == 0) && (a.ldb % 4 == 0) && a.K > 0 &&
-                a.M < (1ll << 31) && a.N < (1ll << 31) && a.K < (1ll << 31);
-  if(a.dual) tma_ok = tma_ok && a_kmaj && b_kmaj && a.A2 == a.B && a.B2 == a.A;
-
-  if(!tma_ok) {
+  if(a.M >= (1ll << 31) - kBM || a.N >= (1ll << 31) - kBN || a.K >= (1ll << 31) - kBK) {
+    // beyond the kernel's 32-bit tile coordinates
     TiledOperand<float> oa = a_kmaj ? TiledOperand<float>{a.A, a.lda, 1} : TiledOperand<float>{a.A, 1, a.lda};
     TiledOperand<float> ob = b_kmaj ? TiledOperand<float>{a.B, a.ldb, 1} : TiledOperand<float>{a.B, 1, a.ldb};
     TiledOperand<float> oa2{a.A2, a.lda2, 1}, ob2{a.B2, a.ldb2, 1};
@@ -423,29 +610,18 @@ gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a) {
         a.M == a.N && (a.dual || symmetric_operand(a)));
   }
 
-  CUtensorMap ta, tb;
-  const auto dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  gbpoly_status st;
-  // op(A) is M x K.  Stored as M x K (K-major) for op N, K x M for op T.
-  if(a_kmaj)
-    st = make_tmap_2d(ctx, &ta, dt, 4, a.A, a.M, a.K, a.lda, kBM, kBK, CU_TENSOR_MAP_SWIZZLE_128B);
-  else
-    st = make_tmap_2d(ctx, &ta, dt, 4, a.A, a.K, a.M, a.lda, kBK, kBM, CU_TENSOR_MAP_SWIZZLE_NONE);
-  if(st != GBPOLY_OK) return st;
+  // op(A) is M x K.  Stored as M x K (K-major) for op N, K x M for op T;
   // op(B) is K x N.  Stored as K x N for op N, N x K (K-major) for op T.
-  if(b_kmaj)
-    st = make_tmap_2d(ctx, &tb, dt, 4, a.B, a.N, a.K, a.ldb, kBN, kBK, CU_TENSOR_MAP_SWIZZLE_128B);
-  else
-    st = make_tmap_2d(ctx, &tb, dt, 4, a.B, a.K, a.N, a.ldb, kBK, kBN, CU_TENSOR_MAP_SWIZZLE_NONE);
-  if(st != GBPOLY_OK) return st;
-
-  // Symmetric product (op(A) == op(B)^T as stored, or syr2k): lower triangle of tiles only.
-  const bool lower = a.M == a.N && (a.dual || symmetric_operand(a));
-  if(a.dual) return launch_tma<true, true, true, 3>(ctx, a, ta, tb, lower);
-  if(a_kmaj && b_kmaj) return launch_tma<true, true, false, 4>(ctx, a, ta, tb, lower);
-  if(a_kmaj && !b_kmaj) return launch_tma<true, false, false, 4>(ctx, a, ta, tb, lower);
-  if(!a_kmaj && b_kmaj) return launch_tma<false, true, false, 4>(ctx, a, ta, tb, lower);
-  return launch_tma<false, false, false, 4>(ctx, a, ta, tb, lower);
+  const int M = int(a.M), N = int(a.N), K = int(a.K);
+  const Operand oa = a_kmaj ? Operand{a.A, a.lda, M, K} : Operand{a.A, a.lda, K, M};
+  const Operand ob = b_kmaj ? Operand{a.B, a.ldb, N, K} : Operand{a.B, a.ldb, K, N};
+  if(a.dual) return launch_sgemm<Fetch::Turn, Fetch::Turn, true>(ctx, a, oa, ob);
+  const Fetch fb = fetch_of(ob, b_kmaj);
+  switch(fetch_of(oa, a_kmaj)) {
+  case Fetch::Tma: return launch_left<Fetch::Tma>(ctx, a, oa, ob, fb);
+  case Fetch::Rows: return launch_left<Fetch::Rows>(ctx, a, oa, ob, fb);
+  default: return launch_left<Fetch::Turn>(ctx, a, oa, ob, fb);
+  }
 }
 
 }  // namespace gbpoly

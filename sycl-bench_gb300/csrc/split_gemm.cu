@@ -1610,7 +1610,7 @@ size_t workspace_bytes(gbpoly_precision prec, int64_t M, int64_t N, int64_t K, b
            align_up(size_t((M + 127) / 128) * kb * 4, 256) + (same ? 0 : align_up(size_t((N + 127) / 128) * kb * 4, 256));
   }
   case GBPOLY_PREC_FP32:
-    // partial products of the K split of small grids, bounded for devices of up to 256 SMs
+    // an upper bound for devices of up to 256 SMs (the kernel uses none of it)
     return fp32_split_k_bytes(256, M, N, K);
   default: return 0;
   }
@@ -2025,14 +2025,8 @@ gbpoly_status gbpoly::grouped_plan_config(gbpoly_ctx* ctx, gbpoly_precision prec
   gbpoly_status st = GBPOLY_OK;
   switch(prec) {
   case GBPOLY_PREC_FP32: {
-    // per-problem launches; the workspace their K splits need is reserved now
-    // so that running the plan (or capturing it) allocates nothing
-    size_t ws = 0;
-    for(auto& d : g->descs) {
-      g->flops += 2 * d.M * d.N * d.K;
-      ws = std::max(ws, fp32_split_k_bytes(ctx->sm_count, d.M, d.N, d.K));
-    }
-    if(ws > 0) st = ensure_workspace(ctx, ws);
+    // per-problem launches, without workspace
+    for(auto& d : g->descs) g->flops += 2 * d.M * d.N * d.K;
     break;
   }
   case GBPOLY_PREC_BF16X3:
