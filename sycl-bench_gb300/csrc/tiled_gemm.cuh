@@ -1,14 +1,18 @@
 // Simple tiled GEMM over general strides, templated on the element type.
 //
-// Used where TMA cannot describe an operand (FP32 operands whose base or
-// leading dimension is not a multiple of 16 bytes) and as the FP64 DGEMM
-// (the FP64 oracle and the double variants of the benchmarks; GB300's FP64
-// rate is low enough that this SIMT tiling is not the limit).
+// The FP64 DGEMM (the FP64 oracle and the double variants of the benchmarks),
+// and FP32 contractions with a dimension beyond 2^31.
 //   op(X)[r][k] = X[r * s_r + k * s_k]
 //   C[m][n] = alpha * (sum_k op(A)[m][k] op(B)[k][n]  [+ op(A2) op(B2)]) + beta * C[m][n]
-// 64x64 tile of C per 256-thread CTA, 4x4 per thread, BK = 16.  beta == 0
+// 16 x 16 of C per 64-thread CTA, BK = 16.  beta == 0
 // does not read C.  `lower` (symmetric products, M == N): only tiles on or
-// below the diagonal compute; a tile below it also stores its transpose.
+// below the diagonal are launched; a tile below it also stores its transpose.
+//
+// Bound: the FP64 pipe, two FMA per cycle and SM (1.26 TFLOP/s), so slow that
+// a small tile's extra loads cost nothing, while the tile count decides how
+// evenly the SMs are loaded: N = 1024 takes 1.81 ms (1.19 TFLOP/s) with 4096
+// tiles of 16 x 16, 2.06 ms with 256 of 64 x 64, 2.10 ms with 1024 of 32 x 32;
+// N = 256 50, 267 and 154 us; N = 2048 13.9, 14.3 and 14.3 ms.
 #pragma once
 #include "gbpoly_internal.cuh"
 
@@ -20,87 +24,79 @@ struct TiledOperand {
   int64_t s_r, s_k;
 };
 
+constexpr int kTiledTile = 16;
+
 template <typename T>
-__global__ void __launch_bounds__(256) tiled_gemm_kernel(int64_t M, int64_t N, int64_t K, T alpha,
-    TiledOperand<T> a, TiledOperand<T> b, bool dual, TiledOperand<T> a2, TiledOperand<T> b2, T beta,
-    T* __restrict__ C, int64_t ldc, bool lower) {
-  __shared__ T As[16][64 + 1];
-  __shared__ T Bs[16][64 + 1];
-  if(lower && blockIdx.x > blockIdx.y) return;  // strictly above the diagonal: the mirror of another tile
+__global__ void __launch_bounds__(64) tiled_gemm_kernel(int64_t M, int64_t N, int64_t K, T alpha, TiledOperand<T> a,
+    TiledOperand<T> b, bool dual, TiledOperand<T> a2, TiledOperand<T> b2, T beta, T* __restrict__ C, int64_t ldc,
+    bool lower, int64_t tiles_n) {
+  constexpr int TILE = kTiledTile, R = TILE / 8, BK = 16;  // R x R outputs per thread (8 x 8 threads)
+  __shared__ T As[BK][TILE + 1];
+  __shared__ T Bs[BK][TILE + 1];
+  int64_t tm = blockIdx.x / tiles_n, tn = blockIdx.x - tm * tiles_n;
+  if(lower) {  // row-major walk of the lower triangle: t = tm (tm + 1) / 2 + tn
+    const int64_t t = blockIdx.x;
+    tm = int64_t((sqrtf(8.f * float(t) + 1.f) - 1.f) * 0.5f);
+    while(tm * (tm + 1) / 2 > t) --tm;
+    while((tm + 1) * (tm + 2) / 2 <= t) ++tm;
+    tn = t - tm * (tm + 1) / 2;
+  }
   const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int64_t m0 = static_cast<int64_t>(blockIdx.y) * 64, n0 = static_cast<int64_t>(blockIdx.x) * 64;
-  T acc[4][4];
+  const int tx = tid & 7, ty = tid >> 3;
+  const int64_t m0 = tm * TILE, n0 = tn * TILE;
+  T acc[R][R];
 #pragma unroll
-  for(int i = 0; i < 4; ++i)
+  for(int i = 0; i < R; ++i)
 #pragma unroll
-    for(int j = 0; j < 4; ++j) acc[i][j] = T(0);
+    for(int j = 0; j < R; ++j) acc[i][j] = T(0);
   const int passes = dual ? 2 : 1;
   for(int p = 0; p < passes; ++p) {
     const TiledOperand<T> oa = p ? a2 : a;
     const TiledOperand<T> ob = p ? b2 : b;
-    for(int64_t k0 = 0; k0 < K; k0 += 16) {
+    for(int64_t k0 = 0; k0 < K; k0 += BK) {
 #pragma unroll
-      for(int e = 0; e < 4; ++e) {
-        const int idx = tid + e * 256;  // 0..1023 over a 64 x 16 tile
+      for(int e = 0; e < TILE * BK / 64; ++e) {
+        const int idx = tid + e * 64;
         // rows fastest when the operand is contiguous along rows, else k fastest
-        const int r = (oa.s_r == 1) ? (idx & 63) : (idx >> 4);
-        const int kk = (oa.s_r == 1) ? (idx >> 6) : (idx & 15);
+        const int r = (oa.s_r == 1) ? (idx % TILE) : (idx / BK);
+        const int kk = (oa.s_r == 1) ? (idx / TILE) : (idx % BK);
         const int64_t gm = m0 + r, gk = k0 + kk;
         As[kk][r] = (gm < M && gk < K) ? oa.p[gm * oa.s_r + gk * oa.s_k] : T(0);
-        const int rb = (ob.s_r == 1) ? (idx & 63) : (idx >> 4);
-        const int kb = (ob.s_r == 1) ? (idx >> 6) : (idx & 15);
+        const int rb = (ob.s_r == 1) ? (idx % TILE) : (idx / BK);
+        const int kb = (ob.s_r == 1) ? (idx / TILE) : (idx % BK);
         const int64_t gn = n0 + rb, gkb = k0 + kb;
         Bs[kb][rb] = (gn < N && gkb < K) ? ob.p[gn * ob.s_r + gkb * ob.s_k] : T(0);
       }
       __syncthreads();
 #pragma unroll
-      for(int kk = 0; kk < 16; ++kk)
+      for(int kk = 0; kk < BK; ++kk)
 #pragma unroll
-        for(int i = 0; i < 4; ++i)
+        for(int i = 0; i < R; ++i)
 #pragma unroll
-          for(int j = 0; j < 4; ++j) acc[i][j] = fma(As[kk][ty * 4 + i], Bs[kk][tx + 16 * j], acc[i][j]);
+          for(int j = 0; j < R; ++j) acc[i][j] = fma(As[kk][ty * R + i], Bs[kk][tx + 8 * j], acc[i][j]);
       __syncthreads();
     }
   }
   // C values are loaded before the first store (a load cannot move above a
-  // store that may alias it)
-  T cv[4][4];
+  // store that may alias it); then, below the diagonal, the transposed tile C[n][m]
 #pragma unroll
-  for(int i = 0; i < 4; ++i)
+  for(int t = 0; t < 2; ++t) {
+    if(t == 1 && !(lower && tm != tn)) break;
+    T cv[R][R];
 #pragma unroll
-    for(int j = 0; j < 4; ++j) {
-      const int64_t m = m0 + ty * 4 + i, n = n0 + tx + 16 * j;
-      cv[i][j] = (beta != T(0) && m < M && n < N) ? C[m * ldc + n] : T(0);
-    }
+    for(int i = 0; i < R; ++i)
 #pragma unroll
-  for(int i = 0; i < 4; ++i) {
-    const int64_t m = m0 + ty * 4 + i;
-    if(m >= M) continue;
-#pragma unroll
-    for(int j = 0; j < 4; ++j) {
-      const int64_t n = n0 + tx + 16 * j;
-      if(n < N) C[m * ldc + n] = fma(beta, cv[i][j], alpha * acc[i][j]);
-    }
-  }
-  if(lower && blockIdx.x < blockIdx.y) {  // the transposed tile, C[n][m]
-#pragma unroll
-    for(int i = 0; i < 4; ++i)
-#pragma unroll
-      for(int j = 0; j < 4; ++j) {
-        const int64_t m = m0 + ty * 4 + i, n = n0 + tx + 16 * j;
-        cv[i][j] = (beta != T(0) && m < M && n < N) ? C[n * ldc + m] : T(0);
+      for(int j = 0; j < R; ++j) {
+        const int64_t m = m0 + ty * R + i, n = n0 + tx + 8 * j;
+        cv[i][j] = (beta != T(0) && m < M && n < N) ? (t ? C[n * ldc + m] : C[m * ldc + n]) : T(0);
       }
 #pragma unroll
-    for(int i = 0; i < 4; ++i) {
-      const int64_t m = m0 + ty * 4 + i;
-      if(m >= M) continue;
+    for(int i = 0; i < R; ++i)
 #pragma unroll
-      for(int j = 0; j < 4; ++j) {
-        const int64_t n = n0 + tx + 16 * j;
-        if(n < N) C[n * ldc + m] = fma(beta, cv[i][j], alpha * acc[i][j]);
+      for(int j = 0; j < R; ++j) {
+        const int64_t m = m0 + ty * R + i, n = n0 + tx + 8 * j;
+        if(m < M && n < N) (t ? C[n * ldc + m] : C[m * ldc + n]) = fma(beta, cv[i][j], alpha * acc[i][j]);
       }
-    }
   }
 }
 
@@ -109,12 +105,13 @@ gbpoly_status launch_tiled_gemm(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K
     TiledOperand<T> b, bool dual, TiledOperand<T> a2, TiledOperand<T> b2, T beta, T* C, int64_t ldc,
     bool lower = false) {
   if(M == 0 || N == 0) return GBPOLY_OK;
-  const int64_t gx = (N + 63) / 64, gy = (M + 63) / 64;
-  if(gy > 65535) return fail(GBPOLY_ERR_UNSUPPORTED, "matrix too tall for the tiled kernel grid");
-  dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
+  const int64_t gx = (N + kTiledTile - 1) / kTiledTile, gy = (M + kTiledTile - 1) / kTiledTile;
+  lower = lower && M == N;
+  const int64_t tiles = lower ? gy * (gy + 1) / 2 : gx * gy;
+  if(tiles >= (1ll << 31)) return fail(GBPOLY_ERR_UNSUPPORTED, "matrix too large for the tiled kernel grid");
   ProfileScope prof(ctx, sizeof(T) == 8 ? "dgemm_tiled" : "sgemm_tiled");
-  tiled_gemm_kernel<T><<<grid, 256, 0, ctx->stream>>>(M, N, K, alpha, a, b, dual, a2, b2, beta, C, ldc,
-      lower && M == N);
+  tiled_gemm_kernel<T><<<unsigned(tiles), 64, 0, ctx->stream>>>(M, N, K, alpha, a, b, dual, a2, b2, beta, C, ldc, lower,
+      gx);
   GBPOLY_CUDA_TRY(cudaGetLastError());
   return GBPOLY_OK;
 }
