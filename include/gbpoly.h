@@ -122,12 +122,14 @@ gbpoly_status gbpoly_workspace_query(gbpoly_precision prec, int64_t M, int64_t N
  * tf32x3, bf16x6: configurations 3, 4 and 5 run CTA pairs, cta_group::2 MMAs
  * on 256 x 256 tiles; 5 keeps the C tile in shared memory, loaded and stored
  * by TMA, for short K, and runs as 3 for symmetric products or C rows that
- * do not start and end on 16-byte boundaries).  The context keeps one per (form, ceil(log2) of
- * M, N, K); unless tuned or set, a shape whose 256 x 256 tiles give every SM
- * pair a tile uses configuration 5 up to K = 256 (tf32: 512, tf32x3: 128)
- * and 3 beyond, smaller ones a 128 x 128 configuration.  fp8: configuration
- * 1 (128 x 256 tiles) when its tiles give every SM one, else 0 (128 x 128,
- * also every symmetric product). */
+ * do not start and end on 16-byte boundaries; 6 runs CTA pairs on 256 x 128
+ * tiles.  fp16x3: 2 pairs on 256 x 256, 3 on 256 x 128).  The context keeps
+ * one per (form, ceil(log2) of M, N, K); unless tuned or set, a shape whose
+ * 256 x 256 tiles give every SM pair a tile uses configuration 5 up to
+ * K = 256 (tf32: 512, tf32x3: 128) and 3 beyond (fp16x3: 2), a smaller or
+ * symmetric one the tile shape (128 x 128, 256 x 256, 256 x 128) of the least
+ * estimated time.  fp8: configuration 1 (128 x 256 tiles) when its tiles give
+ * every SM one, else 0 (128 x 128, also every symmetric product). */
 gbpoly_status gbpoly_gemm_config_count(gbpoly_precision prec, int* count);
 gbpoly_status gbpoly_gemm_config_set(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K,
     int config);
@@ -143,8 +145,9 @@ gbpoly_status gbpoly_autotune_gemm(gbpoly_ctx* ctx, gbpoly_precision prec, int64
 gbpoly_status gbpoly_autotune_save(gbpoly_ctx* ctx, const char* path);
 gbpoly_status gbpoly_autotune_load(gbpoly_ctx* ctx, const char* path, int* loaded);
 /* K-split tail (CTA-pair configurations, on by default): when the last round
- * of 256 x 256 tiles would leave at least half the resident SM pairs idle,
- * each tile of that round runs as two halves of its K range on two pairs;
+ * of tiles would leave at least half the resident SM pairs idle and half a
+ * tile's K takes longer than the handoff (7 to 9 us), each tile of that round
+ * runs as two halves of its K range on two pairs;
  * the first half adds the second half's partial sums (in a fixed order, so
  * results are the same on every run) and writes C.  The workspace query
  * includes the partial sums. */

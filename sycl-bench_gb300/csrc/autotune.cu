@@ -50,9 +50,13 @@ std::tuple<int, int, int, int> shape_bucket(gbpoly_precision prec, int64_t M, in
   return std::make_tuple(int(prec), ceil_log2(M), ceil_log2(N), ceil_log2(K));
 }
 
-int tuned_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K) {
+int tuned_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K, bool c_tma) {
   auto it = ctx->tuned.find(shape_bucket(prec, M, N, K));
-  return it == ctx->tuned.end() ? default_config(ctx, prec, M, N, K) : it->second;
+  return it == ctx->tuned.end() ? default_config(ctx, prec, M, N, K, c_tma) : it->second;
+}
+
+bool is_tuned(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K) {
+  return ctx->tuned.count(shape_bucket(prec, M, N, K)) != 0;
 }
 
 // Problem class of a group: ceil(log2) of the problem count and of the

@@ -202,9 +202,12 @@ gbpoly_status launch_gemm_tensor(gbpoly_ctx* ctx, gbpoly_precision prec, const G
 // explicit configuration; the configuration the context uses for a shape.
 int tensor_config_count(gbpoly_precision prec);
 gbpoly_status launch_gemm_tensor_config(gbpoly_ctx* ctx, gbpoly_precision prec, int config, const GemmF32Args& a);
-int tuned_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K);
+// (c_tma: TMA can address the rows of C, which the rule for untuned shapes asks).
+int tuned_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K, bool c_tma = true);
+// Whether that configuration was tuned or set, not the rule's.
+bool is_tuned(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K);
 // Configuration used for a shape nobody tuned (split_gemm.cu).
-int default_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K);
+int default_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K, bool c_tma);
 std::tuple<int, int, int, int> shape_bucket(gbpoly_precision prec, int64_t M, int64_t N, int64_t K);
 // Row-panel execution of a tensor-core contraction (host-buffer calls): the
 // plan fixes form and configuration for the full shape; each panel call
@@ -214,8 +217,9 @@ struct TensorPlan {
   int config = 0;
   int64_t M = 0;
 };
-gbpoly_status tensor_plan(gbpoly_ctx* ctx, gbpoly_precision prec, gbpoly_op op_a, gbpoly_op op_b, int64_t M, int64_t N,
-    int64_t K, TensorPlan* plan);
+// (C, ldc: the caller's, whose alignment chooses as the device-buffer call would)
+gbpoly_status tensor_plan(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K, const float* C,
+    int64_t ldc, TensorPlan* plan);
 gbpoly_status tensor_plan_panel(gbpoly_ctx* ctx, const TensorPlan& plan, const GemmF32Args& a, bool first, int64_t r0);
 // Grouped plans (split_gemm.cu): the number of tile configurations of a form,
 // the problem class a group belongs to (autotune.cu), and planning with a

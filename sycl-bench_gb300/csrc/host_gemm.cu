@@ -106,7 +106,7 @@ extern "C" gbpoly_status gbpoly_gemm_f32_host(gbpoly_ctx* ctx, gbpoly_precision 
     return st;
   TensorPlan plan;
   if(prec != GBPOLY_PREC_FP32) {
-    if((st = tensor_plan(ctx, prec, op_a, op_b, M, N, K, &plan)) != GBPOLY_OK) return st;
+    if((st = tensor_plan(ctx, prec, M, N, K, C, ldc, &plan)) != GBPOLY_OK) return st;
   }
   for(int p = 0; p < panels; ++p) {
     const int64_t r0 = p * rows_per, rows = std::min<int64_t>(rows_per, M - r0);

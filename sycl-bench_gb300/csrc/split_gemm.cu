@@ -55,6 +55,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "gbpoly_internal.cuh"
@@ -74,6 +75,24 @@ constexpr uint32_t idesc_of() {
     return umma::InstrDesc<M, N,
         E == Elem::BF16 ? umma::AbType::BF16 : (E == Elem::F16 ? umma::AbType::F16 : umma::AbType::TF32)>::value;
 }
+
+// Tile shapes the configuration rule chooses between: 1-CTA 128 x 128, CTA
+// pairs on 256 x 256 and on 256 x 128.
+enum TileShape { kTileSquare, kTilePair, kTileNarrow };
+
+// Time of one 128-byte-deep chunk of K on a busy device, in microseconds
+// (measured on GB300, kernel time over K; the loads of operand panels from L2,
+// 12 to 13 TB/s, bound the smaller tiles, the MMAs the pairs on 256 x 256).
+constexpr double chunk_us(Elem e, int terms, TileShape s) {
+  if(e == Elem::TF32 && terms == 1) return s == kTileSquare ? 0.48 : (s == kTilePair ? 0.62 : 0.45);
+  if(e == Elem::TF32) return s == kTileSquare ? 0.74 : (s == kTilePair ? 0.95 : 0.70);
+  if(e == Elem::F16) return s == kTileSquare ? 0.74 : (s == kTilePair ? 0.88 : 0.68);
+  if(terms == 3) return s == kTileSquare ? 1.15 : (s == kTilePair ? 1.75 : 1.15);
+  return s == kTileSquare ? 0.70 : (s == kTilePair ? 0.86 : 0.66);  // bf16x3
+}
+// What a K-split tile's handoff costs, in microseconds: in a launch of one
+// unit per CTA, and in a last round.
+constexpr double kHandoffUs = 7, kHandoffLastRoundUs = 9;
 
 // CG_ = 2: a CTA pair (cluster of two) computes a (256 x BN) tile with
 // cta_group::2 MMAs: each CTA holds 128 rows of the A tile and BN/2 rows of
@@ -114,15 +133,24 @@ struct Form {
   // buffers in TMEM (all 512 columns: 2 of 256, 4 of 128) so the MMAs run
   // ahead of the epilogue, also across the C stores between two tiles.
   static constexpr int CH = 128 / ROW;
+  // Launches of one unit per CTA may keep C in the pipeline's stages, loaded
+  // and stored by TMA (RING kernels, forms with one stage per chunk).  The
+  // loads start under the last chunk where the other stages hold the whole C tile.
+  static constexpr bool RING_C = !CEPI && CH == 1;
+  static constexpr bool RING_C_EARLY = RING_C && (STAGES - 1) * STAGE >= C_TILE;
   static constexpr int NBUF = BN <= 128 ? 4 : 2;
   // TMEM allocations are powers of two (>= 32 columns); chunk buffer b
   // starts at column b * BUF_COLS
   static constexpr uint32_t TMEM_COLS = NBUF * BN <= 64 ? 64 : (NBUF * BN <= 128 ? 128 : (NBUF * BN <= 256 ? 256 : 512));
   static constexpr uint32_t BUF_COLS = TMEM_COLS / NBUF;
   static constexpr int HALF = BN / 2;  // columns per epilogue warp
-  // Square tiles: symmetric updates compute the lower triangle of tiles and
-  // mirror them.
-  static constexpr bool MIRROR = BM == BN;
+  // Symmetric updates compute the tiles that reach the lower triangle and
+  // mirror what lies below the diagonal: whole tiles of square ones, the two
+  // CTAs' 128-row halves of a 256 x 128 pair tile each by itself.
+  static constexpr bool HALVES = CG == 2 && BN == BM_CTA;
+  static constexpr bool MIRROR = BM == BN || HALVES;
+  // a chunk's time, for the decision to split K
+  static constexpr double CHUNK_US = chunk_us(E, TERMS, BN == 128 ? kTileNarrow : kTilePair);
   static constexpr int THREADS = 384;  // warpgroup 0: producer, MMA; warpgroups 1-2: epilogue
   static constexpr uint32_t REGS_CTRL = 56, REGS_EPI = 208;
   static constexpr uint32_t IDESC = idesc_of<E, BM, BN>();
@@ -131,7 +159,8 @@ struct Form {
   static_assert(STAGE_TX == CG * STAGE, "pair stage bytes");
   static_assert(SMEM <= 232448, "shared memory");
   static_assert(TMEM_COLS <= 512 && BUF_COLS >= BN, "tensor memory");
-  static_assert((2 * STAGES + 2 * NBUF + 1 + (CEPI ? 8 : 0)) * 8 + 4 <= 256, "barriers fit their 256 bytes");
+  static_assert((2 * STAGES + 2 * NBUF + 1 + (CEPI || RING_C ? 8 : 0)) * 8 + 4 <= 256, "barriers fit their 256 bytes");
+  static_assert(!RING_C || (STAGES * STAGE >= C_TILE && STAGE % (HALF / 32 * C_BOX) == 0), "C boxes in the stages");
   static_assert(!CEPI || (ROW == 128 && !scaled && CG == 2), "C-tile epilogue: CTA-pair 128-byte-row forms");
 };
 
@@ -159,6 +188,16 @@ using FormTF32_p = Form<Elem::TF32, 1, 1, 256, 6, 128, 2>;
 using FormBF16x3_p = Form<Elem::BF16, 2, 3, 256, 3, 128, 2>;
 using FormTF32x3_p = Form<Elem::TF32, 2, 3, 256, 3, 128, 2>;
 using FormBF16x6_p = Form<Elem::BF16, 3, 6, 256, 2, 128, 2>;
+// CTA pairs on 256 x 128 tiles, for launches with too few 256 x 256 tiles:
+// small tiles are bound by their operand loads from L2 (12 to 13 TB/s over the
+// device), 64 KB per 64-K chunk of bf16x3 and CTA on 1-CTA 128 x 128 tiles
+// (0.70 us) and 48 KB here (0.66 us for the same 128 x 128 of C per CTA); and
+// a pair's tile can split its K over two pairs.
+using FormTF32_n = Form<Elem::TF32, 1, 1, 128, 7, 128, 2>;
+using FormBF16x3_n = Form<Elem::BF16, 2, 3, 128, 4, 128, 2>;
+using FormTF32x3_n = Form<Elem::TF32, 2, 3, 128, 4, 128, 2>;
+using FormBF16x6_n = Form<Elem::BF16, 3, 6, 128, 2, 128, 2>;
+using FormF16x3_n = Form<Elem::F16, 2, 3, 128, 4, 128, 2>;
 // CTA pairs with 64-byte rows: more, shorter stages
 using FormTF32_q = Form<Elem::TF32, 1, 1, 256, 12, 64, 2>;
 using FormBF16x3_q = Form<Elem::BF16, 2, 3, 256, 6, 64, 2>;
@@ -649,8 +688,25 @@ struct TileInfo {
   const float* sl[2];
   const float* sr[2];
   int kt;
-  bool mirror;  // symmetric update, tile strictly below the diagonal: also write its transpose
+  bool lower;  // symmetric update: only what lies on or below the diagonal is computed, the rest mirrored
 };
+
+// Row from which a CTA's part of tile t is compared with the diagonal (the
+// first row of the tile, or of the CTA's 128 rows where the halves of a pair
+// tile are mirrored by themselves): below it (> n0) the part is also written
+// transposed, above it (< n0) it is the mirror of another and not written.
+template <class F>
+__device__ __forceinline__ int diag_row(const TileInfo& t, uint32_t rank) {
+  return t.m0 + (F::HALVES ? int(rank) * F::BM_CTA : 0);
+}
+
+// Tiles of a symmetric product that reach its lower triangle: tile row tm has
+// BM / BN (tm + 1) of them, the last row at most the matrix's tn.
+template <int BM, int BN>
+__host__ __device__ constexpr int64_t lower_tiles(int64_t tm, int64_t tn) {
+  constexpr int W = BM >= BN ? BM / BN : 1;
+  return W * tm * (tm - 1) / 2 + (W * tm < tn ? W * tm : tn);
+}
 
 // One contraction: tiles in grouped raster order, tensor maps in the
 // kernel's parameter space.
@@ -676,12 +732,13 @@ struct SingleSched {
   // [0, split_it)) waits for all of them (bounded), adds them to its own
   // sums and writes C.  units == 0: one unit per tile.
   int units = 0, full_tiles = 0, split_it = 0;
-  float* partial = nullptr;  // [slot][CTA of the pair][128 rows][BN columns]
+  float* partial = nullptr;  // [slot][CTA of the pair][128 rows x BN columns, or the RING kernels' registers]
   int* flags = nullptr;      // [slot], zero at launch
-  CUtensorMap cmap;          // C-tile epilogue forms: C (M x N, boxes of 32 x 32, 128-byte swizzle)
+  CUtensorMap cmap;          // C (M x N, boxes of 32 x 32, 128-byte swizzle) where TMA can address its rows
+  bool ring_c = false;       // cmap is set
   __device__ int count() const {
     const int tm = (M + BM - 1) / BM, tn = (N + BN - 1) / BN;
-    return lower ? tm * (tm + 1) / 2 : tm * tn;
+    return lower ? lower_tiles<BM, BN>(tm, tn) : tm * tn;
   }
   __device__ int unit_count() const { return units ? units : count(); }
   // unit u -> tile, role (0 whole tile, 1 first K half, 2 second K half),
@@ -697,16 +754,19 @@ struct SingleSched {
   }
   __device__ TileInfo tile(int t) const {
     int tm, tn;
-    if(lower) {  // row-major walk of the lower triangle: t = tm (tm + 1) / 2 + tn
-      tm = int((sqrtf(8.f * float(t) + 1.f) - 1.f) * 0.5f);
-      while(tm * (tm + 1) / 2 > t) --tm;
-      while((tm + 1) * (tm + 2) / 2 <= t) ++tm;
-      tn = t - tm * (tm + 1) / 2;
+    if(lower) {
+      // row-major walk of the tiles that reach the lower triangle: W tm (tm + 1) / 2
+      // of them precede tile row tm, W = BM / BN per diagonal step
+      constexpr int W = BM >= BN ? BM / BN : 1;
+      tm = int((sqrtf(8.f / W * float(t) + 1.f) - 1.f) * 0.5f);
+      while(W * tm * (tm + 1) / 2 > t) --tm;
+      while(W * (tm + 1) * (tm + 2) / 2 <= t) ++tm;
+      tn = t - W * tm * (tm + 1) / 2;
     } else {
       tile_coords(t, (M + BM - 1) / BM, (N + BN - 1) / BN, tm, tn);
     }
     return TileInfo{tm * BM, tn * BN, M, N, Kp, npair, alpha, beta, C, ldc, maps.p, {sl[0], sl[1]}, {sr[0], sr[1]},
-        kt, lower && tm != tn};
+        kt, lower};
   }
 };
 
@@ -744,17 +804,19 @@ struct GroupedSched {
 // h) reads for tile t: its 32 rows x HALF columns, and their mirror.
 template <class F>
 __device__ __forceinline__ void prefetch_c_warp(const TileInfo& t, uint32_t rank, int q, int h, int lane) {
+  const int below = t.lower ? diag_row<F>(t, rank) - t.n0 : 0;
+  if(below < 0) return;
   constexpr int segs = F::HALF / 32;  // 128-byte segments per row
   const int row0 = t.m0 + int(rank) * F::BM_CTA + 32 * q, col0 = t.n0 + h * F::HALF;
 #pragma unroll
   for(int p = 0; p < segs; ++p) {
     const int l = lane + 32 * p, r = row0 + l / segs, n = col0 + 32 * (l % segs);
     if(r < t.M && n < t.N) prefetch_l2(t.C + int64_t(r) * t.ldc + n);
-    if(F::MIRROR && t.mirror && col0 + l < t.N && row0 < t.M) prefetch_l2(t.C + int64_t(col0 + l) * t.ldc + row0);
+    if(F::MIRROR && below > 0 && col0 + l < t.N && row0 < t.M) prefetch_l2(t.C + int64_t(col0 + l) * t.ldc + row0);
   }
 }
 
-template <class F, class S>
+template <class F, class S, bool RING>
 __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_constant__ S sched, int* err) {
   extern __shared__ __align__(1024) char smem_raw[];
   char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -763,8 +825,8 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
   uint64_t* chunk_full = empty + F::STAGES;     // [NBUF]
   uint64_t* chunk_empty = chunk_full + F::NBUF;  // [NBUF]
   uint64_t* drain = chunk_empty + F::NBUF;
-  uint64_t* cbar = drain + 1;  // C-tile epilogue: one barrier per epilogue warp for its C boxes
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1 + (F::CEPI ? 8 : 0));
+  uint64_t* cbar = drain + 1;  // C through TMA: one barrier per epilogue warp for its C boxes
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1 + (F::CEPI || RING ? 8 : 0));
   float(*epi_stage)[33] = reinterpret_cast<float(*)[33]>(smem + F::STAGES * F::STAGE + 256);  // 8 warps x [32][33]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -786,7 +848,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
       mbar_init(&chunk_empty[b], 8 * F::CG);  // one arrival per epilogue warp of the pair
     }
     mbar_init(drain, 1);
-    if constexpr(F::CEPI)
+    if constexpr(F::CEPI || RING)
       for(int w = 0; w < 8; ++w) mbar_init(&cbar[w], 1);
     fence_mbar_init();
   }
@@ -941,10 +1003,8 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
     // C-tile epilogue: this warp's HALF / 32 boxes of C, loads and stores issued so far
     char* const cbox = smem + F::STAGES * F::STAGE + 1024 + (warp - 4) * (F::HALF / 32) * F::C_BOX;
     int c_loads = 0, c_stores = 0;
-    // chunk buffers are released on the first CTA's barrier (MMAs are issued there)
-    static_assert(F::CG == 1 || F::NBUF == 2, "CTA pairs: two chunk buffers");
-    const uint32_t chunk_empty_pair[2] = {F::CG == 2 ? cluster_map(&chunk_empty[0], 0) : 0u,
-        F::CG == 2 ? cluster_map(&chunk_empty[1], 0) : 0u};
+    // chunk buffers are released on the first CTA's barriers (MMAs are issued there)
+    const uint32_t chunk_empty_pair = F::CG == 2 ? cluster_map(chunk_empty, 0) : 0u;
     for(int u = first_tile; u < units && ok; u += tile_step) {
       int tile, role, slot;
       sched.unit(u, tile, role, slot);
@@ -971,6 +1031,25 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
           ++c_loads;
         }
       }
+      // RING: the CTA's only unit.  This warp's HALF / 32 boxes of C live in the
+      // pipeline's stages, which no later tile fills.  The loads start while
+      // the last chunk's MMAs run: every stage but that chunk's has been read
+      // (its chunk was complete), and the boxes lie from the stage after it.
+      const int below = F::MIRROR && ti.lower ? diag_row<F>(ti, rank) - ti.n0 : 0;
+      constexpr int kBoxes = F::HALF / 32;
+      char* ring_box = nullptr;
+      auto load_ring = [&](int last_chunk) {
+        const int at = F::RING_C_EARLY ? (last_chunk + 1) % F::STAGES * F::STAGE : 0;
+        ring_box = smem + (at + (warp - 4) * kBoxes * F::C_BOX) % (F::STAGES * F::STAGE);
+        if constexpr(RING) {
+          if(beta != 0.f && lane == 0) {
+            mbar_arrive_expect_tx(&cbar[warp - 4], kBoxes * F::C_BOX);
+#pragma unroll
+            for(int j = 0; j < kBoxes; ++j)
+              tma_load_2d(ring_box + j * F::C_BOX, &sched.cmap, &cbar[warp - 4], nbase + 32 * j, crow);
+          }
+        }
+      };
       // Scaled forms (E4M3, F16): chunk c (stage iteration it0 + c, CH = 1)
       // is multiplied by the factor of its left row block and right column
       // block, for each of the NCB blocks the warp's columns span.  Lane t
@@ -1024,7 +1103,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         __syncwarp();
         if(lane == 0) {
           if constexpr(F::CG == 2)
-            mbar_arrive_cluster(b ? chunk_empty_pair[1] : chunk_empty_pair[0]);
+            mbar_arrive_cluster(chunk_empty_pair + 8 * b);
           else
             mbar_arrive(&chunk_empty[b]);
         }
@@ -1034,6 +1113,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         auto consume = [&](int c) -> bool {
           const int b = chunk % F::NBUF;
           if(!F::CEPI && c == max(0, chunks - 4) && beta != 0.f && role != 2) prefetch_c_warp<F>(ti, rank, q, h, lane);
+          if(RING && F::RING_C_EARLY && c == chunks - 1 && role != 2 && below >= 0) load_ring(chunk);
           if(!mbar_wait(&chunk_full[b], (chunk / F::NBUF) & 1, err, kDevErrMmaWait)) return false;
           umma::fence_after_sync();
           const uint32_t base = tmem + (uint32_t(32 * q) << 16) + uint32_t(b) * F::BUF_COLS + uint32_t(h * F::HALF);
@@ -1096,6 +1176,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         for(int c = 0; c < chunks; ++c, ++chunk) {
           const int b = chunk % F::NBUF;
           if(!F::CEPI && c == max(0, chunks - 4) && beta != 0.f && role != 2) prefetch_c_warp<F>(ti, rank, q, h, lane);
+          if(RING && F::RING_C_EARLY && c == chunks - 1 && role != 2 && below >= 0) load_ring(chunk);
           if(!mbar_wait(&chunk_full[b], (chunk / F::NBUF) & 1, err, kDevErrMmaWait)) {
             ok = false;
             break;
@@ -1116,7 +1197,11 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
           release(b);
         }
       }
-      if(!ok) continue;
+      if(!ok) {
+        // do not leave while C's copies into the stages are in flight
+        if(RING && ring_box != nullptr && beta != 0.f) mbar_wait(&cbar[warp - 4], 0, err, kDevErrDrainWait);
+        continue;
+      }
       if constexpr(F::CEPI) {
         // C = alpha acc + beta C in the boxes (lane = row: eight 16-byte
         // chunks, swizzled by row, so each quarter warp covers all banks),
@@ -1155,6 +1240,101 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         ++c_stores;
         continue;
       }
+      if(F::HALVES && below < 0) {  // above the diagonal: another CTA's mirror writes it
+        if(role == 2 && lane == 0) atomicAdd(&sched.flags[slot], 1);
+        continue;
+      }
+      if constexpr(RING) {
+        // K-split tile: the second half stores its sums (register i of a warp
+        // as one 128-byte row), the first half waits for them and adds them to
+        // its own (first + second) before writing C
+        if(F::CG == 2 && role != 0) {
+          float* part = sched.partial + ((size_t(slot) * F::CG + rank) * 8 + (warp - 4)) * (F::HALF * 32) + lane;
+          if(role == 2) {
+#pragma unroll
+            for(int i = 0; i < F::HALF; ++i) __stcg(part + 32 * i, acc[i]);
+            __threadfence();
+            __syncwarp();
+            if(lane == 0) atomicAdd(&sched.flags[slot], 1);  // sums stored: count this warp
+            continue;
+          }
+          if(!wait_count(&sched.flags[slot], 8 * F::CG, err, kDevErrSplitWait)) {
+            ok = false;
+            continue;
+          }
+#pragma unroll
+          for(int i0 = 0; i0 < F::HALF; i0 += 32) {
+            float v[32];
+#pragma unroll
+            for(int i = 0; i < 32; ++i) v[i] = __ldcg(part + 32 * (i0 + i));
+#pragma unroll
+            for(int i = 0; i < 32; ++i) acc[i0 + i] += v[i];
+          }
+        }
+        // C = alpha acc + beta C in the boxes (lane = row: eight 16-byte
+        // chunks, swizzled by row), each stored by TMA when done (clipped at
+        // the matrix edges)
+        if(!F::RING_C_EARLY) load_ring(0);
+        if(beta != 0.f && !mbar_wait(&cbar[warp - 4], 0, err, kDevErrMmaWait)) {
+          ok = false;
+          continue;
+        }
+#pragma unroll
+        for(int j = 0; j < kBoxes; ++j) {
+          char* row = ring_box + j * F::C_BOX + lane * 128;
+#pragma unroll
+          for(int k = 0; k < 8; ++k) {
+            float4* p4 = reinterpret_cast<float4*>(row + ((k ^ (lane & 7)) << 4));
+            const float4 cv = beta != 0.f ? *p4 : make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 o;
+            o.x = fmaf(beta, cv.x, alpha * acc[32 * j + 4 * k]);
+            o.y = fmaf(beta, cv.y, alpha * acc[32 * j + 4 * k + 1]);
+            o.z = fmaf(beta, cv.z, alpha * acc[32 * j + 4 * k + 2]);
+            o.w = fmaf(beta, cv.w, alpha * acc[32 * j + 4 * k + 3]);
+            *p4 = o;
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if(lane == 0) {
+            tma_store_2d(&sched.cmap, ring_box + j * F::C_BOX, nbase + 32 * j, crow);
+            bulk_commit();
+          }
+        }
+        if(F::MIRROR && below > 0) {
+          // the transpose, C[nbase + r][crow + lane], in the same boxes once their stores have read them
+          if(lane == 0) {
+            bulk_wait_read_all();
+            if(beta != 0.f) {
+              mbar_arrive_expect_tx(&cbar[warp - 4], kBoxes * F::C_BOX);
+#pragma unroll
+              for(int j = 0; j < kBoxes; ++j)
+                tma_load_2d(ring_box + j * F::C_BOX, &sched.cmap, &cbar[warp - 4], crow, nbase + 32 * j);
+            }
+          }
+          __syncwarp();
+          if(beta != 0.f && !mbar_wait(&cbar[warp - 4], 1, err, kDevErrMmaWait)) {
+            ok = false;
+            continue;
+          }
+#pragma unroll
+          for(int j = 0; j < kBoxes; ++j) {
+#pragma unroll
+            for(int r = 0; r < 32; ++r) {
+              float* p = reinterpret_cast<float*>(
+                  ring_box + j * F::C_BOX + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3));
+              *p = fmaf(beta, beta != 0.f ? *p : 0.f, alpha * acc[32 * j + r]);
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if(lane == 0) {
+              tma_store_2d(&sched.cmap, ring_box + j * F::C_BOX, crow, nbase + 32 * j);
+              bulk_commit();
+            }
+          }
+        }
+        ++c_stores;
+        continue;
+      } else {
       // K-split tile: the second half stores its sums (partial tile of the
       // CTA: 128 rows x BN, row-major), the first half waits for them and
       // adds them to its own (first + second) before writing C
@@ -1207,7 +1387,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
           }
         }
         if constexpr(F::MIRROR) {
-          if(ti.mirror) {
+          if(below > 0) {
           // transpose: C[n0 + 32j + r][row0 + lane] from the product element (row0 + lane, n0 + 32j + r)
           const int mrow0 = nbase + 32 * j, mcol = row0 + lane;
           if(mcol < M) {
@@ -1234,8 +1414,9 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         __syncwarp();
         if(lane == 0) atomicAdd(&sched.flags[slot], 1);
       }
+      }  // staged epilogue
     }
-    if constexpr(F::CEPI)
+    if constexpr(F::CEPI || RING)
       if(lane == 0 && c_stores > 0) bulk_wait_all();  // C written before the CTA leaves
   }
 
@@ -1299,16 +1480,16 @@ gbpoly_status make_product_maps(gbpoly_ctx* ctx, ProductMaps& pm, Panels left, i
 
 // Once per device context: shared-memory opt-in and the register check of
 // the warp split.
-template <class F, class S>
+template <class F, class S, bool RING>
 gbpoly_status tc_prepare(gbpoly_ctx* ctx) {
   static ContextMark prepared;
   if(prepared.valid(ctx->device)) return GBPOLY_OK;
-  GBPOLY_CUDA_TRY(cudaFuncSetAttribute(split_gemm_kernel<F, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
+  GBPOLY_CUDA_TRY(cudaFuncSetAttribute(split_gemm_kernel<F, S, RING>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
   // setmaxnreg redistributes the registers the CTA was launched with: the
   // split must fit in threads x registers-per-thread at launch, or the
   // increase would wait forever.
   cudaFuncAttributes fa;
-  GBPOLY_CUDA_TRY(cudaFuncGetAttributes(&fa, split_gemm_kernel<F, S>));
+  GBPOLY_CUDA_TRY(cudaFuncGetAttributes(&fa, split_gemm_kernel<F, S, RING>));
   const long need = 128l * F::REGS_CTRL + 256l * F::REGS_EPI;
   if(long(fa.numRegs) * F::THREADS < need)
     return fail(GBPOLY_ERR_UNSUPPORTED, "tensor-core kernel built with too few registers for its warp split");
@@ -1341,7 +1522,7 @@ template <class F, class S>
 gbpoly_status pair_clusters(gbpoly_ctx* ctx, int& clusters) {
   static int max_clusters[32] = {};
   static ContextMark known;
-  gbpoly_status st = tc_prepare<F, S>(ctx);
+  gbpoly_status st = tc_prepare<F, S, false>(ctx);
   if(st != GBPOLY_OK) return st;
   if(known.valid(ctx->device)) {
     clusters = max_clusters[ctx->device];
@@ -1349,7 +1530,7 @@ gbpoly_status pair_clusters(gbpoly_ctx* ctx, int& clusters) {
   }
   PairLaunch<F> pl(ctx, ctx->sm_count / 2);
   int n = 0;
-  GBPOLY_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, split_gemm_kernel<F, S>, &pl.cfg));
+  GBPOLY_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, split_gemm_kernel<F, S, false>, &pl.cfg));
   if(n <= 0) return fail(GBPOLY_ERR_UNSUPPORTED, "no CTA pair of this tensor-core configuration fits on the device");
   if(ctx->device >= 0 && ctx->device < 32) {
     max_clusters[ctx->device] = n;
@@ -1366,13 +1547,16 @@ gbpoly_status pair_clusters(gbpoly_ctx* ctx, int& clusters) {
 // full rounds split: with more, the last round is a small share of the time
 // and pairing two clusters on one tile (the first half waits for the second)
 // costs about what it saves (measured on GB300: +6 to +15% at 2560 and 4096,
-// -1 to -3% at 8192).
+// -1 to -3% at 8192).  Nor do tiles whose half K takes less time than the
+// handoff (bf16x3, one round, us split / whole: K = 128 24.2 / 18.7, K = 1024
+// 31.2 / 31.1, 256 x 4096 x 4096 71 / 89).
 struct TailPlan {
   int64_t units = 0;  // work units of the launch
   int full_tiles = 0, split_it = 0, slots = 0;
-  size_t bytes = 0;
+  size_t slot_bytes = 0, bytes = 0;
 };
-constexpr size_t kTailSlotBytes = size_t(256) * 256 * sizeof(float);  // one 256 x 256 FP32 tile
+constexpr int kTailTile = 256;
+constexpr size_t kTailSlotBytes = size_t(kTailTile) * kTailTile * sizeof(float);  // one 256 x 256 FP32 tile
 constexpr int kTailMaxRounds = 8;
 
 template <class F, class S>
@@ -1380,19 +1564,22 @@ gbpoly_status plan_tail(gbpoly_ctx* ctx, int64_t tiles, int64_t iters, TailPlan&
   tp = TailPlan{};
   tp.units = tiles;
   if constexpr(F::CG == 2 && !F::CEPI) {
-    static_assert(size_t(F::BM) * F::BN * sizeof(float) == kTailSlotBytes, "tail slot size");
+    constexpr size_t kSlotBytes = size_t(F::BM) * F::BN * sizeof(float);
+    static_assert(kSlotBytes * (kTailTile / F::BN) == kTailSlotBytes, "tail slot size");
     const int64_t chunks = (iters + F::CH - 1) / F::CH;
     if(!ctx->tail_split || tiles <= 0 || chunks < 2) return GBPOLY_OK;
     int P = 0;
     gbpoly_status st = pair_clusters<F, S>(ctx, P);
     if(st != GBPOLY_OK) return st;
     const int64_t R = tiles % P;
-    if(R > 0 && 2 * R <= P && tiles / P < kTailMaxRounds) {
+    const double saved = double(chunks / 2) * F::CHUNK_US;
+    if(R > 0 && 2 * R <= P && tiles / P < kTailMaxRounds && saved >= (tiles < P ? kHandoffUs : kHandoffLastRoundUs)) {
       tp.full_tiles = int(tiles - R);
       tp.units = tiles + R;
       tp.split_it = int(chunks / 2 * F::CH);
       tp.slots = int(R);
-      tp.bytes = size_t(R) * kTailSlotBytes + align_up(size_t(R) * sizeof(int), 256);
+      tp.slot_bytes = kSlotBytes;
+      tp.bytes = size_t(R) * kSlotBytes + align_up(size_t(R) * sizeof(int), 256);
     }
   }
   return GBPOLY_OK;
@@ -1406,32 +1593,47 @@ gbpoly_status apply_tail(gbpoly_ctx* ctx, const TailPlan& tp, char* base, S& sch
   sched.full_tiles = tp.full_tiles;
   sched.split_it = tp.split_it;
   sched.partial = reinterpret_cast<float*>(base);
-  sched.flags = reinterpret_cast<int*>(base + size_t(tp.slots) * kTailSlotBytes);
+  sched.flags = reinterpret_cast<int*>(base + size_t(tp.slots) * tp.slot_bytes);
   GBPOLY_CUDA_TRY(cudaMemsetAsync(sched.flags, 0, size_t(tp.slots) * sizeof(int), ctx->stream));
   return GBPOLY_OK;
 }
 
 // Launch the tensor-core kernel for scheduler S: one persistent CTA (or CTA
 // pair) per SM (pair of SMs), walking `units` work units.
+template <class F, class S, bool RING>
+gbpoly_status launch_tc_variant(gbpoly_ctx* ctx, const S& sched, int64_t units, int resident, const char* kernel_name) {
+  gbpoly_status st = tc_prepare<F, S, RING>(ctx);
+  if(st != GBPOLY_OK) return st;
+  const int grid = int(std::min<int64_t>(units, resident));
+  ProfileScope prof(ctx, kernel_name);
+  if constexpr(F::CG == 2) {
+    PairLaunch<F> pl(ctx, grid);
+    GBPOLY_CUDA_TRY(cudaLaunchKernelEx(&pl.cfg, split_gemm_kernel<F, S, RING>, sched, ctx->err_dev));
+  } else {
+    split_gemm_kernel<F, S, RING><<<grid, F::THREADS, F::SMEM, ctx->stream>>>(sched, ctx->err_dev);
+    GBPOLY_CUDA_TRY(cudaGetLastError());
+  }
+  return GBPOLY_OK;
+}
+
+// A launch that gives every CTA (or pair) at most one unit moves C through
+// TMA where it can (a whole C tile in flight at once in the stages nobody
+// fills again, instead of 16 rows of 128 bytes per warp): a single 256 x 256
+// pair tile takes 15 us instead of 25 (K = 128), gemm 2048 of bf16x3 39
+// instead of 47.  Launches of more units keep the staged epilogue alone: with
+// both in one kernel its loop lost registers (fp16x3 at 4096 315 -> 375 us).
 template <class F, class S>
 gbpoly_status launch_tc_kernel(gbpoly_ctx* ctx, const S& sched, int64_t units, const char* kernel_name) {
-  gbpoly_status st = tc_prepare<F, S>(ctx);
-  if(st != GBPOLY_OK) return st;
   if(units <= 0) return GBPOLY_OK;
+  int resident = ctx->sm_count;  // CTAs, or clusters of two, resident at once
   if constexpr(F::CG == 2) {
-    // CTA pairs: a cluster of two per tile, as many clusters as fit at once
-    int P = 0;
-    if((st = pair_clusters<F, S>(ctx, P)) != GBPOLY_OK) return st;
-    PairLaunch<F> pl(ctx, int(std::min<int64_t>(units, P)));
-    ProfileScope prof(ctx, kernel_name);
-    GBPOLY_CUDA_TRY(cudaLaunchKernelEx(&pl.cfg, split_gemm_kernel<F, S>, sched, ctx->err_dev));
-    return GBPOLY_OK;
+    gbpoly_status st = pair_clusters<F, S>(ctx, resident);
+    if(st != GBPOLY_OK) return st;
   }
-  const int grid = int(std::min<int64_t>(units, ctx->sm_count));
-  ProfileScope prof(ctx, kernel_name);
-  split_gemm_kernel<F, S><<<grid, F::THREADS, F::SMEM, ctx->stream>>>(sched, ctx->err_dev);
-  GBPOLY_CUDA_TRY(cudaGetLastError());
-  return GBPOLY_OK;
+  if constexpr(F::RING_C && std::is_same_v<S, SingleSched<F::BM, F::BN>>)
+    if(sched.ring_c && units <= resident)
+      return launch_tc_variant<F, S, true>(ctx, sched, units, resident, kernel_name);
+  return launch_tc_variant<F, S, false>(ctx, sched, units, resident, kernel_name);
 }
 
 // Workspace layout: terms x [A panel] then terms x [B panel] (B absent when
@@ -1462,6 +1664,15 @@ bool c_tile_ok(const GemmF32Args& a) {
   return (reinterpret_cast<uintptr_t>(a.C) & 15) == 0 && (a.ldc & 3) == 0 && (a.N & 3) == 0;
 }
 
+// C's tensor map for the configurations that move C through TMA.
+template <class F, class S>
+gbpoly_status set_c_map(gbpoly_ctx* ctx, const GemmF32Args& a, S& sched) {
+  if(!(F::CEPI || F::RING_C) || !c_tile_ok(a)) return GBPOLY_OK;
+  sched.ring_c = true;
+  return make_tmap_2d(ctx, &sched.cmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.C, a.M, a.N, a.ldc, 32, 32,
+      CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
 template <class F>
 gbpoly_status run_form(gbpoly_ctx* ctx, const GemmF32Args& a, const char* kernel_name) {
   if(a.M == 0 || a.N == 0) return GBPOLY_OK;
@@ -1475,10 +1686,7 @@ gbpoly_status run_form(gbpoly_ctx* ctx, const GemmF32Args& a, const char* kernel
   using Sched = SingleSched<F::BM, F::BN>;
   int64_t tiles = ((a.M + F::BM - 1) / F::BM) * ((a.N + F::BN - 1) / F::BN);
   const bool lower = F::MIRROR && (same || a.dual) && a.M == a.N;  // symmetric product: lower triangle of tiles
-  if(lower) {
-    const int64_t t = (a.M + F::BM - 1) / F::BM;
-    tiles = t * (t + 1) / 2;
-  }
+  if(lower) tiles = lower_tiles<F::BM, F::BN>((a.M + F::BM - 1) / F::BM, (a.N + F::BN - 1) / F::BN);
   TailPlan tail;
   gbpoly_status st = plan_tail<F, Sched>(ctx, tiles, (Kp / F::BK) * (a.dual ? 2 : 1), tail);
   if(st != GBPOLY_OK) return st;
@@ -1519,12 +1727,9 @@ gbpoly_status run_form(gbpoly_ctx* ctx, const GemmF32Args& a, const char* kernel
     sched.sl[1] = sb, sched.sr[1] = sa;  // syr2k's second pairing, B_i . A_j^T
     sched.kt = int(kt);
   }
-  if constexpr(F::CEPI) {
-    if(lower || !c_tile_ok(a)) return fail(GBPOLY_ERR_UNSUPPORTED, "C-tile epilogue: non-symmetric, 16-byte-aligned C");
-    if((st = make_tmap_2d(ctx, &sched.cmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.C, a.M, a.N, a.ldc, 32, 32,
-            CU_TENSOR_MAP_SWIZZLE_128B)) != GBPOLY_OK)
-      return st;
-  }
+  if(F::CEPI && (lower || !c_tile_ok(a)))
+    return fail(GBPOLY_ERR_UNSUPPORTED, "C-tile epilogue: non-symmetric, 16-byte-aligned C");
+  if((st = set_c_map<F>(ctx, a, sched)) != GBPOLY_OK) return st;
   if((st = apply_tail(ctx, tail, ws + a_bytes + b_bytes + sa_bytes + sb_bytes, sched)) != GBPOLY_OK) return st;
   return launch_tc_kernel<F>(ctx, sched, tail.units, kernel_name);
 }
@@ -1576,6 +1781,7 @@ gbpoly_status run_fp8(gbpoly_ctx* ctx, const GemmF32Args& a) {
     sched.maps.p[1] = sched.maps.p[0];
   }
   const int64_t tiles = ((a.M + F::BM - 1) / F::BM) * ((a.N + F::BN - 1) / F::BN);
+  if((st = set_c_map<F>(ctx, a, sched)) != GBPOLY_OK) return st;
   return launch_tc_kernel<F>(ctx, sched, tiles, "fp8_gemm");
 }
 
@@ -1591,9 +1797,9 @@ size_t workspace_bytes(gbpoly_precision prec, int64_t M, int64_t N, int64_t K, b
   // The largest over the configurations of the form (they differ only in
   // padding), plus the K-split tail of CTA-pair configurations: at most half
   // the resident pairs of a device of up to 256 SMs, and no more than the
-  // shape's 256 x 256 tiles.
+  // shape's 256 x 256 tiles (or twice as many of half the size).
   const int64_t slots = std::min<int64_t>(64, ((M + 255) / 256) * ((N + 255) / 256));
-  const size_t tail = size_t(slots) * kTailSlotBytes + align_up(size_t(slots) * sizeof(int), 256);
+  const size_t tail = size_t(slots) * kTailSlotBytes + align_up(size_t(2 * slots) * sizeof(int), 256);
   switch(prec) {
   case GBPOLY_PREC_TF32: return bytes_of<FormTF32>(M, N, K, same) + tail;
   case GBPOLY_PREC_BF16X3: return bytes_of<FormBF16x3>(M, N, K, same) + tail;
@@ -1621,9 +1827,9 @@ int tensor_config_count(gbpoly_precision prec) {
   case GBPOLY_PREC_TF32:
   case GBPOLY_PREC_BF16X3:
   case GBPOLY_PREC_TF32X3:
-  case GBPOLY_PREC_BF16X6: return 6;  // configurations 3, 4, 5: CTA pairs (5: C tile in shared memory)
+  case GBPOLY_PREC_BF16X6: return 7;  // 3, 4, 5: CTA pairs (5: C tile in shared memory), 6: pairs on 256 x 128 tiles
   case GBPOLY_PREC_FP8: return 2;  // configuration 1: 128 x 256 tiles
-  case GBPOLY_PREC_FP16X3: return 3;  // 0: 128 x 256, 1: 128 x 128, 2: CTA pairs 256 x 256
+  case GBPOLY_PREC_FP16X3: return 4;  // 0: 128 x 256, 1: 128 x 128, 2: CTA pairs 256 x 256, 3: pairs 256 x 128
   default: return 0;
   }
 }
@@ -1636,29 +1842,34 @@ gbpoly_status launch_gemm_tensor_config(gbpoly_ctx* ctx, gbpoly_precision prec, 
   case GBPOLY_PREC_TF32 * 8 + 3: return run_form<FormTF32_p>(ctx, a, "tf32_gemm");
   case GBPOLY_PREC_TF32 * 8 + 4: return run_form<FormTF32_q>(ctx, a, "tf32_gemm");
   case GBPOLY_PREC_TF32 * 8 + 5: return run_form<FormTF32_t>(ctx, a, "tf32_gemm");
+  case GBPOLY_PREC_TF32 * 8 + 6: return run_form<FormTF32_n>(ctx, a, "tf32_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 0: return run_form<FormBF16x3>(ctx, a, "bf16x3_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 1: return run_form<FormBF16x3_b>(ctx, a, "bf16x3_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 2: return run_form<FormBF16x3_c>(ctx, a, "bf16x3_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 3: return run_form<FormBF16x3_p>(ctx, a, "bf16x3_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 4: return run_form<FormBF16x3_q>(ctx, a, "bf16x3_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 5: return run_form<FormBF16x3_t>(ctx, a, "bf16x3_gemm");
+  case GBPOLY_PREC_BF16X3 * 8 + 6: return run_form<FormBF16x3_n>(ctx, a, "bf16x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 0: return run_form<FormTF32x3>(ctx, a, "tf32x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 1: return run_form<FormTF32x3_b>(ctx, a, "tf32x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 2: return run_form<FormTF32x3_c>(ctx, a, "tf32x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 3: return run_form<FormTF32x3_p>(ctx, a, "tf32x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 4: return run_form<FormTF32x3_q>(ctx, a, "tf32x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 5: return run_form<FormTF32x3_t>(ctx, a, "tf32x3_gemm");
+  case GBPOLY_PREC_TF32X3 * 8 + 6: return run_form<FormTF32x3_n>(ctx, a, "tf32x3_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 0: return run_form<FormBF16x6>(ctx, a, "bf16x6_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 1: return run_form<FormBF16x6_b>(ctx, a, "bf16x6_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 2: return run_form<FormBF16x6_c>(ctx, a, "bf16x6_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 3: return run_form<FormBF16x6_p>(ctx, a, "bf16x6_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 4: return run_form<FormBF16x6_q>(ctx, a, "bf16x6_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 5: return run_form<FormBF16x6_t>(ctx, a, "bf16x6_gemm");
+  case GBPOLY_PREC_BF16X6 * 8 + 6: return run_form<FormBF16x6_n>(ctx, a, "bf16x6_gemm");
   case GBPOLY_PREC_FP8 * 8 + 0: return run_fp8<FormFP8>(ctx, a);
   case GBPOLY_PREC_FP8 * 8 + 1: return run_fp8<FormFP8_w>(ctx, a);
   case GBPOLY_PREC_FP16X3 * 8 + 0: return run_form<FormF16x3>(ctx, a, "fp16x3_gemm");
   case GBPOLY_PREC_FP16X3 * 8 + 1: return run_form<FormF16x3_c>(ctx, a, "fp16x3_gemm");
   case GBPOLY_PREC_FP16X3 * 8 + 2: return run_form<FormF16x3_p>(ctx, a, "fp16x3_gemm");
+  case GBPOLY_PREC_FP16X3 * 8 + 3: return run_form<FormF16x3_n>(ctx, a, "fp16x3_gemm");
   default: return fail(GBPOLY_ERR_UNSUPPORTED, "precision form or tile configuration not available");
   }
 }
@@ -1671,8 +1882,16 @@ template <class F>
 gbpoly_status run_form_panel(gbpoly_ctx* ctx, const GemmF32Args& a, int64_t Mfull, bool first, int64_t r0,
     const char* name) {
   const Layout lay = layout<F>(Mfull, a.N, a.K, false);
-  gbpoly_status st = ensure_workspace(ctx, lay.a_bytes + lay.b_bytes);
+  using Sched = SingleSched<F::BM, F::BN>;
+  // A whole call that would split the K of every tile (a launch of less than
+  // half a round) is split the same way panel by panel, so that the panels
+  // give its bits.
+  TailPlan tail;
+  gbpoly_status st = plan_tail<F, Sched>(ctx, ((Mfull + F::BM - 1) / F::BM) * ((a.N + F::BN - 1) / F::BN), lay.Kp / F::BK,
+      tail);
   if(st != GBPOLY_OK) return st;
+  if(tail.slots > 0 && tail.full_tiles > 0) tail = TailPlan{};
+  if((st = ensure_workspace(ctx, lay.a_bytes + lay.b_bytes + tail.bytes)) != GBPOLY_OK) return st;
   char* ws = static_cast<char*>(ctx->ws.ptr);
   Panels pa{ws + size_t(r0) * lay.Kp * F::esz, lay.a_stride};
   Panels pb{ws + lay.a_bytes, lay.b_stride};
@@ -1682,8 +1901,14 @@ gbpoly_status run_form_panel(gbpoly_ctx* ctx, const GemmF32Args& a, int64_t Mful
   GemmMaps maps;
   if((st = make_product_maps<F>(ctx, maps.p[0], pa, a.M, pb, a.N, lay.Kp)) != GBPOLY_OK) return st;
   maps.p[1] = maps.p[0];
-  SingleSched<F::BM, F::BN> sched{maps, 1, int(a.M), int(a.N), int(lay.Kp), a.alpha, a.beta, a.C, a.ldc};
-  const int64_t tiles = ((a.M + F::BM - 1) / F::BM) * ((a.N + F::BN - 1) / F::BN);
+  Sched sched{maps, 1, int(a.M), int(a.N), int(lay.Kp), a.alpha, a.beta, a.C, a.ldc};
+  int64_t tiles = ((a.M + F::BM - 1) / F::BM) * ((a.N + F::BN - 1) / F::BN);
+  if(tail.slots > 0) {
+    tail.slots = int(tiles);
+    tail.units = tiles = 2 * tiles;
+    if((st = apply_tail(ctx, tail, ws + lay.a_bytes + lay.b_bytes, sched)) != GBPOLY_OK) return st;
+  }
+  if((st = set_c_map<F>(ctx, a, sched)) != GBPOLY_OK) return st;
   return launch_tc_kernel<F>(ctx, sched, tiles, name);
 }
 
@@ -1695,21 +1920,70 @@ bool config_is_square(gbpoly_precision prec, int config) {
   switch(prec) {
   case GBPOLY_PREC_TF32:
   case GBPOLY_PREC_BF16X3:
-  case GBPOLY_PREC_TF32X3: return config == 2 || config == 3 || config == 4;
-  case GBPOLY_PREC_BF16X6: return config == 0 || config == 1 || config == 3 || config == 4;
+  case GBPOLY_PREC_TF32X3: return config == 2 || config == 3 || config == 4 || config == 6;
+  case GBPOLY_PREC_BF16X6: return config == 0 || config == 1 || config == 3 || config == 4 || config == 6;
   case GBPOLY_PREC_FP8: return config == 0;
-  case GBPOLY_PREC_FP16X3: return config == 1 || config == 2;
+  case GBPOLY_PREC_FP16X3: return config == 1 || config == 2 || config == 3;
   default: return false;
   }
 }
 // CTA pairs when their 256 x 256 tiles give every SM pair at least one tile.
 bool pairs_fill(gbpoly_ctx* ctx, int64_t pair_tiles) { return pair_tiles >= std::max(1, ctx->sm_count / 2); }
-int square_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t N) {
+
+int config_of(gbpoly_precision prec, TileShape s) {
+  if(prec == GBPOLY_PREC_FP16X3) return s == kTileSquare ? 1 : (s == kTilePair ? 2 : 3);
+  return s == kTileSquare ? (prec == GBPOLY_PREC_BF16X6 ? 0 : 2) : (s == kTilePair ? 3 : 6);
+}
+
+// Estimated time of a contraction's launch on tiles of shape s, in
+// microseconds: what a launch costs at all, its rounds of tiles over the
+// resident CTAs or pairs (a last round that splits K counting half), and the
+// ends of tiles that no other tile's MMAs cover.  `lower`: symmetric product;
+// `c_tma`: TMA can address C's rows (else a pair's only tile ends like every
+// other one: 256 x 256 tiles 4 to 7 us later, a split one's handoff 10 us).
+// Checked on GB300 against bf16x3, fp16x3, tf32x3, bf16x6 and tf32 on sixteen
+// shapes and ten symmetric ones: the shape chosen is within 5 % of the fastest.
+double tile_cost(gbpoly_ctx* ctx, gbpoly_precision prec, TileShape s, int64_t M, int64_t N, int64_t K, int pairings,
+    bool lower, bool c_tma) {
+  const Elem e = prec == GBPOLY_PREC_FP16X3                                          ? Elem::F16
+                 : (prec == GBPOLY_PREC_TF32 || prec == GBPOLY_PREC_TF32X3) ? Elem::TF32
+                                                                                     : Elem::BF16;
+  const int terms = prec == GBPOLY_PREC_BF16X6 ? 3 : (prec == GBPOLY_PREC_TF32 ? 1 : 2);
+  const int64_t bk = e == Elem::TF32 ? 32 : 64;
+  const int64_t bm = s == kTileSquare ? 128 : 256, bn = s == kTilePair ? 256 : 128;
+  const int64_t tm = (M + bm - 1) / bm, tn = (N + bn - 1) / bn;
+  const int64_t tiles = !lower ? tm * tn : (s == kTileNarrow ? lower_tiles<256, 128>(tm, tn) : tm * (tm + 1) / 2);
+  const int64_t chunks = std::max<int64_t>(1, (K + bk - 1) / bk) * pairings;
+  const int64_t cap = std::max(1, s == kTileSquare ? ctx->sm_count : ctx->sm_count / 2);
+  const double c = chunk_us(e, terms, s);
+  const int64_t full = tiles / cap, rest = tiles % cap;
+  const double handoff = full ? kHandoffLastRoundUs : (c_tma ? kHandoffUs : 10);
+  const bool split = s != kTileSquare && ctx->tail_split && rest > 0 && 2 * rest <= cap && full < kTailMaxRounds &&
+                     double(chunks / 2) * c >= (full ? kHandoffLastRoundUs : kHandoffUs);
+  const double rounds = double(full) + (rest == 0 ? 0.0 : (split ? 0.5 : 1.0));
+  const double ends = double(full + (rest > 0) - 1);  // exposed tile ends before the last
+  double t = (s == kTileSquare ? 9 : 11) + rounds * double(chunks) * c + (split ? handoff : 0);
+  t += ends * (s == kTileSquare ? 1 : (s == kTilePair ? 9 : 6));
+  const bool staged = ends > 0 || !c_tma;  // the last tile's C
+  if(lower && s == kTilePair) t += staged ? 8 * (ends + 1) : 3;  // mirrored C of a 256 x 256 tile
+  if(!c_tma && ends == 0) t += s == kTilePair ? 7 : (s == kTileNarrow ? 3 : 0);
+  return t;
+}
+
+int cheapest_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K, int pairings, bool lower,
+    bool c_tma) {
+  TileShape best = kTileSquare;
+  double best_t = 0;
+  for(TileShape s : {kTileSquare, kTilePair, kTileNarrow}) {
+    const double t = tile_cost(ctx, prec, s, M, N, K, pairings, lower, c_tma);
+    if(s == kTileSquare || t < best_t) best = s, best_t = t;
+  }
+  return config_of(prec, best);
+}
+
+int square_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t N, int64_t K, int pairings, bool c_tma) {
   if(prec == GBPOLY_PREC_FP8) return 0;
-  const int64_t t = (N + 255) / 256;
-  if(prec == GBPOLY_PREC_FP16X3) return pairs_fill(ctx, t * (t + 1) / 2) ? 2 : 1;
-  if(pairs_fill(ctx, t * (t + 1) / 2)) return 3;
-  return prec == GBPOLY_PREC_BF16X6 ? 1 : 2;
+  return cheapest_config(ctx, prec, N, N, K, pairings, true, c_tma);
 }
 }  // namespace
 
@@ -1717,28 +1991,29 @@ int square_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t N) {
 // fill the device, with the C tile in shared memory (configuration 5) while
 // K is short enough that C's traffic bounds the call (measured on GB300 at
 // M = N = 8192: 1.75x faster up to K = 128, ahead up to K = 256 for the
-// BF16 forms and K = 512 for tf32, behind beyond), else the 1-CTA
-// configuration with the most tiles.
-int default_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K) {
+// BF16 forms and K = 512 for tf32, behind beyond), else the tile shape of the
+// least estimated time (bf16x3, us, chosen / 128 x 128 tiles: 2048 cubed 52 /
+// 69, 256 x 4096 x 4096 65 / 81, 4096 x 1024 x 512 25 / 29).
+int default_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K, bool c_tma) {
   // fp8: 128 x 256 tiles (twice the MMA work per scaled chunk: 1.38x at
   // N = 8192) when they give every SM a tile, else 128 x 128
   if(prec == GBPOLY_PREC_FP8) return ((M + 127) / 128) * ((N + 255) / 256) >= ctx->sm_count ? 1 : 0;
-  // fp16x3: CTA pairs when they fill the device, else 128 x 128 tiles
-  if(prec == GBPOLY_PREC_FP16X3) return pairs_fill(ctx, ((M + 255) / 256) * ((N + 255) / 256)) ? 2 : 1;
   if(tensor_config_count(prec) <= 3) return 0;
   if(pairs_fill(ctx, ((M + 255) / 256) * ((N + 255) / 256))) {
+    if(prec == GBPOLY_PREC_FP16X3) return 2;
     const int64_t k_tile = prec == GBPOLY_PREC_TF32 ? 512 : (prec == GBPOLY_PREC_TF32X3 ? 128 : 256);
     return K <= k_tile ? 5 : 3;
   }
-  // 128 x 128 tiles: configuration 2 (0 for bf16x6, whose configuration 0 is 128 x 128)
-  return prec == GBPOLY_PREC_BF16X6 ? 0 : 2;
+  return cheapest_config(ctx, prec, M, N, K, 1, false, c_tma);
 }
 
-gbpoly_status tensor_plan(gbpoly_ctx* ctx, gbpoly_precision prec, gbpoly_op, gbpoly_op, int64_t M, int64_t N,
-    int64_t K, TensorPlan* plan) {
+gbpoly_status tensor_plan(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K, const float* C,
+    int64_t ldc, TensorPlan* plan) {
   if(tensor_config_count(prec) == 0) return fail(GBPOLY_ERR_UNSUPPORTED, "precision form not available");
   plan->prec = prec;
-  plan->config = tuned_config(ctx, prec, M, N, K);
+  GemmF32Args a{};
+  a.N = N, a.C = const_cast<float*>(C), a.ldc = ldc;
+  plan->config = tuned_config(ctx, prec, M, N, K, c_tile_ok(a));
   plan->M = M;
   return GBPOLY_OK;
 }
@@ -1751,38 +2026,44 @@ gbpoly_status tensor_plan_panel(gbpoly_ctx* ctx, const TensorPlan& plan, const G
   case GBPOLY_PREC_TF32 * 8 + 3:
   case GBPOLY_PREC_TF32 * 8 + 5: return run_form_panel<FormTF32_p>(ctx, a, plan.M, first, r0, "tf32_gemm");
   case GBPOLY_PREC_TF32 * 8 + 4: return run_form_panel<FormTF32_q>(ctx, a, plan.M, first, r0, "tf32_gemm");
+  case GBPOLY_PREC_TF32 * 8 + 6: return run_form_panel<FormTF32_n>(ctx, a, plan.M, first, r0, "tf32_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 0: return run_form_panel<FormBF16x3>(ctx, a, plan.M, first, r0, "bf16x3_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 1: return run_form_panel<FormBF16x3_b>(ctx, a, plan.M, first, r0, "bf16x3_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 2: return run_form_panel<FormBF16x3_c>(ctx, a, plan.M, first, r0, "bf16x3_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 3:
   case GBPOLY_PREC_BF16X3 * 8 + 5: return run_form_panel<FormBF16x3_p>(ctx, a, plan.M, first, r0, "bf16x3_gemm");
   case GBPOLY_PREC_BF16X3 * 8 + 4: return run_form_panel<FormBF16x3_q>(ctx, a, plan.M, first, r0, "bf16x3_gemm");
+  case GBPOLY_PREC_BF16X3 * 8 + 6: return run_form_panel<FormBF16x3_n>(ctx, a, plan.M, first, r0, "bf16x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 0: return run_form_panel<FormTF32x3>(ctx, a, plan.M, first, r0, "tf32x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 1: return run_form_panel<FormTF32x3_b>(ctx, a, plan.M, first, r0, "tf32x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 2: return run_form_panel<FormTF32x3_c>(ctx, a, plan.M, first, r0, "tf32x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 3:
   case GBPOLY_PREC_TF32X3 * 8 + 5: return run_form_panel<FormTF32x3_p>(ctx, a, plan.M, first, r0, "tf32x3_gemm");
   case GBPOLY_PREC_TF32X3 * 8 + 4: return run_form_panel<FormTF32x3_q>(ctx, a, plan.M, first, r0, "tf32x3_gemm");
+  case GBPOLY_PREC_TF32X3 * 8 + 6: return run_form_panel<FormTF32x3_n>(ctx, a, plan.M, first, r0, "tf32x3_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 0: return run_form_panel<FormBF16x6>(ctx, a, plan.M, first, r0, "bf16x6_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 1: return run_form_panel<FormBF16x6_b>(ctx, a, plan.M, first, r0, "bf16x6_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 2: return run_form_panel<FormBF16x6_c>(ctx, a, plan.M, first, r0, "bf16x6_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 3:
   case GBPOLY_PREC_BF16X6 * 8 + 5: return run_form_panel<FormBF16x6_p>(ctx, a, plan.M, first, r0, "bf16x6_gemm");
   case GBPOLY_PREC_BF16X6 * 8 + 4: return run_form_panel<FormBF16x6_q>(ctx, a, plan.M, first, r0, "bf16x6_gemm");
+  case GBPOLY_PREC_BF16X6 * 8 + 6: return run_form_panel<FormBF16x6_n>(ctx, a, plan.M, first, r0, "bf16x6_gemm");
   case GBPOLY_PREC_FP8 * 8 + 0: return run_fp8<FormFP8>(ctx, a);  // quantises both operands per panel
   case GBPOLY_PREC_FP8 * 8 + 1: return run_fp8<FormFP8_w>(ctx, a);
   // fp16x3: split both operands (and their block scales) per panel
   case GBPOLY_PREC_FP16X3 * 8 + 0: return run_form<FormF16x3>(ctx, a, "fp16x3_gemm");
   case GBPOLY_PREC_FP16X3 * 8 + 1: return run_form<FormF16x3_c>(ctx, a, "fp16x3_gemm");
   case GBPOLY_PREC_FP16X3 * 8 + 2: return run_form<FormF16x3_p>(ctx, a, "fp16x3_gemm");
+  case GBPOLY_PREC_FP16X3 * 8 + 3: return run_form<FormF16x3_n>(ctx, a, "fp16x3_gemm");
   default: return fail(GBPOLY_ERR_UNSUPPORTED, "precision form or tile configuration not available");
   }
 }
 
 gbpoly_status launch_gemm_tensor(gbpoly_ctx* ctx, gbpoly_precision prec, const GemmF32Args& a) {
-  int config = tuned_config(ctx, prec, a.M, a.N, a.K);
+  int config = tuned_config(ctx, prec, a.M, a.N, a.K, c_tile_ok(a));
   const bool symmetric = (same_operand(a) || a.dual) && a.M == a.N;
-  if(symmetric && !config_is_square(prec, config)) config = square_config(ctx, prec, a.N);
+  if(symmetric && (!config_is_square(prec, config) || !is_tuned(ctx, prec, a.M, a.N, a.K)))
+    config = square_config(ctx, prec, a.N, a.K, a.dual ? 2 : 1, c_tile_ok(a));
   if(config == 5 && !c_tile_ok(a)) config = 3;  // C rows TMA cannot address: the staged epilogue
   return launch_gemm_tensor_config(ctx, prec, config, a);
 }
