@@ -65,6 +65,7 @@ template <bool CENTERED>
 __global__ void __launch_bounds__(kWarps * 32) column_partial_kernel(const float* __restrict__ X, int64_t ldx, int rows,
     int cols, int rows_per_chunk, const float* __restrict__ mean, float* __restrict__ partial) {
   __shared__ float red[kWarps][kColsPerBlock + 1];
+  pdl_enter();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = blockIdx.x * kColsPerBlock + lane;
   const int r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(kWarps * 32) column_partial_kernel(const float
 template <bool STDDEV>
 __global__ void column_final_kernel(const float* __restrict__ partial, int chunks, int cols, float divisor, float eps,
     float* __restrict__ out) {
+  pdl_enter();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if(j >= cols) return;
   float s = 0.f;
@@ -102,6 +104,7 @@ template <bool SCALED>
 __global__ void __launch_bounds__(256) center_columns_kernel(const float* X, int64_t ldx, int rows, int cols,
     const float* __restrict__ mean, const float* __restrict__ stddev, float scale_div, float* Y, int64_t ldy,
     int rows_per_block) {
+  pdl_enter();
   const int j = blockIdx.x * 32 + (threadIdx.x & 31);
   if(j >= cols) return;
   const float m = mean[j];
@@ -128,6 +131,7 @@ __global__ void __launch_bounds__(256) center_columns_kernel(const float* X, int
 }
 
 __global__ void set_diagonal_kernel(int64_t n, float value, float* C, int64_t ldc) {
+  pdl_enter();
   for(int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     C[i * ldc + i] = value;
 }
@@ -163,14 +167,12 @@ gbpoly_status column_reduce(gbpoly_ctx* ctx, int64_t rows, int64_t cols, const f
   float* partial = static_cast<float*>(ctx->stats.ptr);
   {
     ProfileScope prof(ctx, STDDEV ? "column_sumsq" : "column_sum");
-    column_partial_kernel<STDDEV><<<dim3(unsigned(col_blocks), unsigned(chunks)), kWarps * 32, 0, ctx->stream>>>(
-        X, ldx, int(rows), int(cols), std::max(rows_per_chunk, 1), mean, partial);
-    GBPOLY_CUDA_TRY(cudaGetLastError());
+    GBPOLY_CUDA_TRY(launch_pdl(ctx, column_partial_kernel<STDDEV>, dim3(unsigned(col_blocks), unsigned(chunks)),
+        kWarps * 32, 0, X, ldx, int(rows), int(cols), std::max(rows_per_chunk, 1), mean, partial));
   }
   ProfileScope prof(ctx, STDDEV ? "column_stddev_final" : "column_mean_final");
-  column_final_kernel<STDDEV><<<unsigned((cols + 255) / 256), 256, 0, ctx->stream>>>(partial, int(rows > 0 ? chunks : 0),
-      int(cols), divisor, eps, out);
-  GBPOLY_CUDA_TRY(cudaGetLastError());
+  GBPOLY_CUDA_TRY(launch_pdl(ctx, column_final_kernel<STDDEV>, unsigned((cols + 255) / 256), 256, 0, partial,
+      int(rows > 0 ? chunks : 0), int(cols), divisor, eps, out));
   return GBPOLY_OK;
 }
 
@@ -213,12 +215,11 @@ gbpoly_status gbpoly_center_columns_f32(gbpoly_ctx* ctx, int64_t rows, int64_t c
   if(grid.y > 65535u) return fail(GBPOLY_ERR_UNSUPPORTED, "too many rows");
   ProfileScope prof(ctx, stddev ? "normalize_columns" : "center_columns");
   if(stddev)
-    center_columns_kernel<true><<<grid, 256, 0, ctx->stream>>>(X, ldx, int(rows), int(cols), mean, stddev, scale_div, Y,
-        ldy, kRowsPerBlock);
+    GBPOLY_CUDA_TRY(launch_pdl(ctx, center_columns_kernel<true>, grid, 256, 0, X, ldx, int(rows), int(cols), mean, stddev,
+        scale_div, Y, ldy, kRowsPerBlock));
   else
-    center_columns_kernel<false><<<grid, 256, 0, ctx->stream>>>(X, ldx, int(rows), int(cols), mean, nullptr, 1.f, Y,
-        ldy, kRowsPerBlock);
-  GBPOLY_CUDA_TRY(cudaGetLastError());
+    GBPOLY_CUDA_TRY(launch_pdl(ctx, center_columns_kernel<false>, grid, 256, 0, X, ldx, int(rows), int(cols), mean,
+        nullptr, 1.f, Y, ldy, kRowsPerBlock));
   return GBPOLY_OK;
 }
 
@@ -261,8 +262,8 @@ gbpoly_status gbpoly_set_diagonal_f32(gbpoly_ctx* ctx, int64_t n, float value, f
   if((st = check_block("C", C, n, n, ldc)) != GBPOLY_OK) return st;
   if(n == 0) return GBPOLY_OK;
   ProfileScope prof(ctx, "set_diagonal");
-  set_diagonal_kernel<<<unsigned(std::min<int64_t>((n + 255) / 256, 4096)), 256, 0, ctx->stream>>>(n, value, C, ldc);
-  GBPOLY_CUDA_TRY(cudaGetLastError());
+  GBPOLY_CUDA_TRY(launch_pdl(ctx, set_diagonal_kernel, unsigned(std::min<int64_t>((n + 255) / 256, 4096)), 256, 0, n,
+      value, C, ldc));
   return GBPOLY_OK;
 }
 

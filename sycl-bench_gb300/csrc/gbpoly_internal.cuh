@@ -16,6 +16,7 @@
 #include <map>
 #include <string>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "../../include/gbpoly.h"
@@ -232,7 +233,36 @@ gbpoly_status grouped_plan_config(gbpoly_ctx* ctx, gbpoly_precision prec, const 
 // Workspace bytes launch_gemm_tensor needs for this shape (0 for FP32).
 size_t workspace_bytes(gbpoly_precision prec, int64_t M, int64_t N, int64_t K, bool same_operand);
 
+// Launch on the context's stream so that the kernel's CTAs may become resident
+// while the kernel queued before it still runs (programmatic stream
+// serialization).  Every kernel launched this way calls pdl_trigger and then,
+// before it touches global memory, pdl_wait, which returns when all earlier
+// work of the stream has completed: what overlaps is launch latency and the
+// set-up of shared and tensor memory, never data.
+template <class... Params, class... Args>
+cudaError_t launch_pdl(gbpoly_ctx* ctx, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
 // ---------------------------------------------------------------- device side
+
+// launch_pdl: the next kernel of the stream may become resident; wait for the earlier ones.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter() {
+  pdl_trigger();
+  pdl_wait();
+}
 
 constexpr unsigned long long kWaitTimeoutNs = 2000000000ull;  // 2 s
 

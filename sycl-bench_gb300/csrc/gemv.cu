@@ -86,6 +86,7 @@ __device__ __forceinline__ float reduce_rows(float (&v)[V], int lane) {
 template <int NR, bool NC, bool TWO, bool VEC>
 __global__ void __launch_bounds__(kThreads, 2) gemv_partial_kernel(const GemvArgs g) {
   __shared__ float red[NR > 0 ? NR : 1][kThreads / 32][kRowBlock];
+  pdl_enter();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tile = blockIdx.x;
   const int c = tile * kTileCols + 4 * tid;
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(256) gemv_final_kernel(const float* __restrict
     const float* __restrict__ col_part, int row_groups, int cols, Term r0, Term r1, Term cterm) {
   constexpr int kSums = (NR > 0 ? NR : 0) + (NC ? 1 : 0);
   __shared__ float red[kSums > 0 ? kSums : 1][8][32];
+  pdl_enter();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
   if constexpr(NR > 0) {
@@ -252,18 +254,16 @@ gbpoly_status launch_gemv(gbpoly_ctx* ctx, GemvArgs g, Term r0, Term r1, Term ct
     ProfileScope prof(ctx, name);
     const dim3 grid{unsigned(col_tiles), unsigned(row_groups), 1u};
     if(vec)
-      gemv_partial_kernel<NR, NC, TWO, true><<<grid, kThreads, 0, ctx->stream>>>(g);
+      GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_partial_kernel<NR, NC, TWO, true>, grid, kThreads, 0, g));
     else
-      gemv_partial_kernel<NR, NC, TWO, false><<<grid, kThreads, 0, ctx->stream>>>(g);
-    GBPOLY_CUDA_TRY(cudaGetLastError());
+      GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_partial_kernel<NR, NC, TWO, false>, grid, kThreads, 0, g));
   }
   const int n = std::max(g.rows, g.cols);
   if(n == 0) return GBPOLY_OK;
   ProfileScope prof(ctx, "gemv_final");
-  gemv_final_kernel<NR, NC, GESUMMV><<<unsigned((n + 31) / 32), 256, 0, ctx->stream>>>(g.row_part,
-      (g.rows > 0 && g.cols > 0) ? col_tiles : 0, g.rows, g.col_part, (g.rows > 0 && g.cols > 0) ? row_groups : 0,
-      g.cols, r0, r1, ct);
-  GBPOLY_CUDA_TRY(cudaGetLastError());
+  const bool some = g.rows > 0 && g.cols > 0;
+  GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_final_kernel<NR, NC, GESUMMV>, unsigned((n + 31) / 32), 256, 0, g.row_part,
+      some ? col_tiles : 0, g.rows, g.col_part, some ? row_groups : 0, g.cols, r0, r1, ct));
   return GBPOLY_OK;
 }
 
@@ -282,6 +282,7 @@ __global__ void __launch_bounds__(kThreads, 1) atax_kernel(const float* __restri
     const float* __restrict__ x, float* __restrict__ tmp, float* __restrict__ col_part, int groups) {
   __shared__ float red[kThreads / 32][kAtaxRows];
   __shared__ float tmp_s[kAtaxRows];
+  pdl_enter();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float4 xr[CHUNKS], colacc[CHUNKS];
 #pragma unroll
@@ -361,13 +362,11 @@ gbpoly_status launch_atax(gbpoly_ctx* ctx, const float* A, int64_t lda, int rows
   float* col_part = static_cast<float*>(ctx->stats.ptr);
   {
     ProfileScope prof(ctx, "atax");
-    atax_kernel<CHUNKS><<<grid, kThreads, 0, ctx->stream>>>(A, lda, rows, cols, x, tmp, col_part, groups);
-    GBPOLY_CUDA_TRY(cudaGetLastError());
+    GBPOLY_CUDA_TRY(launch_pdl(ctx, atax_kernel<CHUNKS>, grid, kThreads, 0, A, lda, rows, cols, x, tmp, col_part, groups));
   }
   ProfileScope prof(ctx, "gemv_final");
-  gemv_final_kernel<0, true, false><<<unsigned((cols + 31) / 32), 256, 0, ctx->stream>>>(nullptr, 0, rows, col_part,
-      grid, cols, Term{}, Term{}, Term{1.f, 1.f, y});
-  GBPOLY_CUDA_TRY(cudaGetLastError());
+  GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_final_kernel<0, true, false>, unsigned((cols + 31) / 32), 256, 0, nullptr, 0, rows,
+      col_part, grid, cols, Term{}, Term{}, Term{1.f, 1.f, y}));
   return GBPOLY_OK;
 }
 

@@ -239,7 +239,9 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
     }
     fence_mbar_init();
   }
+  pdl_trigger();
   __syncthreads();
+  pdl_wait();
 
   if(warp < kProducers / 32) {
     // ------------------------------------------------------------ producer
@@ -463,16 +465,18 @@ struct Kernel {
 
   struct Launch {
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     Launch(gbpoly_ctx* ctx, unsigned tiles, unsigned splits) {
       cfg.gridDim = dim3(tiles, splits);
       cfg.blockDim = dim3(kThreads);
       cfg.dynamicSmemBytes = kSmem;
       cfg.stream = ctx->stream;
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = splits, attr[0].val.clusterDim.z = 1;
+      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_pdl
+      attr[0].val.programmaticStreamSerializationAllowed = 1;
+      attr[1].id = cudaLaunchAttributeClusterDimension;
+      attr[1].val.clusterDim.x = 1, attr[1].val.clusterDim.y = splits, attr[1].val.clusterDim.z = 1;
       cfg.attrs = attr;
-      cfg.numAttrs = splits > 1 ? 1 : 0;
+      cfg.numAttrs = splits > 1 ? 2 : 1;
     }
   };
 };
@@ -492,6 +496,7 @@ gbpoly_status cluster_capacity(gbpoly_ctx* ctx, int (&cap)[kMaxSplit + 1]) {
   cap[1] = std::max(1, ctx->sm_count);
   for(int s = 2; s <= kMaxSplit; ++s) {
     typename K::Launch l(ctx, unsigned(ctx->sm_count), unsigned(s));
+    l.cfg.attrs = l.attr + 1, l.cfg.numAttrs = 1;  // the cluster size alone
     int n = 0;
     GBPOLY_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, K::fn, &l.cfg));
     cap[s] = n;  // 0: no cluster of this size

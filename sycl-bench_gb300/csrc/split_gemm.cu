@@ -471,32 +471,56 @@ __device__ __forceinline__ float block_pow2_scale(const float (&v)[16], float* i
   return __uint_as_float(uint32_t(127 + e) << 23);
 }
 
-// panel[t][r][k] (r < R, k < Kp) = term t of op(X)[r][k] for k < K, 0 beyond,
-// op(X)[r][k] = X[r*ld + k] (k_major) or X[k*ld + r].  Panels are Kp-strided
-// and `panel_stride` elements apart.  One 64 x 64 block per CTA.  F16 terms:
-// the block is scaled by a power of two first (block_pow2_scale) and its
-// inverse scale stored at inv_scale[blockIdx.y * gridDim.x + blockIdx.x].
+// One operand of the split pass: panel[t][r][k] (r < R, k < Kp) = term t of
+// op(X)[r][k] for k < K, 0 beyond, op(X)[r][k] = X[r*ld + k] (k_major) or
+// X[k*ld + r].  Panels are Kp-strided and `panel_stride` elements apart.  F16
+// terms: each 64 x 64 block is scaled by a power of two first
+// (block_pow2_scale) and its inverse scale stored in inv_scale[row block][k block].
+struct SplitSide {
+  const float* X;
+  int64_t ld;
+  int k_major, R;
+  void* out;
+  int64_t panel_stride;
+  RowXform xf;
+  float* inv_scale;
+};
+
+// Both operands of a contraction in one launch (with the kernels' set-up under
+// the one before, a 200 x 136 x 328 call takes 10.5 us instead of 18.4), one
+// 64 x 64 block per CTA:
+// blocks [0, blocks_a) are the left operand's, the rest the right one's, kb
+// along K.  The first CTA also clears the `nflags` counters of a K-split tail.
 template <Elem E, int TERMS>
-__global__ void __launch_bounds__(256) split_kernel(const float* __restrict__ X, int64_t ld, int k_major, int R, int K,
-    int Kp, typename Term<E>::T* __restrict__ out, int64_t panel_stride, RowXform xf, float* __restrict__ inv_scale) {
-  const int64_t r0 = int64_t(blockIdx.y) * 64, k0 = int64_t(blockIdx.x) * 64;
+__global__ void __launch_bounds__(256) split_kernel(const SplitSide a, const SplitSide b, int blocks_a, int kb, int K,
+    int* __restrict__ flags, int nflags) {
+  using T = typename Term<E>::T;
+  pdl_enter();
+  const bool left = int(blockIdx.x) < blocks_a;
+  const SplitSide& s = left ? a : b;
+  const int local = int(blockIdx.x) - (left ? 0 : blocks_a);
+  const int rb = local / kb, kbi = local - rb * kb;
+  const int64_t r0 = int64_t(rb) * 64, k0 = int64_t(kbi) * 64;
+  if(blockIdx.x == 0)
+    for(int i = threadIdx.x; i < nflags; i += 256) flags[i] = 0;
   float v[16];
-  if(k_major) {
-    split_load(X, ld, 1, R, K, r0, k0, v);
+  if(s.k_major) {
+    split_load(s.X, s.ld, 1, s.R, K, r0, k0, v);
   } else {
     float t[16];
-    split_load(X, ld, 0, R, K, r0, k0, t);
+    split_load(s.X, s.ld, 0, s.R, K, r0, k0, t);
     mn_to_kmajor(t, v);
   }
+  const int Kp = 64 * kb;
   if constexpr(E == Elem::F16) {
-    xform_kmajor(v, R, r0, k0, xf, K);
+    xform_kmajor(v, s.R, r0, k0, s.xf, K);
     __shared__ float red[8];
-    const float s = block_pow2_scale(v, inv_scale + int64_t(blockIdx.y) * gridDim.x + blockIdx.x, red);
+    const float sc = block_pow2_scale(v, s.inv_scale + local, red);
 #pragma unroll
-    for(int i = 0; i < 16; ++i) v[i] *= s;
-    split_convert_kmajor<E, TERMS>(v, out, panel_stride, R, Kp, r0, k0);
+    for(int i = 0; i < 16; ++i) v[i] *= sc;
+    split_convert_kmajor<E, TERMS>(v, static_cast<T*>(s.out), s.panel_stride, s.R, Kp, r0, k0);
   } else {
-    split_convert_kmajor<E, TERMS>(v, out, panel_stride, R, Kp, r0, k0, xf, K);
+    split_convert_kmajor<E, TERMS>(v, static_cast<T*>(s.out), s.panel_stride, s.R, Kp, r0, k0, s.xf, K);
   }
 }
 
@@ -522,6 +546,7 @@ template <Elem E, int TERMS>
 __global__ void __launch_bounds__(256, 4) grouped_split_kernel(const SplitJob* __restrict__ jobs,
     const int4* __restrict__ blocks, int nblocks) {
   using T = typename Term<E>::T;
+  pdl_enter();
   int b = blockIdx.x;
   if(b >= nblocks) return;
   int4 bl = blocks[b];
@@ -590,6 +615,7 @@ __device__ __forceinline__ uint16_t e4m3x2(float a, float b) {
 __global__ void __launch_bounds__(512, 2) quantize_e4m3_kernel(const QuantJob ja, const QuantJob jb, int blocks_a,
     int nblocks) {
   __shared__ float red[16];
+  pdl_enter();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for(int blk = blockIdx.x; blk < nblocks; blk += gridDim.x) {
     const bool first = blk < blocks_a;
@@ -867,6 +893,12 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
   else
     __syncthreads();
   umma::fence_after_sync();
+  // The panels (and whatever else the stream wrote before) are complete.  This
+  // kernel does not trigger the next one: CTAs of the next call's split pass,
+  // resident early on SMs between two tiles' CTAs, cost more than they saved
+  // (us with / without the trigger: grouped 64 problems 197 / 173, fp16x3
+  // 4096 x 3000 x 2560 178 / 168, syrk 4096 181 / 173).
+  pdl_wait();
   const uint32_t tmem = *tmem_slot;
 
   if(warp < 4) {
@@ -1446,16 +1478,31 @@ struct Panels {
 };
 
 template <class F>
-gbpoly_status launch_split(gbpoly_ctx* ctx, const float* X, int64_t ld, bool k_major, int64_t rows, int64_t K,
-    int64_t Kp, Panels out, RowXform xf = RowXform{}, float* inv_scale = nullptr) {
-  using T = typename Term<F::elem>::T;
-  dim3 grid(static_cast<unsigned>(Kp / 64), static_cast<unsigned>((rows + 63) / 64));
-  if(grid.y > 65535u) return fail(GBPOLY_ERR_UNSUPPORTED, "operand too large for the split pass (over 65535 row blocks)");
-  ProfileScope prof(ctx, "split_terms");
-  split_kernel<F::elem, F::terms><<<grid, 256, 0, ctx->stream>>>(X, ld, k_major ? 1 : 0, int(rows), int(K), int(Kp),
-      reinterpret_cast<T*>(out.base), int64_t(out.stride / sizeof(T)), xf, inv_scale);
-  GBPOLY_CUDA_TRY(cudaGetLastError());
+gbpoly_status check_split_rows(int64_t rows) {
+  if((rows + 63) / 64 > 65535)
+    return fail(GBPOLY_ERR_UNSUPPORTED, "operand too large for the split pass (over 65535 row blocks)");
   return GBPOLY_OK;
+}
+
+// The split pass over one (b == nullptr) or both operands; flags: counters to
+// clear for the contraction that follows.
+template <class F>
+gbpoly_status launch_split(gbpoly_ctx* ctx, const SplitSide& a, const SplitSide* b, int64_t K, int64_t Kp,
+    int* flags = nullptr, int nflags = 0) {
+  gbpoly_status st = check_split_rows<F>(a.R);
+  if(st != GBPOLY_OK || (b && (st = check_split_rows<F>(b->R)) != GBPOLY_OK)) return st;
+  const int64_t kb = Kp / 64, blocks_a = (a.R + 63) / 64 * kb, blocks = blocks_a + (b ? (b->R + 63) / 64 * kb : 0);
+  if(blocks >= (1ll << 31)) return fail(GBPOLY_ERR_UNSUPPORTED, "too many blocks for the split pass");
+  ProfileScope prof(ctx, "split_terms");
+  GBPOLY_CUDA_TRY(launch_pdl(ctx, split_kernel<F::elem, F::terms>, unsigned(blocks), 256, 0, a, b ? *b : a, int(blocks_a),
+      int(kb), int(K), flags, nflags));
+  return GBPOLY_OK;
+}
+
+template <class F>
+SplitSide split_side(const float* X, int64_t ld, bool k_major, int64_t rows, Panels out, RowXform xf = RowXform{},
+    float* inv_scale = nullptr) {
+  return SplitSide{X, ld, k_major ? 1 : 0, int(rows), out.base, int64_t(out.stride / F::esz), xf, inv_scale};
 }
 
 template <class F>
@@ -1501,7 +1548,7 @@ gbpoly_status tc_prepare(gbpoly_ctx* ctx) {
 template <class F>
 struct PairLaunch {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   PairLaunch(gbpoly_ctx* ctx, int clusters) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
@@ -1511,8 +1558,10 @@ struct PairLaunch {
     cfg.blockDim = dim3(F::THREADS);
     cfg.dynamicSmemBytes = F::SMEM;
     cfg.stream = ctx->stream;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_pdl
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
   }
 };
 
@@ -1529,6 +1578,7 @@ gbpoly_status pair_clusters(gbpoly_ctx* ctx, int& clusters) {
     return GBPOLY_OK;
   }
   PairLaunch<F> pl(ctx, ctx->sm_count / 2);
+  pl.cfg.numAttrs = 1;
   int n = 0;
   GBPOLY_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, split_gemm_kernel<F, S, false>, &pl.cfg));
   if(n <= 0) return fail(GBPOLY_ERR_UNSUPPORTED, "no CTA pair of this tensor-core configuration fits on the device");
@@ -1585,21 +1635,21 @@ gbpoly_status plan_tail(gbpoly_ctx* ctx, int64_t tiles, int64_t iters, TailPlan&
   return GBPOLY_OK;
 }
 
-// Point the scheduler at the tail's workspace (at `base`) and clear its counters.
+// Point the scheduler at the tail's workspace (at `base`), whose counters are
+// zero when the launch starts.
+int* tail_flags(const TailPlan& tp, char* base) {
+  return reinterpret_cast<int*>(base + size_t(tp.slots) * tp.slot_bytes);
+}
 template <class S>
-gbpoly_status apply_tail(gbpoly_ctx* ctx, const TailPlan& tp, char* base, S& sched) {
-  if(tp.slots == 0) return GBPOLY_OK;
+void apply_tail(const TailPlan& tp, char* base, S& sched) {
+  if(tp.slots == 0) return;
   sched.units = int(tp.units);
   sched.full_tiles = tp.full_tiles;
   sched.split_it = tp.split_it;
   sched.partial = reinterpret_cast<float*>(base);
-  sched.flags = reinterpret_cast<int*>(base + size_t(tp.slots) * tp.slot_bytes);
-  GBPOLY_CUDA_TRY(cudaMemsetAsync(sched.flags, 0, size_t(tp.slots) * sizeof(int), ctx->stream));
-  return GBPOLY_OK;
+  sched.flags = tail_flags(tp, base);
 }
 
-// Launch the tensor-core kernel for scheduler S: one persistent CTA (or CTA
-// pair) per SM (pair of SMs), walking `units` work units.
 template <class F, class S, bool RING>
 gbpoly_status launch_tc_variant(gbpoly_ctx* ctx, const S& sched, int64_t units, int resident, const char* kernel_name) {
   gbpoly_status st = tc_prepare<F, S, RING>(ctx);
@@ -1610,8 +1660,7 @@ gbpoly_status launch_tc_variant(gbpoly_ctx* ctx, const S& sched, int64_t units, 
     PairLaunch<F> pl(ctx, grid);
     GBPOLY_CUDA_TRY(cudaLaunchKernelEx(&pl.cfg, split_gemm_kernel<F, S, RING>, sched, ctx->err_dev));
   } else {
-    split_gemm_kernel<F, S, RING><<<grid, F::THREADS, F::SMEM, ctx->stream>>>(sched, ctx->err_dev);
-    GBPOLY_CUDA_TRY(cudaGetLastError());
+    GBPOLY_CUDA_TRY(launch_pdl(ctx, split_gemm_kernel<F, S, RING>, grid, F::THREADS, F::SMEM, sched, ctx->err_dev));
   }
   return GBPOLY_OK;
 }
@@ -1701,12 +1750,17 @@ gbpoly_status run_form(gbpoly_ctx* ctx, const GemmF32Args& a, const char* kernel
   float* const sa = F::elem == Elem::F16 ? reinterpret_cast<float*>(ws + a_bytes + b_bytes) : nullptr;
   float* const sb = same ? sa : (F::elem == Elem::F16 ? reinterpret_cast<float*>(ws + a_bytes + b_bytes + sa_bytes) : nullptr);
   if(a.K > 0 || F::elem == Elem::F16) {  // (F16: the split also writes the scales; with K = 0 they are 1)
-    if((st = launch_split<F>(ctx, a.A, a.lda, a.op_a == GBPOLY_OP_N, a.M, a.K, Kp, pa, a.xf, sa)) != GBPOLY_OK)
-      return st;
-    if(!same && (st = launch_split<F>(ctx, a.B, a.ldb, a.op_b == GBPOLY_OP_T, a.N, a.K, Kp, pb, RowXform{}, sb)) !=
-                    GBPOLY_OK)
+    const SplitSide left = split_side<F>(a.A, a.lda, a.op_a == GBPOLY_OP_N, a.M, pa, a.xf, sa);
+    const SplitSide right = split_side<F>(a.B, a.ldb, a.op_b == GBPOLY_OP_T, a.N, pb, RowXform{}, sb);
+    char* const tail_ws = ws + a_bytes + b_bytes + sa_bytes + sb_bytes;
+    if((st = launch_split<F>(ctx, left, same ? nullptr : &right, a.K, Kp, tail_flags(tail, tail_ws), tail.slots)) !=
+        GBPOLY_OK)
       return st;
   } else {
+    // (the tail's counters, which the split pass clears otherwise, too)
+    if(tail.slots > 0)
+      GBPOLY_CUDA_TRY(cudaMemsetAsync(tail_flags(tail, ws + a_bytes + b_bytes + sa_bytes + sb_bytes), 0,
+          size_t(tail.slots) * sizeof(int), ctx->stream));
     GBPOLY_CUDA_TRY(cudaMemsetAsync(ws, 0, a_bytes + b_bytes, ctx->stream));
   }
 
@@ -1730,7 +1784,7 @@ gbpoly_status run_form(gbpoly_ctx* ctx, const GemmF32Args& a, const char* kernel
   if(F::CEPI && (lower || !c_tile_ok(a)))
     return fail(GBPOLY_ERR_UNSUPPORTED, "C-tile epilogue: non-symmetric, 16-byte-aligned C");
   if((st = set_c_map<F>(ctx, a, sched)) != GBPOLY_OK) return st;
-  if((st = apply_tail(ctx, tail, ws + a_bytes + b_bytes + sa_bytes + sb_bytes, sched)) != GBPOLY_OK) return st;
+  apply_tail(tail, ws + a_bytes + b_bytes + sa_bytes + sb_bytes, sched);
   return launch_tc_kernel<F>(ctx, sched, tail.units, kernel_name);
 }
 
@@ -1761,8 +1815,7 @@ gbpoly_status run_fp8(gbpoly_ctx* ctx, const GemmF32Args& a) {
     if(blocks >= (1ll << 31)) return fail(GBPOLY_ERR_UNSUPPORTED, "too many quantisation blocks");
     // persistent: two CTAs per SM walk the blocks (no launch and drain per block)
     const unsigned ctas = unsigned(std::min<int64_t>(blocks, 2 * int64_t(std::max(1, ctx->sm_count))));
-    quantize_e4m3_kernel<<<ctas, 512, 0, ctx->stream>>>(ja, jb, int(blocks_a), int(blocks));
-    GBPOLY_CUDA_TRY(cudaGetLastError());
+    GBPOLY_CUDA_TRY(launch_pdl(ctx, quantize_e4m3_kernel, ctas, 512, 0, ja, jb, int(blocks_a), int(blocks)));
   }
   GemmMaps maps;
   int npair = 1;
@@ -1895,19 +1948,22 @@ gbpoly_status run_form_panel(gbpoly_ctx* ctx, const GemmF32Args& a, int64_t Mful
   char* ws = static_cast<char*>(ctx->ws.ptr);
   Panels pa{ws + size_t(r0) * lay.Kp * F::esz, lay.a_stride};
   Panels pb{ws + lay.a_bytes, lay.b_stride};
-  if(first && (st = launch_split<F>(ctx, a.B, a.ldb, a.op_b == GBPOLY_OP_T, a.N, a.K, lay.Kp, pb)) != GBPOLY_OK)
-    return st;
-  if((st = launch_split<F>(ctx, a.A, a.lda, a.op_a == GBPOLY_OP_N, a.M, a.K, lay.Kp, pa)) != GBPOLY_OK) return st;
-  GemmMaps maps;
-  if((st = make_product_maps<F>(ctx, maps.p[0], pa, a.M, pb, a.N, lay.Kp)) != GBPOLY_OK) return st;
-  maps.p[1] = maps.p[0];
-  Sched sched{maps, 1, int(a.M), int(a.N), int(lay.Kp), a.alpha, a.beta, a.C, a.ldc};
   int64_t tiles = ((a.M + F::BM - 1) / F::BM) * ((a.N + F::BN - 1) / F::BN);
   if(tail.slots > 0) {
     tail.slots = int(tiles);
     tail.units = tiles = 2 * tiles;
-    if((st = apply_tail(ctx, tail, ws + lay.a_bytes + lay.b_bytes, sched)) != GBPOLY_OK) return st;
   }
+  char* const tail_ws = ws + lay.a_bytes + lay.b_bytes;
+  const SplitSide left = split_side<F>(a.A, a.lda, a.op_a == GBPOLY_OP_N, a.M, pa);
+  const SplitSide right = split_side<F>(a.B, a.ldb, a.op_b == GBPOLY_OP_T, a.N, pb);
+  if((st = launch_split<F>(ctx, left, first ? &right : nullptr, a.K, lay.Kp, tail_flags(tail, tail_ws), tail.slots)) !=
+      GBPOLY_OK)
+    return st;
+  GemmMaps maps;
+  if((st = make_product_maps<F>(ctx, maps.p[0], pa, a.M, pb, a.N, lay.Kp)) != GBPOLY_OK) return st;
+  maps.p[1] = maps.p[0];
+  Sched sched{maps, 1, int(a.M), int(a.N), int(lay.Kp), a.alpha, a.beta, a.C, a.ldc};
+  apply_tail(tail, tail_ws, sched);
   if((st = set_c_map<F>(ctx, a, sched)) != GBPOLY_OK) return st;
   return launch_tc_kernel<F>(ctx, sched, tiles, name);
 }
@@ -2202,8 +2258,8 @@ gbpoly_status run_grouped(gbpoly_ctx* ctx, gbpoly_grouped* g, const char* name) 
     ProfileScope prof(ctx, "grouped_split");
     // persistent: 4 CTAs per SM
     const int ctas = std::min(g->split_blocks, 4 * std::max(1, ctx->sm_count));
-    grouped_split_kernel<F::elem, F::terms><<<ctas, 256, 0, ctx->stream>>>(g->jobs, g->split_table, g->split_blocks);
-    GBPOLY_CUDA_TRY(cudaGetLastError());
+    GBPOLY_CUDA_TRY(launch_pdl(ctx, grouped_split_kernel<F::elem, F::terms>, ctas, 256, 0, g->jobs, g->split_table,
+        g->split_blocks));
   }
   (void)sizeof(T);
   GroupedSched<F::BM, F::BN> sched{g->probs, g->maps, g->tiles, g->ntiles};
@@ -2493,9 +2549,9 @@ gbpoly_status launch_gemm_bf16x3_noalloc(gbpoly_ctx* ctx, const GemmF32Args& a) 
   Panels pb = same ? pa : Panels{ws + lay.a_bytes, lay.b_stride};
   if(a.K > 0) {
     // the split pass writes every panel element it is read from (zero K padding included)
-    if((st = launch_split<F>(ctx, a.A, a.lda, a.op_a == GBPOLY_OP_N, a.M, a.K, lay.Kp, pa)) != GBPOLY_OK) return st;
-    if(!same && (st = launch_split<F>(ctx, a.B, a.ldb, a.op_b == GBPOLY_OP_T, a.N, a.K, lay.Kp, pb)) != GBPOLY_OK)
-      return st;
+    const SplitSide left = split_side<F>(a.A, a.lda, a.op_a == GBPOLY_OP_N, a.M, pa);
+    const SplitSide right = split_side<F>(a.B, a.ldb, a.op_b == GBPOLY_OP_T, a.N, pb);
+    if((st = launch_split<F>(ctx, left, same ? nullptr : &right, a.K, lay.Kp)) != GBPOLY_OK) return st;
   } else {
     GBPOLY_CUDA_TRY(cudaMemsetAsync(ws, 0, need, ctx->stream));  // the array keeps the previous call's panels
   }

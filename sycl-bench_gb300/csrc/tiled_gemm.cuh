@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(64) tiled_gemm_kernel(int64_t M, int64_t N, in
   constexpr int TILE = kTiledTile, R = TILE / 8, BK = 16;  // R x R outputs per thread (8 x 8 threads)
   __shared__ T As[BK][TILE + 1];
   __shared__ T Bs[BK][TILE + 1];
+  pdl_enter();
   int64_t tm = blockIdx.x / tiles_n, tn = blockIdx.x - tm * tiles_n;
   if(lower) {  // row-major walk of the lower triangle: t = tm (tm + 1) / 2 + tn
     const int64_t t = blockIdx.x;
@@ -110,9 +111,8 @@ gbpoly_status launch_tiled_gemm(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K
   const int64_t tiles = lower ? gy * (gy + 1) / 2 : gx * gy;
   if(tiles >= (1ll << 31)) return fail(GBPOLY_ERR_UNSUPPORTED, "matrix too large for the tiled kernel grid");
   ProfileScope prof(ctx, sizeof(T) == 8 ? "dgemm_tiled" : "sgemm_tiled");
-  tiled_gemm_kernel<T><<<unsigned(tiles), 64, 0, ctx->stream>>>(M, N, K, alpha, a, b, dual, a2, b2, beta, C, ldc, lower,
-      gx);
-  GBPOLY_CUDA_TRY(cudaGetLastError());
+  GBPOLY_CUDA_TRY(launch_pdl(ctx, tiled_gemm_kernel<T>, unsigned(tiles), 64, 0, M, N, K, alpha, a, b, dual, a2, b2, beta,
+      C, ldc, lower, gx));
   return GBPOLY_OK;
 }
 
