@@ -6,16 +6,18 @@
 // column (polybench/atax.cpp:73-97, bicg.cpp:77-100, mvt.cpp:75-98,
 // gesummv.cpp:84-98).  Here one pass over the matrix serves up to two row
 // dots (y = A x, or A x and B x for gesummv) and one column sum (A^T v):
-//   * a CTA of 256 threads owns a 1024-column tile (4 adjacent columns per
-//     thread, 128-bit loads) and a group of rows; each row of the tile is one
-//     coalesced 4 KB read, 16 rows in flight per thread (8 per matrix for two);
+//   * a CTA of 256 threads owns a 1024-column tile (per thread 4 adjacent
+//     columns, one 128-bit load, where rows are 16-byte aligned; else columns
+//     t, t + 256, ..., four 32-bit loads of adjacent lanes) and a group of
+//     rows; each row of the tile is one coalesced 4 KB read, 16 rows in flight
+//     per thread (8 per matrix for two);
 //   * row dots: a thread's 4 columns give one term per row; each group of 8
 //     rows in flight is reduced across the warp at once (a halving transpose
 //     exchange: 16 shuffles for 16 rows), the 8 warps in shared memory per
 //     32-row block, into one partial per (column tile, row);
 //   * column sums: 4 accumulators per thread over all rows of the group,
 //     one partial per (row group, column);
-//   * a final kernel (8 warps per 32 outputs) adds the partials in a fixed order and applies
+//   * a final kernel (16 warps per 32 outputs) adds the partials in a fixed order and applies
 //     y = beta * y + alpha * sum (gesummv: tmp += A x, y = alpha tmp + beta (y + B x)).
 // Deterministic: the summation tree depends only on the shape and SM count.
 #include "gbpoly_internal.cuh"
@@ -45,14 +47,34 @@ struct GemvArgs {
   int col_tiles, rows_per_group;
 };
 
-__device__ __forceinline__ float4 load4(const float* p, int c, int cols, bool vec) {
-  if(vec) return *reinterpret_cast<const float4*>(p + c);
-  float4 v;
-  v.x = c < cols ? p[c] : 0.f;
-  v.y = c + 1 < cols ? p[c + 1] : 0.f;
-  v.z = c + 2 < cols ? p[c + 2] : 0.f;
-  v.w = c + 3 < cols ? p[c + 3] : 0.f;
-  return v;
+// The four columns of thread t in a 1024-column tile starting at c0: 4 t .. + 3
+// (VEC), or t, t + 256, t + 512, t + 768, so that every 32-bit load of a warp is
+// one 128-byte segment (measured with odd rows: bicg 6990 x 12897 70.8 -> YY us,
+// gesummv 8434 x 6453 89.5 -> YY, against 4 t .. + 3 in both cases).
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float* __restrict__ p, int c0, int cols) {
+  const int t = threadIdx.x;
+  if constexpr(VEC) {
+    const int c = c0 + 4 * t;
+    return c < cols ? *reinterpret_cast<const float4*>(p + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  const int c = c0 + t;
+  return make_float4(c < cols ? p[c] : 0.f, c + 256 < cols ? p[c + 256] : 0.f, c + 512 < cols ? p[c + 512] : 0.f,
+      c + 768 < cols ? p[c + 768] : 0.f);
+}
+template <bool VEC>
+__device__ __forceinline__ void store4(float* __restrict__ p, int c0, int cols, float4 v) {
+  const int t = threadIdx.x;
+  if constexpr(VEC) {
+    const int c = c0 + 4 * t;
+    if(c < cols) *reinterpret_cast<float4*>(p + c) = v;
+    return;
+  }
+  const int c = c0 + t;
+  if(c < cols) p[c] = v.x;
+  if(c + 256 < cols) p[c + 256] = v.y;
+  if(c + 512 < cols) p[c + 512] = v.z;
+  if(c + 768 < cols) p[c + 768] = v.w;
 }
 
 __device__ __forceinline__ float dot4(float4 a, float4 x) {
@@ -89,14 +111,13 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_partial_kernel(const GemvArg
   pdl_enter();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tile = blockIdx.x;
-  const int c = tile * kTileCols + 4 * tid;
-  const bool col_ok = c < g.cols;
+  const int c0 = tile * kTileCols;
   const int rg0 = blockIdx.y * g.rows_per_group;
   const int rg1 = min(g.rows, rg0 + g.rows_per_group);
 
   float4 xr[NR > 0 ? NR : 1];
 #pragma unroll
-  for(int t = 0; t < NR; ++t) xr[t] = col_ok ? load4(g.xr[t], c, g.cols, VEC) : make_float4(0.f, 0.f, 0.f, 0.f);
+  for(int t = 0; t < NR; ++t) xr[t] = load4<VEC>(g.xr[t], c0, g.cols);
   float4 colacc = make_float4(0.f, 0.f, 0.f, 0.f);
 
   constexpr int kInFlight = rows_in_flight<TWO>();
@@ -109,9 +130,9 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_partial_kernel(const GemvArg
 #pragma unroll
       for(int k = 0; k < kInFlight; ++k) {
         const int r = r0 + rr + k;
-        const bool ok = col_ok && r < rg1;
-        a[k] = ok ? load4(g.A + int64_t(r) * g.lda, c, g.cols, VEC) : make_float4(0.f, 0.f, 0.f, 0.f);
-        if constexpr(TWO) b[k] = ok ? load4(g.B + int64_t(r) * g.ldb, c, g.cols, VEC) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const bool ok = r < rg1;
+        a[k] = ok ? load4<VEC>(g.A + int64_t(r) * g.lda, c0, g.cols) : make_float4(0.f, 0.f, 0.f, 0.f);
+        if constexpr(TWO) b[k] = ok ? load4<VEC>(g.B + int64_t(r) * g.ldb, c0, g.cols) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for(int t = 0; t < NR; ++t) {
@@ -145,17 +166,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_partial_kernel(const GemvArg
       __syncthreads();
     }
   }
-  if constexpr(NC) {
-    float* out = g.col_part + int64_t(blockIdx.y) * g.cols;
-    if(VEC && c + 3 < g.cols) {
-      *reinterpret_cast<float4*>(out + c) = colacc;
-    } else {
-      if(c < g.cols) out[c] = colacc.x;
-      if(c + 1 < g.cols) out[c + 1] = colacc.y;
-      if(c + 2 < g.cols) out[c + 2] = colacc.z;
-      if(c + 3 < g.cols) out[c + 3] = colacc.w;
-    }
-  }
+  if constexpr(NC) store4<VEC>(g.col_part + int64_t(blockIdx.y) * g.cols, c0, g.cols, colacc);
 }
 
 struct Term {
@@ -169,42 +180,41 @@ __device__ __forceinline__ float apply(const Term& t, float s, int i) {
 }
 
 // Final pass, one CTA per 32 outputs: warp w adds the partials with index
-// w, w + 8, ... of output (blockIdx.x * 32 + lane); the 8 warp sums are
-// combined in shared memory in warp order.
+// w, w + 16, ... of output (blockIdx.x * 32 + lane), eight loads in flight; the
+// 16 warp sums are combined in shared memory in warp order.
 //   row terms:   y_r[i] = beta y_r[i] + alpha sum over column tiles of row_part[t][.][i]
 //   column term: y_c[j] = beta y_c[j] + alpha sum over row groups of col_part[.][j]
 //   GESUMMV:     tmp += S0, y = alpha tmp + beta (y + S1) (row terms 0, 1)
+constexpr int kFinalWarps = 16;
+
+// Sum over p[g * stride], g = warp, warp + 16, ... < n.
+__device__ __forceinline__ float strided_sum(const float* __restrict__ p, int64_t stride, int n, int warp) {
+  constexpr int kLoads = 8;
+  float s[kLoads];
+#pragma unroll
+  for(int k = 0; k < kLoads; ++k) s[k] = 0.f;
+  for(int g = warp; g < n; g += kLoads * kFinalWarps) {
+#pragma unroll
+    for(int k = 0; k < kLoads; ++k) {
+      const int i = g + k * kFinalWarps;
+      s[k] += i < n ? p[int64_t(i) * stride] : 0.f;
+    }
+  }
+  return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+}
+
 template <int NR, bool NC, bool GESUMMV>
-__global__ void __launch_bounds__(256) gemv_final_kernel(const float* __restrict__ row_part, int col_tiles, int rows,
-    const float* __restrict__ col_part, int row_groups, int cols, Term r0, Term r1, Term cterm) {
+__global__ void __launch_bounds__(32 * kFinalWarps) gemv_final_kernel(const float* __restrict__ row_part, int col_tiles,
+    int rows, const float* __restrict__ col_part, int row_groups, int cols, Term r0, Term r1, Term cterm) {
   constexpr int kSums = (NR > 0 ? NR : 0) + (NC ? 1 : 0);
-  __shared__ float red[kSums > 0 ? kSums : 1][8][32];
+  __shared__ float red[kSums > 0 ? kSums : 1][kFinalWarps][32];
   pdl_enter();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
-  if constexpr(NR > 0) {
 #pragma unroll
-    for(int t = 0; t < NR; ++t) {
-      float s = 0.f;
-      if(i < rows)
-        for(int ct = warp; ct < col_tiles; ct += 8) s += row_part[(int64_t(t) * col_tiles + ct) * rows + i];
-      red[t][warp][lane] = s;
-    }
-  }
-  if constexpr(NC) {
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;  // four loads in flight
-    if(i < cols) {
-      int g = warp;
-      for(; g + 24 < row_groups; g += 32) {
-        s0 += col_part[int64_t(g) * cols + i];
-        s1 += col_part[int64_t(g + 8) * cols + i];
-        s2 += col_part[int64_t(g + 16) * cols + i];
-        s3 += col_part[int64_t(g + 24) * cols + i];
-      }
-      for(; g < row_groups; g += 8) s0 += col_part[int64_t(g) * cols + i];
-    }
-    red[kSums - 1][warp][lane] = (s0 + s1) + (s2 + s3);
-  }
+  for(int t = 0; t < NR; ++t)
+    red[t][warp][lane] = i < rows ? strided_sum(row_part + int64_t(t) * col_tiles * rows + i, rows, col_tiles, warp) : 0.f;
+  if constexpr(NC) red[kSums - 1][warp][lane] = i < cols ? strided_sum(col_part + i, cols, row_groups, warp) : 0.f;
   __syncthreads();
   if(warp != 0) return;
   float sum[kSums > 0 ? kSums : 1];
@@ -212,7 +222,7 @@ __global__ void __launch_bounds__(256) gemv_final_kernel(const float* __restrict
   for(int t = 0; t < kSums; ++t) {
     sum[t] = 0.f;
 #pragma unroll
-    for(int w = 0; w < 8; ++w) sum[t] += red[t][w][lane];
+    for(int w = 0; w < kFinalWarps; ++w) sum[t] += red[t][w][lane];
   }
   if(NR > 0 && i < rows) {
     if constexpr(GESUMMV) {
@@ -232,9 +242,13 @@ gbpoly_status launch_gemv(gbpoly_ctx* ctx, GemvArgs g, Term r0, Term r1, Term ct
   // An empty matrix runs only the final kernel, with empty sums: y = beta y,
   // and for gesummv tmp unchanged, y = alpha tmp + beta y.
   const int col_tiles = std::max(1, (g.cols + kTileCols - 1) / kTileCols);
-  const int64_t want_groups = std::max<int64_t>(1, (4ll * std::max(ctx->sm_count, 1) + col_tiles - 1) / col_tiles);
-  int rpg = int((int64_t(g.rows) + want_groups - 1) / want_groups);
-  rpg = std::max(kRowBlock, (rpg + kRowBlock - 1) / kRowBlock * kRowBlock);
+  // Two CTAs per SM are resident.  Long row groups run as two full waves; where
+  // those would be short (under 64 rows; 16 of two matrices), one wave of twice the rows leaves no
+  // part-filled second one (bicg 4096: 17.7 us against 18.4 with 128 groups of 32 rows).
+  const int64_t ctas = 2ll * std::max(ctx->sm_count, 1);
+  const int64_t two_waves = std::max<int64_t>(1, 2 * ctas / col_tiles), one_wave = std::max<int64_t>(1, ctas / col_tiles);
+  const int64_t want_groups = g.rows / two_waves >= (TWO ? 16 : 64) ? two_waves : one_wave;
+  const int rpg = std::max<int>(rows_in_flight<TWO>(), int((g.rows + want_groups - 1) / want_groups));
   const int row_groups = std::max(1, (g.rows + rpg - 1) / rpg);
   if(row_groups > 65535) return fail(GBPOLY_ERR_UNSUPPORTED, "too many rows");
   g.col_tiles = col_tiles;
@@ -262,111 +276,96 @@ gbpoly_status launch_gemv(gbpoly_ctx* ctx, GemvArgs g, Term r0, Term r1, Term ct
   if(n == 0) return GBPOLY_OK;
   ProfileScope prof(ctx, "gemv_final");
   const bool some = g.rows > 0 && g.cols > 0;
-  GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_final_kernel<NR, NC, GESUMMV>, unsigned((n + 31) / 32), 256, 0, g.row_part,
+  GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_final_kernel<NR, NC, GESUMMV>, unsigned((n + 31) / 32), 32 * kFinalWarps, 0, g.row_part,
       some ? col_tiles : 0, g.rows, g.col_part, some ? row_groups : 0, g.cols, r0, r1, ct));
   return GBPOLY_OK;
 }
 
-// atax in one kernel: tmp += A x, then y += A^T tmp, each row group's rows
-// read from HBM once.  A persistent CTA walks row groups of kAtaxRows rows:
-// phase 1 reads the group's rows over all column chunks and completes their
-// row dots (so tmp of those rows is final), phase 2 reads the same rows again
-// (just read: from L2) and adds A[r][c] tmp[r] into the thread's column
-// accumulators, which stay in registers across the CTA's row groups and are
-// written once as the CTA's partial row of col_part.  CHUNKS 1024-column
-// chunks (cols <= CHUNKS * 1024, at most 8), 128-bit loads, one CTA per SM.
-constexpr int kAtaxRows = 16;
+// atax in one kernel and one read of A: tmp += A x, then y += A^T tmp.  A CTA
+// owns a contiguous range of rows and holds ROWS of them at a time in registers
+// (CHUNKS 1024-column tiles, cols <= CHUNKS * 1024, at most 8): it reduces their
+// row dots over the CTA (one barrier; tmp of those rows is then final) and adds
+// A[r][c] tmp[r] from the same registers into its column accumulators, written
+// once at the end as the CTA's row of col_part.  Two CTAs per SM up to 4096
+// columns, so that one's loads run while the other reduces.
+//
+// Bound: HBM, one read of A.  Reading the rows again from L2 for the second
+// product (16 rows, two barriers) kept fewer loads in flight: 4096 x 4096, A
+// from HBM, 21.6 -> 18.9 us (floor 9.9); odd rows, which took two passes, 45 ->
+// 21.5 us at 4095 x 4097 and 88.6 -> 43.7 at 7000 x 7001.
+constexpr int atax_rows(int chunks) { return chunks == 1 ? 16 : (chunks == 2 ? 8 : 4); }
+constexpr int atax_ctas(int chunks) { return chunks <= 4 ? 2 : 1; }  // per SM
 
-template <int CHUNKS>
-__global__ void __launch_bounds__(kThreads, 1) atax_kernel(const float* __restrict__ A, int64_t lda, int rows, int cols,
-    const float* __restrict__ x, float* __restrict__ tmp, float* __restrict__ col_part, int groups) {
-  __shared__ float red[kThreads / 32][kAtaxRows];
-  __shared__ float tmp_s[kAtaxRows];
+template <int CHUNKS, bool VEC>
+__global__ void __launch_bounds__(kThreads, atax_ctas(CHUNKS)) atax_kernel(const float* __restrict__ A, int64_t lda,
+    int rows, int cols, const float* __restrict__ x, float* __restrict__ tmp, float* __restrict__ col_part) {
+  constexpr int R = atax_rows(CHUNKS);
+  __shared__ float red[2][kThreads / 32 + 1][R];  // warp sums and the old tmp, alternating sets
   pdl_enter();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int begin = int(int64_t(rows) * blockIdx.x / gridDim.x), end = int(int64_t(rows) * (blockIdx.x + 1) / gridDim.x);
   float4 xr[CHUNKS], colacc[CHUNKS];
 #pragma unroll
   for(int ch = 0; ch < CHUNKS; ++ch) {
-    const int c = ch * kTileCols + 4 * tid;
-    xr[ch] = c < cols ? *reinterpret_cast<const float4*>(x + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    xr[ch] = load4<VEC>(x, ch * kTileCols, cols);
     colacc[ch] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  for(int g = blockIdx.x; g < groups; g += gridDim.x) {
-    const int r0 = g * kAtaxRows, nr = min(kAtaxRows, rows - r0);
-    // phase 1: row dots of the group over all columns
-    float acc[kAtaxRows];
+  for(int r0 = begin, it = 0; r0 < end; r0 += R, it ^= 1) {
+    const int nr = min(R, end - r0);
+    float4 a[R][CHUNKS];
 #pragma unroll
-    for(int k = 0; k < kAtaxRows; ++k) acc[k] = 0.f;
+    for(int k = 0; k < R; ++k)
 #pragma unroll
-    for(int ch = 0; ch < CHUNKS; ++ch) {
-      const int c = ch * kTileCols + 4 * tid;
-      if(c < cols) {
-        float4 a[kAtaxRows];
+      for(int ch = 0; ch < CHUNKS; ++ch)
+        a[k][ch] = k < nr ? load4<VEC>(A + int64_t(r0 + k) * lda, ch * kTileCols, cols) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if(tid < R) red[it][kThreads / 32][tid] = tid < nr ? tmp[r0 + tid] : 0.f;
+    float acc[R];
 #pragma unroll
-        for(int k = 0; k < kAtaxRows; ++k)
-          a[k] = k < nr ? *reinterpret_cast<const float4*>(A + int64_t(r0 + k) * lda + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for(int k = 0; k < R; ++k) {
+      acc[k] = 0.f;
 #pragma unroll
-        for(int k = 0; k < kAtaxRows; ++k) acc[k] += dot4(a[k], xr[ch]);
-      }
+      for(int ch = 0; ch < CHUNKS; ++ch) acc[k] += dot4(a[k][ch], xr[ch]);
     }
-    const float rs = reduce_rows<kAtaxRows>(acc, lane);
-    if(lane < kAtaxRows) red[warp][lane] = rs;
-    __syncthreads();
-    if(warp == 0 && lane < kAtaxRows) {
+    const float rs = reduce_rows<R>(acc, lane);
+    if(lane < R) red[it][warp][lane] = rs;
+    __syncthreads();  // (a set is rewritten two groups later, after the next group's barrier)
+#pragma unroll
+    for(int k = 0; k < R; ++k) {
       float sum = 0.f;
 #pragma unroll
-      for(int w = 0; w < kThreads / 32; ++w) sum += red[w][lane];
-      float t = 0.f;
-      if(lane < nr) {
-        t = tmp[r0 + lane] + sum;  // tmp += A x (atax.cpp:78-83)
-        tmp[r0 + lane] = t;
-      }
-      tmp_s[lane] = t;
-    }
-    __syncthreads();
-    // phase 2: the same rows again, y += A^T tmp (atax.cpp:91-96)
+      for(int w = 0; w < kThreads / 32; ++w) sum += red[it][w][k];
+      const float t = red[it][kThreads / 32][k] + sum;  // tmp += A x (atax.cpp:78-83)
+      if(tid == 0 && k < nr) tmp[r0 + k] = t;
 #pragma unroll
-    for(int ch = 0; ch < CHUNKS; ++ch) {
-      const int c = ch * kTileCols + 4 * tid;
-      if(c < cols) {
-        float4 a[kAtaxRows];
-#pragma unroll
-        for(int k = 0; k < kAtaxRows; ++k)
-          a[k] = k < nr ? *reinterpret_cast<const float4*>(A + int64_t(r0 + k) * lda + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for(int k = 0; k < kAtaxRows; ++k) {
-          const float w = tmp_s[k];
-          colacc[ch].x = fmaf(a[k].x, w, colacc[ch].x);
-          colacc[ch].y = fmaf(a[k].y, w, colacc[ch].y);
-          colacc[ch].z = fmaf(a[k].z, w, colacc[ch].z);
-          colacc[ch].w = fmaf(a[k].w, w, colacc[ch].w);
-        }
+      for(int ch = 0; ch < CHUNKS; ++ch) {  // y += A^T tmp (atax.cpp:91-96); a is zero beyond nr
+        colacc[ch].x = fmaf(a[k][ch].x, t, colacc[ch].x);
+        colacc[ch].y = fmaf(a[k][ch].y, t, colacc[ch].y);
+        colacc[ch].z = fmaf(a[k][ch].z, t, colacc[ch].z);
+        colacc[ch].w = fmaf(a[k][ch].w, t, colacc[ch].w);
       }
     }
-    __syncthreads();  // red and tmp_s are rewritten by the next group
   }
 #pragma unroll
-  for(int ch = 0; ch < CHUNKS; ++ch) {
-    const int c = ch * kTileCols + 4 * tid;
-    if(c < cols) *reinterpret_cast<float4*>(col_part + int64_t(blockIdx.x) * cols + c) = colacc[ch];
-  }
+  for(int ch = 0; ch < CHUNKS; ++ch)
+    store4<VEC>(col_part + int64_t(blockIdx.x) * cols, ch * kTileCols, cols, colacc[ch]);
 }
 
 template <int CHUNKS>
 gbpoly_status launch_atax(gbpoly_ctx* ctx, const float* A, int64_t lda, int rows, int cols, const float* x, float* tmp,
-    float* y) {
-  const int groups = (rows + kAtaxRows - 1) / kAtaxRows;
-  const int grid = std::max(1, std::min(groups, std::max(ctx->sm_count, 1)));  // one CTA per SM
+    float* y, bool vec) {
+  const int ctas = atax_ctas(CHUNKS) * std::max(ctx->sm_count, 1);
+  const int grid = std::max(1, std::min((rows + atax_rows(CHUNKS) - 1) / atax_rows(CHUNKS), ctas));
   gbpoly_status st = ensure_scratch(ctx, ctx->stats, size_t(grid) * size_t(cols) * 4 + 256, "matrix-vector scratch");
   if(st != GBPOLY_OK) return st;
   float* col_part = static_cast<float*>(ctx->stats.ptr);
   {
     ProfileScope prof(ctx, "atax");
-    GBPOLY_CUDA_TRY(launch_pdl(ctx, atax_kernel<CHUNKS>, grid, kThreads, 0, A, lda, rows, cols, x, tmp, col_part, groups));
+    GBPOLY_CUDA_TRY(launch_pdl(ctx, vec ? atax_kernel<CHUNKS, true> : atax_kernel<CHUNKS, false>, grid, kThreads, 0, A, lda,
+        rows, cols, x, tmp, col_part));
   }
   ProfileScope prof(ctx, "gemv_final");
-  GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_final_kernel<0, true, false>, unsigned((cols + 31) / 32), 256, 0, nullptr, 0, rows,
-      col_part, grid, cols, Term{}, Term{}, Term{1.f, 1.f, y}));
+  GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_final_kernel<0, true, false>, unsigned((cols + 31) / 32), 32 * kFinalWarps, 0,
+      nullptr, 0, rows, col_part, grid, cols, Term{}, Term{}, Term{1.f, 1.f, y}));
   return GBPOLY_OK;
 }
 
@@ -436,19 +435,19 @@ gbpoly_status gbpoly_atax_f32(gbpoly_ctx* ctx, int64_t rows, int64_t cols, const
   const bool vec = (cols % 4 == 0) && (lda % 4 == 0) && ((reinterpret_cast<uintptr_t>(A) & 15) == 0) &&
                    ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
   const int chunks = int((cols + kTileCols - 1) / kTileCols);
-  if(vec && chunks <= 8) {
+  if(chunks <= 8) {
     switch(chunks) {
-    case 1: return launch_atax<1>(ctx, A, lda, int(rows), int(cols), x, tmp, y);
-    case 2: return launch_atax<2>(ctx, A, lda, int(rows), int(cols), x, tmp, y);
-    case 3: return launch_atax<3>(ctx, A, lda, int(rows), int(cols), x, tmp, y);
-    case 4: return launch_atax<4>(ctx, A, lda, int(rows), int(cols), x, tmp, y);
-    case 5: return launch_atax<5>(ctx, A, lda, int(rows), int(cols), x, tmp, y);
-    case 6: return launch_atax<6>(ctx, A, lda, int(rows), int(cols), x, tmp, y);
-    case 7: return launch_atax<7>(ctx, A, lda, int(rows), int(cols), x, tmp, y);
-    default: return launch_atax<8>(ctx, A, lda, int(rows), int(cols), x, tmp, y);
+    case 1: return launch_atax<1>(ctx, A, lda, int(rows), int(cols), x, tmp, y, vec);
+    case 2: return launch_atax<2>(ctx, A, lda, int(rows), int(cols), x, tmp, y, vec);
+    case 3: return launch_atax<3>(ctx, A, lda, int(rows), int(cols), x, tmp, y, vec);
+    case 4: return launch_atax<4>(ctx, A, lda, int(rows), int(cols), x, tmp, y, vec);
+    case 5: return launch_atax<5>(ctx, A, lda, int(rows), int(cols), x, tmp, y, vec);
+    case 6: return launch_atax<6>(ctx, A, lda, int(rows), int(cols), x, tmp, y, vec);
+    case 7: return launch_atax<7>(ctx, A, lda, int(rows), int(cols), x, tmp, y, vec);
+    default: return launch_atax<8>(ctx, A, lda, int(rows), int(cols), x, tmp, y, vec);
     }
   }
-  // wide or unaligned matrices: the two passes
+  // wide matrices: the two passes
   if((st = gbpoly_gemv_f32(ctx, GBPOLY_OP_N, rows, cols, 1.f, A, lda, x, 1.f, tmp)) != GBPOLY_OK) return st;
   return gbpoly_gemv_f32(ctx, GBPOLY_OP_T, rows, cols, 1.f, A, lda, tmp, 1.f, y);
 }
