@@ -126,8 +126,8 @@ gbpoly_status gbpoly_workspace_query(gbpoly_precision prec, int64_t M, int64_t N
  * tiles.  fp16x3: 2 pairs on 256 x 256, 3 on 256 x 128).  The context keeps
  * one per (form, ceil(log2) of M, N, K); unless tuned or set, a shape whose
  * 256 x 256 tiles give every SM pair a tile uses configuration 5 up to
- * K = 256 (tf32: 512, tf32x3: 128) and 3 beyond (fp16x3: 2), a smaller or
- * symmetric one the tile shape (128 x 128, 256 x 256, 256 x 128) of the least
+ * K = 128 (tf32: 512, tf32x3, bf16x6: 64), 6 up to K = 384 (tf32x3: 192) and 3
+ * beyond (fp16x3: 3, then 2), a smaller or symmetric one the tile shape (128 x 128, 256 x 256, 256 x 128) of the least
  * estimated time.  fp8: configuration 1 (128 x 256 tiles) when its tiles give
  * every SM one, else 0 (128 x 128, also every symmetric product). */
 gbpoly_status gbpoly_gemm_config_count(gbpoly_precision prec, int* count);

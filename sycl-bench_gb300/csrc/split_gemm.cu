@@ -92,7 +92,7 @@ constexpr double chunk_us(Elem e, int terms, TileShape s) {
 }
 // What a K-split tile's handoff costs, in microseconds: in a launch of one
 // unit per CTA, and in a last round.
-constexpr double kHandoffUs = 7, kHandoffLastRoundUs = 9;
+constexpr double kHandoffUs = 7, kHandoffLastRoundUs = 8;
 
 // CG_ = 2: a CTA pair (cluster of two) computes a (256 x BN) tile with
 // cta_group::2 MMAs: each CTA holds 128 rows of the A tile and BN/2 rows of
@@ -136,7 +136,9 @@ struct Form {
   // Launches of one unit per CTA may keep C in the pipeline's stages, loaded
   // and stored by TMA (RING kernels, forms with one stage per chunk).  The
   // loads start under the last chunk where the other stages hold the whole C tile.
-  static constexpr bool RING_C = !CEPI && CH == 1;
+  // (not the 1-CTA 128 x 256 configurations, which no rule chooses but fp8's)
+  static constexpr bool RING_C = !CEPI && CH == 1 && (CG == 2 || BN == 128 || E == Elem::E4M3);
+  static constexpr bool BOX_C = RING_C && (CG == 2 || E == Elem::E4M3);
   static constexpr bool RING_C_EARLY = RING_C && (STAGES - 1) * STAGE >= C_TILE;
   static constexpr int NBUF = BN <= 128 ? 4 : 2;
   // TMEM allocations are powers of two (>= 32 columns); chunk buffer b
@@ -842,8 +844,16 @@ __device__ __forceinline__ void prefetch_c_warp(const TileInfo& t, uint32_t rank
   }
 }
 
-template <class F, class S, bool RING>
+// How the epilogue reads and writes C:
+//   Staged  through a per-warp 32 x 33 staging tile with coalesced loads and
+//           stores (any alignment; every C-tile form's kernel, too);
+//   Ring    one unit per CTA: the whole C tile by TMA in the pipeline's idle stages;
+//   Boxes   any number of units: by TMA, one 32 x 32 box per warp at a time.
+enum class Epi { Staged, Ring, Boxes };
+
+template <class F, class S, Epi EPI>
 __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_constant__ S sched, int* err) {
+  constexpr bool RING = EPI == Epi::Ring, BOXES = EPI == Epi::Boxes;
   extern __shared__ __align__(1024) char smem_raw[];
   char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + F::STAGES * F::STAGE);
@@ -852,7 +862,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
   uint64_t* chunk_empty = chunk_full + F::NBUF;  // [NBUF]
   uint64_t* drain = chunk_empty + F::NBUF;
   uint64_t* cbar = drain + 1;  // C through TMA: one barrier per epilogue warp for its C boxes
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1 + (F::CEPI || RING ? 8 : 0));
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1 + (F::CEPI || EPI != Epi::Staged ? 8 : 0));
   float(*epi_stage)[33] = reinterpret_cast<float(*)[33]>(smem + F::STAGES * F::STAGE + 256);  // 8 warps x [32][33]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -874,7 +884,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
       mbar_init(&chunk_empty[b], 8 * F::CG);  // one arrival per epilogue warp of the pair
     }
     mbar_init(drain, 1);
-    if constexpr(F::CEPI || RING)
+    if constexpr(F::CEPI || EPI != Epi::Staged)
       for(int w = 0; w < 8; ++w) mbar_init(&cbar[w], 1);
     fence_mbar_init();
   }
@@ -1037,6 +1047,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
     int c_loads = 0, c_stores = 0;
     // chunk buffers are released on the first CTA's barriers (MMAs are issued there)
     const uint32_t chunk_empty_pair = F::CG == 2 ? cluster_map(chunk_empty, 0) : 0u;
+    auto below_of = [&](const TileInfo& t) { return F::MIRROR && t.lower ? diag_row<F>(t, rank) - t.n0 : 0; };
     for(int u = first_tile; u < units && ok; u += tile_step) {
       int tile, role, slot;
       sched.unit(u, tile, role, slot);
@@ -1063,11 +1074,26 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
           ++c_loads;
         }
       }
+      // BOXES: this warp's box, loaded with the first 32 x 32 of C while the
+      // MMAs run (once the previous unit's last store has read it)
+      const bool writes = role != 2 && below_of(ti) >= 0;
+      char* const my_box = smem + F::STAGES * F::STAGE + 1024 + (warp - 4) * F::C_BOX;
+      auto load_box = [&](int x, int y) {
+        if constexpr(BOXES) {
+          if(lane == 0) {
+            if(c_stores > 0) bulk_wait_read_all();
+            mbar_arrive_expect_tx(&cbar[warp - 4], F::C_BOX);
+            tma_load_2d(my_box, &sched.cmap, &cbar[warp - 4], x, y);
+          }
+          ++c_loads;
+        }
+      };
+      if(BOXES && writes && beta != 0.f) load_box(nbase, crow);
       // RING: the CTA's only unit.  This warp's HALF / 32 boxes of C live in the
       // pipeline's stages, which no later tile fills.  The loads start while
       // the last chunk's MMAs run: every stage but that chunk's has been read
       // (its chunk was complete), and the boxes lie from the stage after it.
-      const int below = F::MIRROR && ti.lower ? diag_row<F>(ti, rank) - ti.n0 : 0;
+      const int below = below_of(ti);
       constexpr int kBoxes = F::HALF / 32;
       char* ring_box = nullptr;
       auto load_ring = [&](int last_chunk) {
@@ -1232,6 +1258,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
       if(!ok) {
         // do not leave while C's copies into the stages are in flight
         if(RING && ring_box != nullptr && beta != 0.f) mbar_wait(&cbar[warp - 4], 0, err, kDevErrDrainWait);
+        if(BOXES && writes && beta != 0.f) mbar_wait(&cbar[warp - 4], (c_loads - 1) & 1, err, kDevErrDrainWait);
         continue;
       }
       if constexpr(F::CEPI) {
@@ -1276,7 +1303,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         if(role == 2 && lane == 0) atomicAdd(&sched.flags[slot], 1);
         continue;
       }
-      if constexpr(RING) {
+      if constexpr(EPI != Epi::Staged) {
         // K-split tile: the second half stores its sums (register i of a warp
         // as one 128-byte row), the first half waits for them and adds them to
         // its own (first + second) before writing C
@@ -1294,15 +1321,18 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
             ok = false;
             continue;
           }
+          constexpr int kPart = RING ? 32 : 16;  // loads in flight at a time
 #pragma unroll
-          for(int i0 = 0; i0 < F::HALF; i0 += 32) {
-            float v[32];
+          for(int i0 = 0; i0 < F::HALF; i0 += kPart) {
+            float v[kPart];
 #pragma unroll
-            for(int i = 0; i < 32; ++i) v[i] = __ldcg(part + 32 * (i0 + i));
+            for(int i = 0; i < kPart; ++i) v[i] = __ldcg(part + 32 * (i0 + i));
 #pragma unroll
-            for(int i = 0; i < 32; ++i) acc[i0 + i] += v[i];
+            for(int i = 0; i < kPart; ++i) acc[i0 + i] += v[i];
           }
         }
+      }
+      if constexpr(RING) {
         // C = alpha acc + beta C in the boxes (lane = row: eight 16-byte
         // chunks, swizzled by row), each stored by TMA when done (clipped at
         // the matrix edges)
@@ -1366,6 +1396,51 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         }
         ++c_stores;
         continue;
+      } else if constexpr(BOXES) {
+        // the same box by box: load, alpha acc + beta C in place, store
+        const int boxes = below > 0 ? 2 * kBoxes : kBoxes;
+#pragma unroll
+        for(int t = 0; t < (F::MIRROR ? 2 : 1); ++t) {
+          if(t == 1 && below <= 0) break;
+#pragma unroll
+          for(int j = 0; j < kBoxes; ++j) {
+            if(beta != 0.f) {
+              if(!mbar_wait(&cbar[warp - 4], (c_loads - 1) & 1, err, kDevErrMmaWait)) ok = false;
+            } else {
+              if(lane == 0 && c_stores > 0) bulk_wait_read_all();
+              __syncwarp();
+            }
+            if(t == 0) {
+#pragma unroll
+              for(int k = 0; k < 8; ++k) {
+                float4* p4 = reinterpret_cast<float4*>(my_box + lane * 128 + ((k ^ (lane & 7)) << 4));
+                const float4 cv = beta != 0.f ? *p4 : make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 o;
+                o.x = fmaf(beta, cv.x, alpha * acc[32 * j + 4 * k]);
+                o.y = fmaf(beta, cv.y, alpha * acc[32 * j + 4 * k + 1]);
+                o.z = fmaf(beta, cv.z, alpha * acc[32 * j + 4 * k + 2]);
+                o.w = fmaf(beta, cv.w, alpha * acc[32 * j + 4 * k + 3]);
+                *p4 = o;
+              }
+            } else {  // the transpose, C[nbase + r][crow + lane]
+#pragma unroll
+              for(int r = 0; r < 32; ++r) {
+                float* p = reinterpret_cast<float*>(my_box + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + 4 * (lane & 3));
+                *p = fmaf(beta, beta != 0.f ? *p : 0.f, alpha * acc[32 * j + r]);
+              }
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if(lane == 0) {
+              tma_store_2d(&sched.cmap, my_box, t ? crow : nbase + 32 * j, t ? nbase + 32 * j : crow);
+              bulk_commit();
+            }
+            ++c_stores;
+            const int next = kBoxes * t + j + 1, jn = next % kBoxes;
+            if(beta != 0.f && next < boxes)
+              load_box(next >= kBoxes ? crow : nbase + 32 * jn, next >= kBoxes ? nbase + 32 * jn : crow);
+          }
+        }
       } else {
       // K-split tile: the second half stores its sums (partial tile of the
       // CTA: 128 rows x BN, row-major), the first half waits for them and
@@ -1448,7 +1523,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
       }
       }  // staged epilogue
     }
-    if constexpr(F::CEPI || RING)
+    if constexpr(F::CEPI || EPI != Epi::Staged)
       if(lane == 0 && c_stores > 0) bulk_wait_all();  // C written before the CTA leaves
   }
 
@@ -1527,16 +1602,16 @@ gbpoly_status make_product_maps(gbpoly_ctx* ctx, ProductMaps& pm, Panels left, i
 
 // Once per device context: shared-memory opt-in and the register check of
 // the warp split.
-template <class F, class S, bool RING>
+template <class F, class S, Epi EPI>
 gbpoly_status tc_prepare(gbpoly_ctx* ctx) {
   static ContextMark prepared;
   if(prepared.valid(ctx->device)) return GBPOLY_OK;
-  GBPOLY_CUDA_TRY(cudaFuncSetAttribute(split_gemm_kernel<F, S, RING>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
+  GBPOLY_CUDA_TRY(cudaFuncSetAttribute(split_gemm_kernel<F, S, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, F::SMEM));
   // setmaxnreg redistributes the registers the CTA was launched with: the
   // split must fit in threads x registers-per-thread at launch, or the
   // increase would wait forever.
   cudaFuncAttributes fa;
-  GBPOLY_CUDA_TRY(cudaFuncGetAttributes(&fa, split_gemm_kernel<F, S, RING>));
+  GBPOLY_CUDA_TRY(cudaFuncGetAttributes(&fa, split_gemm_kernel<F, S, EPI>));
   const long need = 128l * F::REGS_CTRL + 256l * F::REGS_EPI;
   if(long(fa.numRegs) * F::THREADS < need)
     return fail(GBPOLY_ERR_UNSUPPORTED, "tensor-core kernel built with too few registers for its warp split");
@@ -1571,7 +1646,7 @@ template <class F, class S>
 gbpoly_status pair_clusters(gbpoly_ctx* ctx, int& clusters) {
   static int max_clusters[32] = {};
   static ContextMark known;
-  gbpoly_status st = tc_prepare<F, S, false>(ctx);
+  gbpoly_status st = tc_prepare<F, S, Epi::Staged>(ctx);
   if(st != GBPOLY_OK) return st;
   if(known.valid(ctx->device)) {
     clusters = max_clusters[ctx->device];
@@ -1580,7 +1655,7 @@ gbpoly_status pair_clusters(gbpoly_ctx* ctx, int& clusters) {
   PairLaunch<F> pl(ctx, ctx->sm_count / 2);
   pl.cfg.numAttrs = 1;
   int n = 0;
-  GBPOLY_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, split_gemm_kernel<F, S, false>, &pl.cfg));
+  GBPOLY_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, split_gemm_kernel<F, S, Epi::Staged>, &pl.cfg));
   if(n <= 0) return fail(GBPOLY_ERR_UNSUPPORTED, "no CTA pair of this tensor-core configuration fits on the device");
   if(ctx->device >= 0 && ctx->device < 32) {
     max_clusters[ctx->device] = n;
@@ -1650,27 +1725,33 @@ void apply_tail(const TailPlan& tp, char* base, S& sched) {
   sched.flags = tail_flags(tp, base);
 }
 
-template <class F, class S, bool RING>
+template <class F, class S, Epi EPI>
 gbpoly_status launch_tc_variant(gbpoly_ctx* ctx, const S& sched, int64_t units, int resident, const char* kernel_name) {
-  gbpoly_status st = tc_prepare<F, S, RING>(ctx);
+  gbpoly_status st = tc_prepare<F, S, EPI>(ctx);
   if(st != GBPOLY_OK) return st;
   const int grid = int(std::min<int64_t>(units, resident));
   ProfileScope prof(ctx, kernel_name);
   if constexpr(F::CG == 2) {
     PairLaunch<F> pl(ctx, grid);
-    GBPOLY_CUDA_TRY(cudaLaunchKernelEx(&pl.cfg, split_gemm_kernel<F, S, RING>, sched, ctx->err_dev));
+    GBPOLY_CUDA_TRY(cudaLaunchKernelEx(&pl.cfg, split_gemm_kernel<F, S, EPI>, sched, ctx->err_dev));
   } else {
-    GBPOLY_CUDA_TRY(launch_pdl(ctx, split_gemm_kernel<F, S, RING>, grid, F::THREADS, F::SMEM, sched, ctx->err_dev));
+    GBPOLY_CUDA_TRY(launch_pdl(ctx, split_gemm_kernel<F, S, EPI>, grid, F::THREADS, F::SMEM, sched, ctx->err_dev));
   }
   return GBPOLY_OK;
 }
 
-// A launch that gives every CTA (or pair) at most one unit moves C through
-// TMA where it can (a whole C tile in flight at once in the stages nobody
-// fills again, instead of 16 rows of 128 bytes per warp): a single 256 x 256
-// pair tile takes 15 us instead of 25 (K = 128), gemm 2048 of bf16x3 39
-// instead of 47.  Launches of more units keep the staged epilogue alone: with
-// both in one kernel its loop lost registers (fp16x3 at 4096 315 -> 375 us).
+// Which epilogue a launch gets.  Where TMA can address C's rows, C moves
+// through it: 32 KB in flight per SM without a register or an address
+// computed, against 16 KB in 16-row batches of staged loads.  A launch of at
+// most one unit per CTA (or pair) has the whole C tile in flight at once, in
+// the stages nobody fills again (a single 256 x 256 pair tile of K = 128: 15 us
+// instead of 25).  Launches of more units take it box by box (us, staged /
+// boxes: bf16x3 2560 106 / 88, 4096 300 / 280, 4096 x 3000 x 600 70 / 55, fp16x3
+// 4096 x 3000 x 2560 172 / 163, syrk 4096 173 / 159, fp8 4096 146 / 131, bf16x3
+// 8192 2085 / 2045), but for 1-CTA tiles of symmetric products (syrk 3072 of
+// bf16x3 91.6 / 93.9: the mirrored box is a second pass over it).  Each is a
+// kernel of its own: two epilogues in one cost its loop registers (fp16x3 at
+// 4096 315 -> 375 us with a staged and a whole-tile one).
 template <class F, class S>
 gbpoly_status launch_tc_kernel(gbpoly_ctx* ctx, const S& sched, int64_t units, const char* kernel_name) {
   if(units <= 0) return GBPOLY_OK;
@@ -1679,10 +1760,15 @@ gbpoly_status launch_tc_kernel(gbpoly_ctx* ctx, const S& sched, int64_t units, c
     gbpoly_status st = pair_clusters<F, S>(ctx, resident);
     if(st != GBPOLY_OK) return st;
   }
-  if constexpr(F::RING_C && std::is_same_v<S, SingleSched<F::BM, F::BN>>)
-    if(sched.ring_c && units <= resident)
-      return launch_tc_variant<F, S, true>(ctx, sched, units, resident, kernel_name);
-  return launch_tc_variant<F, S, false>(ctx, sched, units, resident, kernel_name);
+  if constexpr(std::is_same_v<S, SingleSched<F::BM, F::BN>>) {
+    if constexpr(F::RING_C)
+      if(sched.ring_c && units <= resident)
+        return launch_tc_variant<F, S, Epi::Ring>(ctx, sched, units, resident, kernel_name);
+    if constexpr(F::BOX_C)
+      if(sched.ring_c && !(F::CG == 1 && sched.lower))
+        return launch_tc_variant<F, S, Epi::Boxes>(ctx, sched, units, resident, kernel_name);
+  }
+  return launch_tc_variant<F, S, Epi::Staged>(ctx, sched, units, resident, kernel_name);
 }
 
 // Workspace layout: terms x [A panel] then terms x [B panel] (B absent when
@@ -2019,7 +2105,7 @@ double tile_cost(gbpoly_ctx* ctx, gbpoly_precision prec, TileShape s, int64_t M,
   const double rounds = double(full) + (rest == 0 ? 0.0 : (split ? 0.5 : 1.0));
   const double ends = double(full + (rest > 0) - 1);  // exposed tile ends before the last
   double t = (s == kTileSquare ? 9 : 11) + rounds * double(chunks) * c + (split ? handoff : 0);
-  t += ends * (s == kTileSquare ? 1 : (s == kTilePair ? 9 : 6));
+  t += ends * (s == kTileSquare ? 1 : (s == kTilePair ? (c_tma ? 5 : 9) : (c_tma ? 4 : 6)));
   const bool staged = ends > 0 || !c_tma;  // the last tile's C
   if(lower && s == kTilePair) t += staged ? 8 * (ends + 1) : 3;  // mirrored C of a 256 x 256 tile
   if(!c_tma && ends == 0) t += s == kTilePair ? 7 : (s == kTileNarrow ? 3 : 0);
@@ -2043,24 +2129,27 @@ int square_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t N, int64_t K, 
 }
 }  // namespace
 
-// Configuration of an untuned shape: CTA pairs (256 x 256 tiles) when they
-// fill the device, with the C tile in shared memory (configuration 5) while
-// K is short enough that C's traffic bounds the call (measured on GB300 at
-// M = N = 8192: 1.75x faster up to K = 128, ahead up to K = 256 for the
-// BF16 forms and K = 512 for tf32, behind beyond), else the tile shape of the
-// least estimated time (bf16x3, us, chosen / 128 x 128 tiles: 2048 cubed 52 /
-// 69, 256 x 4096 x 4096 65 / 81, 4096 x 1024 x 512 25 / 29).
+// Configuration of an untuned shape.  When 256 x 256 tiles give every SM pair
+// one: while K is so short that C's traffic bounds the call, the C tile in
+// shared memory (configuration 5), then up to six chunks of K pairs on
+// 256 x 128 tiles, whose C overlaps more of the chunks, then 256 x 256 (us for
+// configurations 5 / 256 x 128 / 256 x 256, M = N = 8192, bf16x3: K = 64 102 /
+// 111 / 106, 128 111 / 116 / 111, 256 184 / 124 / 142, 384 243 / 161 / 169, 512
+// 301 / 201 / 189; tf32x3 64 110 / 115 / 110, 128 181 / 122 / 140; bf16x6 64
+// 104 / 113 / 109, 256 227 / 160 / 175; at 4096, bf16x3 K = 256: 48 / 38 / 48).
+// tf32 keeps configuration 5 up to K = 512.  Else the tile shape of the least
+// estimated time (bf16x3, us, chosen / 128 x 128 tiles: 2048 cubed 52 / 69,
+// 256 x 4096 x 4096 65 / 81, 4096 x 1024 x 512 25 / 29).
 int default_config(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K, bool c_tma) {
   // fp8: 128 x 256 tiles (twice the MMA work per scaled chunk: 1.38x at
   // N = 8192) when they give every SM a tile, else 128 x 128
   if(prec == GBPOLY_PREC_FP8) return ((M + 127) / 128) * ((N + 255) / 256) >= ctx->sm_count ? 1 : 0;
   if(tensor_config_count(prec) <= 3) return 0;
-  if(pairs_fill(ctx, ((M + 255) / 256) * ((N + 255) / 256))) {
-    if(prec == GBPOLY_PREC_FP16X3) return 2;
-    const int64_t k_tile = prec == GBPOLY_PREC_TF32 ? 512 : (prec == GBPOLY_PREC_TF32X3 ? 128 : 256);
-    return K <= k_tile ? 5 : 3;
-  }
-  return cheapest_config(ctx, prec, M, N, K, 1, false, c_tma);
+  if(!pairs_fill(ctx, ((M + 255) / 256) * ((N + 255) / 256))) return cheapest_config(ctx, prec, M, N, K, 1, false, c_tma);
+  if(prec == GBPOLY_PREC_TF32) return K <= 512 ? 5 : 3;
+  const int64_t bk = prec == GBPOLY_PREC_TF32X3 ? 32 : 64, chunks = (K + bk - 1) / bk;
+  if(prec != GBPOLY_PREC_FP16X3 && chunks <= (prec == GBPOLY_PREC_BF16X6 ? 1 : 2)) return 5;
+  return config_of(prec, c_tma && chunks <= 6 ? kTileNarrow : kTilePair);
 }
 
 gbpoly_status tensor_plan(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K, const float* C,

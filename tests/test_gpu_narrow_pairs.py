@@ -107,3 +107,37 @@ def test_host_panels_split_like_the_whole_call(ctx):
         np.testing.assert_array_equal(out.view(np.uint32), ctx.download(dC, C.shape).view(np.uint32))
     for b in (dA, dB, dC):
         ctx.free(b)
+
+
+@pytest.mark.parametrize("prec", list(FORMS), ids=lambda p: p.name.lower())
+@pytest.mark.parametrize("beta", [0.0, -0.5])
+def test_rounds_of_boxes_are_bitwise_the_square_tiles(ctx, prec, beta):
+    # more pair tiles than pairs: C box by box, ragged in rows and columns; and
+    # the same through rows TMA cannot address
+    A, B, C = matrices((2570, 2436, 100), 11)
+    square, *pairs = (run(ctx, prec, c, A, B, C, beta, False) for c in FORMS[prec])
+    staged = run(ctx, prec, FORMS[prec][1], A, B, C, beta, False, ldc=2437)
+    for got in (*pairs, staged):
+        np.testing.assert_array_equal(got.view(np.uint32), square.view(np.uint32))
+
+
+@pytest.mark.parametrize("op", ["syrk", "syr2k"])
+@pytest.mark.parametrize("prec", [Precision.BF16X3, Precision.FP16X3], ids=lambda p: p.name.lower())
+def test_rounds_of_mirrored_boxes(ctx, prec, op):
+    # 91 and 182 pair tiles; 256 x 256 tiles as in the symmetric test above
+    A, B, C = matrices((3212, 3212, 70), 12, symmetric=True)
+    square, pair, narrow = (run(ctx, prec, c, A, B, C, 0.75, False, op=op) for c in FORMS[prec])
+    np.testing.assert_array_equal(narrow.view(np.uint32), square.view(np.uint32))
+    assert np.linalg.norm(pair - square) / np.linalg.norm(square) < 1e-6
+    tail = run(ctx, prec, FORMS[prec][1], A, B, C, 0.75, True, op=op)  # a split last round, where it pays
+    assert np.linalg.norm(tail - square) / np.linalg.norm(square) < 1e-6
+
+
+@pytest.mark.parametrize("mnk", [(1300, 2500, 130), (2450, 2308, 300)], ids=str)
+def test_fp8_boxes_are_bitwise_the_square_tiles(ctx, mnk):
+    M, N, K = mnk
+    A, B, C = matrices(mnk, M)
+    outs = [run(ctx, Precision.FP8, c, A, B, C, 0.5, True) for c in (0, 1)]
+    staged = run(ctx, Precision.FP8, 1, A, B, C, 0.5, True, ldc=N + 1)
+    np.testing.assert_array_equal(outs[1].view(np.uint32), outs[0].view(np.uint32))
+    np.testing.assert_array_equal(staged.view(np.uint32), outs[0].view(np.uint32))
