@@ -2072,6 +2072,12 @@ bool config_is_square(gbpoly_precision prec, int config) {
 // CTA pairs when their 256 x 256 tiles give every SM pair at least one tile.
 bool pairs_fill(gbpoly_ctx* ctx, int64_t pair_tiles) { return pair_tiles >= std::max(1, ctx->sm_count / 2); }
 
+Elem elem_of(gbpoly_precision prec) {
+  if(prec == GBPOLY_PREC_FP16X3) return Elem::F16;
+  return prec == GBPOLY_PREC_TF32 || prec == GBPOLY_PREC_TF32X3 ? Elem::TF32 : Elem::BF16;
+}
+int terms_of(gbpoly_precision prec) { return prec == GBPOLY_PREC_BF16X6 ? 3 : (prec == GBPOLY_PREC_TF32 ? 1 : 2); }
+
 int config_of(gbpoly_precision prec, TileShape s) {
   if(prec == GBPOLY_PREC_FP16X3) return s == kTileSquare ? 1 : (s == kTilePair ? 2 : 3);
   return s == kTileSquare ? (prec == GBPOLY_PREC_BF16X6 ? 0 : 2) : (s == kTilePair ? 3 : 6);
@@ -2087,10 +2093,8 @@ int config_of(gbpoly_precision prec, TileShape s) {
 // shapes and ten symmetric ones: the shape chosen is within 5 % of the fastest.
 double tile_cost(gbpoly_ctx* ctx, gbpoly_precision prec, TileShape s, int64_t M, int64_t N, int64_t K, int pairings,
     bool lower, bool c_tma) {
-  const Elem e = prec == GBPOLY_PREC_FP16X3                                          ? Elem::F16
-                 : (prec == GBPOLY_PREC_TF32 || prec == GBPOLY_PREC_TF32X3) ? Elem::TF32
-                                                                                     : Elem::BF16;
-  const int terms = prec == GBPOLY_PREC_BF16X6 ? 3 : (prec == GBPOLY_PREC_TF32 ? 1 : 2);
+  const Elem e = elem_of(prec);
+  const int terms = terms_of(prec);
   const int64_t bk = e == Elem::TF32 ? 32 : 64;
   const int64_t bm = s == kTileSquare ? 128 : 256, bn = s == kTilePair ? 256 : 128;
   const int64_t tm = (M + bm - 1) / bm, tn = (N + bn - 1) / bn;
@@ -2358,10 +2362,9 @@ gbpoly_status run_grouped(gbpoly_ctx* ctx, gbpoly_grouped* g, const char* name) 
 // Tile configurations of grouped plans: 0 = 1-CTA 128 x 128 tiles (least
 // padding of small problems), 1 = CTA pairs on 256 x 256 tiles (a few large
 // products, as matmulchain's two independent stages), and for bf16x3 and
-// fp16x3 2 = 1-CTA 128 x 256 tiles.  Untuned, a group uses 1 when every problem is
-// large enough that 256 x 256 tiles pad it about as little as 128 x 128 ones
-// and the group fills at least two rounds of pairs, else 0; the autotuner
-// (gbpoly_autotune_grouped) times them per problem class.
+// fp16x3 2 = 1-CTA 128 x 256 tiles.  Untuned, a group uses the one of the least
+// estimated time (grouped_cost); the autotuner (gbpoly_autotune_grouped) times
+// them per problem class.
 using GroupBF16x3_w = FormBF16x3;
 using GroupBF16x3 = FormBF16x3_c;
 using GroupTF32x3 = FormTF32x3_c;
@@ -2375,17 +2378,36 @@ using GroupF16x3 = FormF16x3_c;
 using GroupF16x3_p = FormF16x3_p;
 using GroupF16x3_w = FormF16x3;
 
-bool grouped_pairs(gbpoly_ctx* ctx, const std::vector<gbpoly_gemm_desc>& descs) {
-  double work128 = 0, work256 = 0;
-  int64_t pair_tiles = 0;
-  for(const auto& d : descs) {
+// Estimated time of a grouped launch in configuration `config`, in
+// microseconds: its tiles in the plan's order (decreasing K) walked round
+// robin by the resident CTAs or pairs, each tile its chunks of K and its end.
+// Within 10 % of the measured time on GB300 for pairs of equal products of 512
+// to 3072 and groups of 6 to 512 problems of 64 to 2048, in bf16x3, fp16x3,
+// tf32x3 and bf16x6 (bf16x3, us, 128 x 128 / pairs, estimate in parentheses:
+// two products of 2048 102 (104) / 74 (73), of 1300 39 (40) / 31 (32); 64
+// problems 119 (111) / 128 (135)).
+double grouped_cost(gbpoly_ctx* ctx, gbpoly_precision prec, const gbpoly_gemm_desc* descs, int count, int config) {
+  const TileShape shape = config == 1 ? kTilePair : kTileSquare;
+  const Elem e = elem_of(prec);
+  const double wide = prec == GBPOLY_PREC_FP16X3 ? 1.15 : 1.09;  // a chunk of a 1-CTA 128 x 256 tile
+  const double c = config == 2 ? wide : chunk_us(e, terms_of(prec), shape);
+  const int64_t bk = e == Elem::TF32 ? 32 : 64, bm = config == 1 ? 256 : 128, bn = config == 0 ? 128 : 256;
+  const size_t cap = size_t(std::max(1, config == 1 ? ctx->sm_count / 2 : ctx->sm_count));
+  std::vector<std::pair<double, int64_t>> problems;  // time of a tile, tiles
+  for(int i = 0; i < count; ++i) {
+    const auto& d = descs[i];
     if(d.M <= 0 || d.N <= 0) continue;
-    const double k = double(std::max<int64_t>(d.K, 1));
-    work128 += double((d.M + 127) / 128 * 128) * double((d.N + 127) / 128 * 128) * k;
-    work256 += double((d.M + 255) / 256 * 256) * double((d.N + 255) / 256 * 256) * k;
-    pair_tiles += ((d.M + 255) / 256) * ((d.N + 255) / 256);
+    const double end = config == 0 ? 1.5 : (config == 1 ? (d.beta != 0.f ? 9 : 4) : (d.beta != 0.f ? 6 : 3));
+    problems.push_back({double(std::max<int64_t>(1, (d.K + bk - 1) / bk)) * c + end, ((d.M + bm - 1) / bm) * ((d.N + bn - 1) / bn)});
   }
-  return pair_tiles >= ctx->sm_count && work256 <= 1.05 * work128;
+  std::sort(problems.begin(), problems.end(), [](const auto& a, const auto& b) { return a.first > b.first; });
+  std::vector<double> busy(cap, 0.0);
+  size_t at = 0;
+  for(const auto& [t, tiles] : problems) {
+    for(auto& b : busy) b += t * double(tiles / int64_t(cap));  // whole rounds
+    for(int64_t k = tiles % int64_t(cap); k > 0; --k, at = (at + 1) % cap) busy[at] += t;
+  }
+  return *std::max_element(busy.begin(), busy.end()) + (config == 1 ? 10 : 8);
 }
 
 }  // namespace
@@ -2405,7 +2427,13 @@ int default_grouped_config(gbpoly_ctx* ctx, gbpoly_precision prec, const gbpoly_
   if(grouped_config_count(prec) == 0) return 0;
   auto it = ctx->tuned_grouped.find(group_class(prec, descs, count));
   if(it != ctx->tuned_grouped.end() && it->second < grouped_config_count(prec)) return it->second;
-  return grouped_pairs(ctx, std::vector<gbpoly_gemm_desc>(descs, descs + count)) ? 1 : 0;
+  int best = 0;
+  double best_t = grouped_cost(ctx, prec, descs, count, 0);
+  for(int c = 1; c < grouped_config_count(prec); ++c) {
+    const double t = grouped_cost(ctx, prec, descs, count, c);
+    if(t < 0.97 * best_t) best = c, best_t = t;
+  }
+  return best;
 }
 
 }  // namespace gbpoly
