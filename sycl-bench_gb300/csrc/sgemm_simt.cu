@@ -620,6 +620,10 @@ gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a) {
   const int M = int(a.M), N = int(a.N), K = int(a.K);
   const Operand oa = a_kmaj ? Operand{a.A, a.lda, M, K} : Operand{a.A, a.lda, K, M};
   const Operand ob = b_kmaj ? Operand{a.B, a.ldb, N, K} : Operand{a.B, a.ldb, K, N};
+  const bool aligned = ((reinterpret_cast<uintptr_t>(a.A) | reinterpret_cast<uintptr_t>(a.B)) & 15) == 0 &&
+                       ((a.lda | a.ldb) & 3) == 0 && K > 0;
+  if(!aligned && (a.M + 63) / 64 > 65535)  // the limit of these calls, unchanged
+    return fail(GBPOLY_ERR_UNSUPPORTED, "matrix too tall for operands off 16-byte boundaries");
   if(a.dual) return launch_sgemm<Fetch::Turn, Fetch::Turn, true>(ctx, a, oa, ob);
   const Fetch fb = fetch_of(ob, b_kmaj);
   switch(fetch_of(oa, a_kmaj)) {
