@@ -4,18 +4,26 @@
 //
 // The reference gives one work-item per column and walks the rows
 // sequentially through global memory (covariance.cpp:84-96,
-// correlation.cpp:111-142).  Here a column reduction is two launches:
-//   * partial pass: a CTA of 8 warps owns 32 adjacent columns and one chunk
-//     of rows; lane j of every warp reads column j (a warp reads 128
-//     contiguous bytes of a row), each thread keeps eight independent loads
-//     in flight, and the 8 warps are combined in shared memory into one
-//     partial sum per (chunk, column);
-//   * final pass: one thread per column adds its chunks' partials in chunk
-//     order and applies the division (and, for standard deviations, the
-//     square root and the eps clamp).
-// The chunk count is chosen so that about four CTAs per SM stream the
-// matrix; the result does not depend on the launch beyond that fixed
-// summation tree (same inputs and shape, same bits).  All arithmetic is FP32.
+// correlation.cpp:111-142).  Here a CTA of 8 warps owns 32 adjacent columns and
+// one chunk of rows; lane j of every warp reads column j (a warp reads 128
+// contiguous bytes of a row), each thread keeps sixteen independent loads in
+// flight, and the 8 warps are combined in shared memory into one partial sum
+// per (chunk, column).  Then, in chunk order, the partials are added and the
+// division (and, for standard deviations, the square root and the eps clamp)
+// applied:
+//   * wide matrices (the column blocks times eight chunks give every SM two
+//     CTAs): the chunks of a column block are a cluster, whose first CTA reads
+//     the others' partials from their shared memory: one launch;
+//   * narrow ones: partials in global memory, a second launch of one thread
+//     per column; about four CTAs per SM stream the matrix.
+// The result does not depend on the launch beyond that fixed summation tree
+// (same inputs and shape, same bits).  All arithmetic is FP32.
+//
+// Bound: HBM or L2, one read of the matrix (3000 x 2000: 3.5 us at the measured
+// copy rate); the remainder of a chunk's rows is part of the last batch of
+// loads (loaded one by one it cost as much as the batches).  Mean and standard
+// deviation together, us, partials in global memory / clusters: 4000 x 4000
+// 40.8 / 34.6, 3000 x 2000 21.5 / 21.0, 1000 x 1300 13.7 / 10.3.
 #include "gbpoly_internal.cuh"
 
 namespace gbpoly {
@@ -25,60 +33,90 @@ constexpr int kColsPerBlock = 32;
 constexpr int kWarps = 8;
 
 // sum over rows [r0, r1) of f(X[r][j]) for this thread's column j, rows
-// warp, warp + 8, ... of the chunk; eight loads in flight.
+// warp, warp + 8, ... of the chunk; sixteen loads in flight.
 template <bool CENTERED>
 __device__ __forceinline__ float column_chunk_sum(const float* __restrict__ col, int64_t ldx, int r0, int r1, int warp,
     float m) {
-  constexpr int kLoads = 8;
-  float a[kLoads];
+  constexpr int kLoads = 16, kSums = 8;
+  float a[kSums];
 #pragma unroll
-  for(int k = 0; k < kLoads; ++k) a[k] = 0.f;
-  int r = r0 + warp;
-  for(; r + (kLoads - 1) * kWarps < r1; r += kLoads * kWarps) {
+  for(int k = 0; k < kSums; ++k) a[k] = 0.f;
+  for(int r = r0 + warp; r < r1; r += kLoads * kWarps) {
     float v[kLoads];
 #pragma unroll
-    for(int k = 0; k < kLoads; ++k) v[k] = col[int64_t(r + k * kWarps) * ldx];
+    for(int k = 0; k < kLoads; ++k) {
+      const int rk = r + k * kWarps;
+      v[k] = rk < r1 ? col[int64_t(rk) * ldx] : (CENTERED ? m : 0.f);  // beyond the chunk: adds zero
+    }
 #pragma unroll
     for(int k = 0; k < kLoads; ++k) {
       if constexpr(CENTERED) {
         const float c = v[k] - m;
-        a[k] = fmaf(c, c, a[k]);
+        a[k % kSums] = fmaf(c, c, a[k % kSums]);
       } else {
-        a[k] += v[k];
+        a[k % kSums] += v[k];
       }
     }
   }
-  for(; r < r1; r += kWarps) {
-    float v = col[int64_t(r) * ldx];
-    if constexpr(CENTERED) {
-      v -= m;
-      a[0] = fmaf(v, v, a[0]);
-    } else {
-      a[0] += v;
-    }
-  }
   return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
+}
+
+// The chunk's sum for column lane of the block, in every lane of warp 0 (all threads call it).
+template <bool CENTERED>
+__device__ __forceinline__ float block_chunk_sum(const float* __restrict__ X, int64_t ldx, int cols, int r0, int r1, int j,
+    const float* __restrict__ mean) {
+  __shared__ float red[kWarps][kColsPerBlock + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float s = 0.f;
+  if(j < cols) s = column_chunk_sum<CENTERED>(X + j, ldx, r0, r1, warp, CENTERED ? mean[j] : 0.f);
+  red[warp][lane] = s;
+  __syncthreads();
+  float t = red[0][lane];
+#pragma unroll
+  for(int w = 1; w < kWarps; ++w) t += red[w][lane];
+  return t;
+}
+
+template <bool STDDEV>
+__device__ __forceinline__ float finish(float s, float divisor, float eps) {
+  s = s / divisor;
+  if constexpr(STDDEV) {
+    s = sqrtf(s);
+    s = s <= eps ? 1.f : s;
+  }
+  return s;
+}
+
+// Cluster of 1 x gridDim.y CTAs: one column block, its chunks of rows.
+template <bool STDDEV>
+__global__ void __launch_bounds__(kWarps * 32) column_cluster_kernel(const float* __restrict__ X, int64_t ldx, int rows,
+    int cols, int rows_per_chunk, const float* __restrict__ mean, float divisor, float eps, float* __restrict__ out) {
+  __shared__ float part[kColsPerBlock];
+  pdl_enter();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j = blockIdx.x * kColsPerBlock + lane;
+  const int r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
+  const float t = block_chunk_sum<STDDEV>(X, ldx, cols, r0, r1, j, mean);
+  if(warp == 0) part[lane] = t;
+  cluster_sync();
+  if(blockIdx.y == 0 && warp == 0) {
+    float s = 0.f;
+    for(unsigned c = 0; c < gridDim.y; ++c) s += ld_cluster_f32(cluster_map(&part[lane], c));
+    if(j < cols) out[j] = finish<STDDEV>(s, divisor, eps);
+  }
+  cluster_sync();  // no CTA leaves while its partials are being read
 }
 
 // partial[chunk][j] = sum over the chunk's rows of X[r][j] (or (X[r][j] - mean[j])^2).
 template <bool CENTERED>
 __global__ void __launch_bounds__(kWarps * 32) column_partial_kernel(const float* __restrict__ X, int64_t ldx, int rows,
     int cols, int rows_per_chunk, const float* __restrict__ mean, float* __restrict__ partial) {
-  __shared__ float red[kWarps][kColsPerBlock + 1];
   pdl_enter();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = blockIdx.x * kColsPerBlock + lane;
   const int r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
-  float s = 0.f;
-  if(j < cols) s = column_chunk_sum<CENTERED>(X + j, ldx, r0, r1, warp, CENTERED ? mean[j] : 0.f);
-  red[warp][lane] = s;
-  __syncthreads();
-  if(warp == 0 && j < cols) {
-    float t = red[0][lane];
-#pragma unroll
-    for(int w = 1; w < kWarps; ++w) t += red[w][lane];
-    partial[int64_t(blockIdx.y) * cols + j] = t;
-  }
+  const float t = block_chunk_sum<CENTERED>(X, ldx, cols, r0, r1, j, mean);
+  if(warp == 0 && j < cols) partial[int64_t(blockIdx.y) * cols + j] = t;
 }
 
 // out[j] = (sum of the chunks' partials) / divisor; for standard deviations
@@ -90,13 +128,9 @@ __global__ void column_final_kernel(const float* __restrict__ partial, int chunk
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if(j >= cols) return;
   float s = 0.f;
+#pragma unroll 8
   for(int c = 0; c < chunks; ++c) s += partial[int64_t(c) * cols + j];
-  s = s / divisor;
-  if constexpr(STDDEV) {
-    s = sqrtf(s);
-    s = s <= eps ? 1.f : s;
-  }
-  out[j] = s;
+  out[j] = finish<STDDEV>(s, divisor, eps);
 }
 
 // Y[r][j] = X[r][j] - mean[j], or ((X[r][j] - mean[j]) / scale_div) / stddev[j].
@@ -158,6 +192,24 @@ gbpoly_status column_reduce(gbpoly_ctx* ctx, int64_t rows, int64_t cols, const f
     float divisor, float eps, float* out) {
   if(cols == 0) return GBPOLY_OK;
   const int col_blocks = int((cols + kColsPerBlock - 1) / kColsPerBlock);
+  const int cluster = int(std::max<int64_t>(1, std::min<int64_t>(8, (rows + 63) / 64)));
+  if(int64_t(col_blocks) * 8 >= 2ll * std::max(ctx->sm_count, 1)) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[2];
+    cfg.gridDim = dim3(unsigned(col_blocks), unsigned(cluster));
+    cfg.blockDim = dim3(kWarps * 32);
+    cfg.stream = ctx->stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = unsigned(cluster), attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_pdl
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    ProfileScope prof(ctx, STDDEV ? "column_stddev" : "column_mean");
+    GBPOLY_CUDA_TRY(cudaLaunchKernelEx(&cfg, column_cluster_kernel<STDDEV>, X, ldx, int(rows), int(cols),
+        std::max(int((rows + cluster - 1) / cluster), 1), mean, divisor, eps, out));
+    return GBPOLY_OK;
+  }
   // about four CTAs per SM, at least 64 rows per chunk
   const int64_t want = std::max<int64_t>(1, (4ll * std::max(ctx->sm_count, 1) + col_blocks - 1) / col_blocks);
   const int64_t chunks = std::max<int64_t>(1, std::min<int64_t>(want, (rows + 63) / 64));

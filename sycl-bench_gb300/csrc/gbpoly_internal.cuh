@@ -401,6 +401,11 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
                : "memory");
   return v;
 }
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
 // Arrive on an mbarrier given by its cluster address (this CTA's or a
 // peer's), with the default (CTA-scope) release: the arrival only counts,
 // the data it stands for (tensor-memory reads) is ordered by tcgen05 fences.

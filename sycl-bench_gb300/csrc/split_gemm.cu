@@ -362,11 +362,10 @@ struct SplitTerms<Elem::BF16, TERMS, NV> {
 
 // K-major operands (op(X) rows contiguous in X) need no transposition: each
 // thread converts the values split_load gave it (rows t / 16 + 16 e, k
-// elements [4 (t % 16), +4)) straight into the panels, the same arithmetic as
-// split_convert (row transform included), without the shared tile.
+// elements [4 (t % 16), +4)) straight into the panels, without the shared tile.
 template <Elem E, int TERMS>
 __device__ __forceinline__ void split_convert_kmajor(const float (&v)[16], typename Term<E>::T* __restrict__ out,
-    int64_t panel_stride, int R, int Kp, int64_t r0, int64_t k0, RowXform xf = RowXform{}, int K = 0) {
+    int64_t panel_stride, int R, int Kp, int64_t r0, int64_t k0) {
   using T = typename Term<E>::T;
   const int tid = threadIdx.x;
   const int rr = tid >> 4, kc = 4 * (tid & 15);
@@ -374,16 +373,7 @@ __device__ __forceinline__ void split_convert_kmajor(const float (&v)[16], typen
   for(int e = 0; e < 4; ++e) {
     const int64_t r = r0 + rr + 16 * e;
     if(r >= R) continue;
-    float x[4] = {v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]};
-    if(xf.mean) {
-      const float m = xf.mean[r], sd = xf.sd ? xf.sd[r] : 1.f;
-#pragma unroll
-      for(int i = 0; i < 4; ++i) {
-        float y = x[i] - m;
-        if(xf.sd) y = (y / xf.div) / sd;
-        x[i] = k0 + kc + i < K ? y : 0.f;
-      }
-    }
+    const float x[4] = {v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]};
     __align__(16) T t[TERMS][4];
     SplitTerms<E, TERMS, 4>::run(x, t);
 #pragma unroll
@@ -419,22 +409,31 @@ __device__ __forceinline__ void mn_to_kmajor(const float (&v)[16], float (&w)[16
     for(int i = 0; i < 4; ++i) w[4 * e + i] = tile[o + 16 * e][4 * q + i];
 }
 
-// The row transform of split_convert_kmajor applied in place to a thread's
-// values (same arithmetic), for the F16 form, whose block scale is taken
-// after the transform.
-__device__ __forceinline__ void xform_kmajor(float (&v)[16], int R, int64_t r0, int64_t k0, const RowXform& xf, int K) {
+// A thread's four rows' values of the row transform, loaded before the block's
+// own loads are waited for, and the transform of its K-major values.
+struct RowValues {
+  float m[4], sd[4];
+};
+__device__ __forceinline__ void load_row_values(RowValues& v, const RowXform& xf, int R, int64_t r0) {
   if(!xf.mean) return;
-  const int tid = threadIdx.x;
-  const int rr = tid >> 4, kc = 4 * (tid & 15);
 #pragma unroll
   for(int e = 0; e < 4; ++e) {
-    const int64_t r = r0 + rr + 16 * e;
-    if(r >= R) continue;
-    const float m = xf.mean[r], sd = xf.sd ? xf.sd[r] : 1.f;
+    const int64_t r = r0 + (threadIdx.x >> 4) + 16 * e;
+    v.m[e] = r < R ? xf.mean[r] : 0.f;
+    v.sd[e] = xf.sd && r < R ? xf.sd[r] : 1.f;
+  }
+}
+__device__ __forceinline__ void xform_kmajor(float (&v)[16], const RowValues& row, int R, int64_t r0, int64_t k0,
+    const RowXform& xf, int K) {
+  if(!xf.mean) return;
+  const int rr = threadIdx.x >> 4, kc = 4 * (threadIdx.x & 15);
+#pragma unroll
+  for(int e = 0; e < 4; ++e) {
+    if(r0 + rr + 16 * e >= R) continue;
 #pragma unroll
     for(int i = 0; i < 4; ++i) {
-      float y = v[4 * e + i] - m;
-      if(xf.sd) y = (y / xf.div) / sd;
+      float y = v[4 * e + i] - row.m[e];
+      if(xf.sd) y = (y / xf.div) / row.sd[e];
       v[4 * e + i] = k0 + kc + i < K ? y : 0.f;
     }
   }
@@ -506,6 +505,8 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitSide a, const Spl
   if(blockIdx.x == 0)
     for(int i = threadIdx.x; i < nflags; i += 256) flags[i] = 0;
   float v[16];
+  RowValues row;
+  load_row_values(row, s.xf, s.R, r0);
   if(s.k_major) {
     split_load(s.X, s.ld, 1, s.R, K, r0, k0, v);
   } else {
@@ -514,16 +515,14 @@ __global__ void __launch_bounds__(256) split_kernel(const SplitSide a, const Spl
     mn_to_kmajor(t, v);
   }
   const int Kp = 64 * kb;
+  xform_kmajor(v, row, s.R, r0, k0, s.xf, K);
   if constexpr(E == Elem::F16) {
-    xform_kmajor(v, s.R, r0, k0, s.xf, K);
     __shared__ float red[8];
     const float sc = block_pow2_scale(v, s.inv_scale + local, red);
 #pragma unroll
     for(int i = 0; i < 16; ++i) v[i] *= sc;
-    split_convert_kmajor<E, TERMS>(v, static_cast<T*>(s.out), s.panel_stride, s.R, Kp, r0, k0);
-  } else {
-    split_convert_kmajor<E, TERMS>(v, static_cast<T*>(s.out), s.panel_stride, s.R, Kp, r0, k0, s.xf, K);
   }
+  split_convert_kmajor<E, TERMS>(v, static_cast<T*>(s.out), s.panel_stride, s.R, Kp, r0, k0);
 }
 
 // One operand of a grouped call; its 64 x 64 blocks are listed in the
