@@ -11,11 +11,12 @@
 // per (chunk, column).  Then, in chunk order, the partials are added and the
 // division (and, for standard deviations, the square root and the eps clamp)
 // applied:
-//   * wide matrices (the column blocks times eight chunks give every SM two
-//     CTAs): the chunks of a column block are a cluster, whose first CTA reads
-//     the others' partials from their shared memory: one launch;
-//   * narrow ones: partials in global memory, a second launch of one thread
-//     per column; about four CTAs per SM stream the matrix.
+//   * wide or low matrices (the column blocks times eight chunks give every SM
+//     two CTAs, or a chunk has at most 384 rows): the chunks of a column block
+//     are a cluster, whose first CTA reads the others' partials from their
+//     shared memory: one launch;
+//   * high, narrow ones: partials in global memory, a second launch of one
+//     thread per column; about four CTAs per SM stream the matrix.
 // The result does not depend on the launch beyond that fixed summation tree
 // (same inputs and shape, same bits).  All arithmetic is FP32.
 //
@@ -23,7 +24,8 @@
 // copy rate); the remainder of a chunk's rows is part of the last batch of
 // loads (loaded one by one it cost as much as the batches).  Mean and standard
 // deviation together, us, partials in global memory / clusters: 4000 x 4000
-// 40.8 / 34.6, 3000 x 2000 21.5 / 21.0, 1000 x 1300 13.7 / 10.3.
+// 40.8 / 34.6, 3000 x 2000 21.5 / 21.0, 1000 x 1300 13.7 / 10.3, 1000 x 300 9.8 /
+// 6.8, 3000 x 160 14.0 / 9.7; 4096 x 600 12.8 / 19.2.
 #include "gbpoly_internal.cuh"
 
 namespace gbpoly {
@@ -193,7 +195,7 @@ gbpoly_status column_reduce(gbpoly_ctx* ctx, int64_t rows, int64_t cols, const f
   if(cols == 0) return GBPOLY_OK;
   const int col_blocks = int((cols + kColsPerBlock - 1) / kColsPerBlock);
   const int cluster = int(std::max<int64_t>(1, std::min<int64_t>(8, (rows + 63) / 64)));
-  if(int64_t(col_blocks) * 8 >= 2ll * std::max(ctx->sm_count, 1)) {
+  if(int64_t(col_blocks) * 8 >= 2ll * std::max(ctx->sm_count, 1) || rows <= 8 * 384) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     cfg.gridDim = dim3(unsigned(col_blocks), unsigned(cluster));

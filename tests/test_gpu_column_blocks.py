@@ -15,7 +15,7 @@ U = 2.0 ** -24
 
 @pytest.mark.parametrize("pad", [0, 1])
 @pytest.mark.parametrize("shape", [(1, 1), (7, 33), (65, 31), (513, 40), (1, 1300), (63, 1249), (130, 1216), (1030, 1217),
-                                   (129, 2050)], ids=str)
+                                   (129, 2050), (3073, 70)], ids=str)
 def test_mean_and_stddev(ctx, shape, pad):
     rows, cols = shape
     rng = np.random.default_rng(rows + cols + pad)
