@@ -192,8 +192,28 @@ __device__ __forceinline__ void lower_coords(int t, int& tile_m, int& tile_n) {
   tile_n = t - tm * (tm + 1) / 2;
 }
 
+// syr2k's walk: the tiles below the diagonal, then the diagonal ones, which take half as long.
+__device__ __forceinline__ void dual_coords(int t, int tiles, int& tile_m, int& tile_n) {
+  const int below = tiles * (tiles - 1) / 2;
+  if(t < below) {
+    lower_coords(t, tile_m, tile_n);
+    ++tile_m;
+  } else {
+    tile_m = tile_n = t - below;
+  }
+}
+
 // FA, FB: how op(A)'s and op(B)'s tiles are fetched.  DUAL: syr2k (both
-// operands K-major), tiles A_i, B_j, B_i, A_j.
+// operands K-major), tiles A_i, B_j, B_i, A_j.  On the diagonal the second
+// product is the first one's transpose, S + S^T: half the copies and half the
+// products, the transpose added through shared memory before the exchange.
+// (1536: 78 tiles, 12 of them diagonal, as 78 clusters of two on 76 places;
+// the last two start when the first diagonal ones end.  132 us against 176
+// with both products on every tile, then best as clusters of three in two
+// rounds; 512 25.2 -> 20.8, 1280 135 -> 105.  Sizes that run unsplit in whole
+// rounds of clusters gain nothing and lose up to 1.6 % to the branch around
+// the second product, 2048 330 -> 335; the loop written twice lost 4 % there,
+// one body run once or twice 2 % at 1024.)
 //
 // K split: the gridDim.y CTAs of a cluster take consecutive K ranges of one
 // tile.  Each writes its sums to its own shared memory (the drained ring);
@@ -220,10 +240,13 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
   const int warp = tid >> 5, lane = tid & 31;
   const int tiles_m = (M + kBM - 1) / kBM, tiles_n = (N + kBN - 1) / kBN;
   int tile_m, tile_n;
-  if(lower)
+  if constexpr(DUAL)
+    dual_coords(blockIdx.x, tiles_m, tile_m, tile_n);
+  else if(lower)
     lower_coords(blockIdx.x, tile_m, tile_n);
   else
     tile_coords(blockIdx.x, tiles_m, tiles_n, tile_m, tile_n);
+  const bool diagonal = DUAL && tile_m == tile_n;
   const int m0 = tile_m * kBM, n0 = tile_n * kBN;
   const bool mirror = lower && tile_m != tile_n;
   const int splits = int(gridDim.y), split = int(blockIdx.y);  // the cluster is 1 x splits: split == rank
@@ -266,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
           const uint32_t d = smem_u32(st);
           if constexpr(FA != Fetch::Tma) fetch_words<FA>(d, oa, m0, k0);
           if constexpr(FB != Fetch::Tma) fetch_words<FB>(d + kTileBytes, ob, n0, k0);
-          if constexpr(DUAL) {
+          if(DUAL && !diagonal) {
             fetch_words<FB>(d + 2 * kTileBytes, ob, m0, k0);
             fetch_words<FA>(d + 3 * kTileBytes, oa, n0, k0);
           }
@@ -320,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
     }
     const char* st = smem + s * kStageBytes;
     mma_tile<FA == Fetch::Turn, FB == Fetch::Turn>(st, st + kTileBytes, 4 * wr + 16 * li, 4 * wc + 16 * lj, acc2);
-    if constexpr(DUAL)
+    if(DUAL && !diagonal)
       mma_tile<true, true>(st + 2 * kTileBytes, st + 3 * kTileBytes, 4 * wr + 16 * li, 4 * wc + 16 * lj, acc2);
     __syncwarp();
     if(lane == 0) mbar_arrive(&empty[s]);
@@ -382,6 +405,22 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
     if(c + 3 < N) p[3 * ldc] = fmaf(beta, old.w, alpha * s.w);
   };
 
+  if(DUAL && diagonal) {
+    asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");  // as before the exchange below
+    constexpr int kPitch = kBN + 1;
+    float* t = reinterpret_cast<float*>(smem);
+#pragma unroll
+    for(int f = 0; f < 16; ++f) {
+      float* q = t + (row_of(f) - m0) * kPitch + col_of(f) - n0;
+      q[0] = acc[f].x, q[1] = acc[f].y, q[2] = acc[f].z, q[3] = acc[f].w;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");
+#pragma unroll
+    for(int f = 0; f < 16; ++f) {
+      const float* q = t + (col_of(f) - n0) * kPitch + row_of(f) - m0;
+      acc[f].x += q[0], acc[f].y += q[kPitch], acc[f].z += q[2 * kPitch], acc[f].w += q[3 * kPitch];
+    }
+  }
   if(splits > 1) {
     // every consumer warp has read its last stage, every copy has landed (each was waited for)
     asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");
@@ -508,14 +547,26 @@ gbpoly_status cluster_capacity(gbpoly_ctx* ctx, int (&cap)[kMaxSplit + 1]) {
   return GBPOLY_OK;
 }
 
-// K split of a launch of `tiles` tiles (measured on GB300, all splits 1 to 8 of
-// eighteen shapes: within 4 % of the fastest but for syr2k at 512, 27 against
-// 23 us; gemm 1024 47 us with 2 against 59 with a workspace split and its
-// reduction launch, syr2k 1536 178 with 3 against 299 unsplit, 2048 and up unsplit) of `ktiles` k tiles each: the count
-// whose rounds of clusters take the least time, in units of one k tile's
-// products: each CTA spends its share of the k tiles, a fixed part (launch,
-// first copies, C) and, when split, the exchange of sums.
-int best_split(const int (&cap)[kMaxSplit + 1], int64_t tiles, int64_t ktiles, bool dual) {
+// Time of `whole` tiles of u and then `half` of h on n places: the half ones on
+// the places that the last round leaves free, however long these take, or on
+// those until the round ends and then on all.
+double span(int64_t whole, double u, int64_t half, double h, int n) {
+  const int64_t busy = whole % n;
+  const double begin = double(whole / n) * u, end = begin + (busy ? u : 0);
+  if(half == 0) return end;
+  const int64_t early = busy ? std::min<int64_t>(half, (n - busy) * int64_t(u / h)) : 0;
+  const double beside = begin + double((half + n - busy - 1) / (n - busy)) * h;
+  return std::min(std::max(end, beside), end + double((half - early + n - 1) / n) * h);
+}
+
+// K split of a launch of `tiles` tiles and, syr2k, `diagonal` ones of half the
+// work, of `ktiles` k tiles each: the count whose clusters take the least
+// time, in units of one k tile's products.  Each CTA spends its share of the k
+// tiles, a fixed part (launch, first copies, C) and, when split, the exchange
+// of sums.  Measured on GB300, all splits 1 to 8 of eighteen shapes: within
+// 4 % of the fastest (gemm 1024 47 us with 2 against 59 with a workspace split
+// and its reduction launch; syr2k 1536 132 with 2 against 299 unsplit).
+int best_split(const int (&cap)[kMaxSplit + 1], int64_t tiles, int64_t diagonal, int64_t ktiles, bool dual) {
   const double unit = dual ? 2.0 : 1.0;  // syr2k: a k tile is two products
   int best = 1;
   double best_t = 0;
@@ -523,7 +574,8 @@ int best_split(const int (&cap)[kMaxSplit + 1], int64_t tiles, int64_t ktiles, b
     if(cap[s] <= 0) continue;
     const int64_t per = (ktiles + s - 1) / s;
     if(s > 1 && (ktiles + per - 1) / per != s) continue;  // an empty split
-    const double t = double((tiles + cap[s] - 1) / cap[s]) * (unit * double(per) + kFixedTiles + (s > 1 ? kSplitTiles : 0));
+    const double fixed = kFixedTiles + (s > 1 ? kSplitTiles : 0);
+    const double t = span(tiles, unit * double(per) + fixed, diagonal, double(per) + fixed, cap[s]);
     if(s == 1 || t < 0.97 * best_t) best = s, best_t = t;
   }
   return best;
@@ -538,8 +590,11 @@ gbpoly_status split_count(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, bool
   gbpoly_status st = cluster_capacity(ctx, cap);
   if(st != GBPOLY_OK) return st;
   const int64_t tm = (M + kBM - 1) / kBM, tn = (N + kBN - 1) / kBN;
-  const int64_t tiles = lower && tm * tn > 25 ? tm * (tm + 1) / 2 : tm * tn;
-  splits = best_split(cap, tiles, (K + kBK - 1) / kBK, dual);
+  const int64_t ktiles = (K + kBK - 1) / kBK;
+  if(dual)
+    splits = best_split(cap, tm * (tm - 1) / 2, tm, ktiles, true);
+  else
+    splits = best_split(cap, lower && tm * tn > 25 ? tm * (tm + 1) / 2 : tm * tn, 0, ktiles, false);
   return GBPOLY_OK;
 }
 
