@@ -158,6 +158,14 @@ struct RowXform {
   float div = 1.f;
 };
 
+// K split of an FP32 contraction, in CTAs per output tile: `first` in the rows
+// of C before row `rows`, `rest` (1 or more, 0: chosen from the shape) in the
+// others.
+struct Fp32Split {
+  int64_t rows = 0;
+  int first = 1, rest = 0;
+};
+
 struct GemmF32Args {
   int64_t M, N, K;
   float alpha, beta;
@@ -174,10 +182,11 @@ struct GemmF32Args {
   int64_t lda2 = 0;
   const float* B2 = nullptr;
   int64_t ldb2 = 0;
-  // FP32 only: K split count (0: chosen from the shape; 1: none).  Callers
-  // that run a contraction in row panels pass the full shape's split so the
-  // panels add K in the same order as the whole call.
-  int ksplit = 0;
+  // FP32 only: the K split.  Callers that run a contraction in row panels pass
+  // the full shape's split and the panel's first row, so that the panels add K
+  // in the same order as the whole call.
+  Fp32Split split;
+  int64_t split_row = 0;
   // Tensor-core forms, symmetric products only: transform of op(A)'s rows.
   RowXform xf;
 };
@@ -193,9 +202,8 @@ gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a);
 // shared memory of its clusters and needs none of it; the figure stays for
 // callers that reserve by it.
 size_t fp32_split_k_bytes(int sm_count, int64_t M, int64_t N, int64_t K);
-// The K split count gbpoly_gemm_f32 uses for a non-symmetric FP32 contraction
-// of this shape (1: no split).
-gbpoly_status fp32_split_k_count(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, int& splits);
+// The K split gbpoly_gemm_f32 uses for a non-symmetric FP32 contraction of this shape.
+gbpoly_status fp32_split(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, Fp32Split& split);
 // Tensor-core forms (split_gemm.cu): tf32, bf16x3, tf32x3, bf16x6, fp16x3,
 // fp8.  The split term panels live in the context workspace.
 gbpoly_status launch_gemm_tensor(gbpoly_ctx* ctx, gbpoly_precision prec, const GemmF32Args& a);

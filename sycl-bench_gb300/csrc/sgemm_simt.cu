@@ -559,58 +559,90 @@ double span(int64_t whole, double u, int64_t half, double h, int n) {
   return std::min(std::max(end, beside), end + double((half - early + n - 1) / n) * h);
 }
 
-// K split of a launch of `tiles` tiles and, syr2k, `diagonal` ones of half the
-// work, of `ktiles` k tiles each: the count whose clusters take the least
-// time, in units of one k tile's products.  Each CTA spends its share of the k
-// tiles, a fixed part (launch, first copies, C) and, when split, the exchange
-// of sums.  Measured on GB300, all splits 1 to 8 of eighteen shapes: within
-// 4 % of the fastest (gemm 1024 47 us with 2 against 59 with a workspace split
-// and its reduction launch; syr2k 1536 132 with 2 against 299 unsplit).
-int best_split(const int (&cap)[kMaxSplit + 1], int64_t tiles, int64_t diagonal, int64_t ktiles, bool dual) {
-  const double unit = dual ? 2.0 : 1.0;  // syr2k: a k tile is two products
+// Time of a launch of `tiles` tiles and, syr2k, `diagonal` ones of half the
+// work, of `ktiles` k tiles each, split over clusters of s, in units of one k
+// tile's products; negative where such a launch is not made.  Each CTA spends
+// its share of the k tiles, a fixed part (launch, first copies, C) and, when
+// split, the exchange of sums.
+double split_time(const int (&cap)[kMaxSplit + 1], int64_t tiles, int64_t diagonal, int64_t ktiles, bool dual, int s) {
+  if(cap[s] <= 0) return -1;
+  const int64_t per = (ktiles + s - 1) / s;
+  if(s > 1 && (s > ktiles || (ktiles + per - 1) / per != s)) return -1;  // an empty split
+  const double unit = dual ? 2.0 : 1.0;                                   // syr2k: a k tile is two products
+  const double fixed = kFixedTiles + (s > 1 ? kSplitTiles : 0);
+  return span(tiles, unit * double(per) + fixed, diagonal, double(per) + fixed, cap[s]);
+}
+
+// The split that takes the least time.  Measured on GB300, all splits 1 to 8
+// of eighteen shapes: within 4 % of the fastest (gemm 1024 47 us with 2
+// against 59 with a workspace split and its reduction launch; syr2k 1536 132
+// with 2 against 299 unsplit).
+int best_split(const int (&cap)[kMaxSplit + 1], int64_t tiles, int64_t diagonal, int64_t ktiles, bool dual,
+    double* time = nullptr) {
   int best = 1;
-  double best_t = 0;
-  for(int s = 1; s <= kMaxSplit && s <= std::max<int64_t>(ktiles, 1); ++s) {
-    if(cap[s] <= 0) continue;
-    const int64_t per = (ktiles + s - 1) / s;
-    if(s > 1 && (ktiles + per - 1) / per != s) continue;  // an empty split
-    const double fixed = kFixedTiles + (s > 1 ? kSplitTiles : 0);
-    const double t = span(tiles, unit * double(per) + fixed, diagonal, double(per) + fixed, cap[s]);
-    if(s == 1 || t < 0.97 * best_t) best = s, best_t = t;
+  double best_t = split_time(cap, tiles, diagonal, ktiles, dual, 1);
+  for(int s = 2; s <= kMaxSplit; ++s) {
+    const double t = split_time(cap, tiles, diagonal, ktiles, dual, s);
+    if(t >= 0 && t < 0.97 * best_t) best = s, best_t = t;
   }
+  if(time) *time = best_t;
   return best;
 }
 
-// The K split of an FP32 contraction.  A symmetric product launches the lower
+// A contraction of a few rounds as two launches, by rows of tiles: the first
+// one full rounds of clusters of one size, the rest split on its own.  The
+// bits of an output depend on its row's split alone, so row panels give the
+// whole call's.  1007 x 2632 x 400 66 -> 50 us, 1501 x 1023 x 2047 (72 tiles as
+// pairs, 24 as clusters of five) 142 -> 130, 2048 cubed 320 -> 295; of 35
+// shapes of 200 to 4000 twelve took two launches, ten of them 1.5 to 31 %
+// faster, two 2 % slower.  Not beyond four rounds of CTAs, where the last one
+// matters less and the search takes longer.  Products of at most 25 tiles stay
+// one launch: their symmetric form gives their bits (triangle_split).
+void best_regions(const int (&cap)[kMaxSplit + 1], int64_t tm, int64_t tn, int64_t ktiles, Fp32Split& split) {
+  constexpr double kSecondLaunch = 0.5, kWorth = 0.96;
+  double best;
+  split = Fp32Split{0, 1, best_split(cap, tm * tn, 0, ktiles, false, &best)};
+  if(tm * tn <= 25 || tm * tn > 4 * cap[1]) return;
+  best *= kWorth;
+  for(int s = 1; s <= kMaxSplit; ++s) {
+    if(split_time(cap, 1, 0, ktiles, false, s) < 0) continue;
+    for(int64_t rows, round = 1; (rows = round * cap[s] / tn) < tm; ++round) {
+      if(rows == 0) continue;
+      double rest;
+      const int r = best_split(cap, (tm - rows) * tn, 0, ktiles, false, &rest);
+      const double t = split_time(cap, rows * tn, 0, ktiles, false, s) + rest + kSecondLaunch;
+      if(t < best) best = t, split = Fp32Split{rows * kBM, s, r};
+    }
+  }
+}
+
+// The K split of a symmetric FP32 contraction, which launches the lower
 // triangle of tiles; small ones take the full square's split all the same, so
 // that they give the bits of the same product computed in full (with at most
 // 25 tiles the full square's split is 6 to 8, near the limit of 8 in any case).
-gbpoly_status split_count(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, bool lower, bool dual, int& splits) {
+gbpoly_status triangle_split(gbpoly_ctx* ctx, int64_t M, int64_t K, bool dual, int& splits) {
   int cap[kMaxSplit + 1] = {};
   gbpoly_status st = cluster_capacity(ctx, cap);
   if(st != GBPOLY_OK) return st;
-  const int64_t tm = (M + kBM - 1) / kBM, tn = (N + kBN - 1) / kBN;
-  const int64_t ktiles = (K + kBK - 1) / kBK;
+  const int64_t tm = (M + kBM - 1) / kBM, ktiles = (K + kBK - 1) / kBK;
   if(dual)
     splits = best_split(cap, tm * (tm - 1) / 2, tm, ktiles, true);
   else
-    splits = best_split(cap, lower && tm * tn > 25 ? tm * (tm + 1) / 2 : tm * tn, 0, ktiles, false);
+    splits = best_split(cap, tm * tm > 25 ? tm * (tm + 1) / 2 : tm * tm, 0, ktiles, false);
   return GBPOLY_OK;
 }
 
+// splits 0: symmetric product (op(A) == op(B)^T as stored, or syr2k), the lower triangle of tiles only.
 template <Fetch FA, Fetch FB, bool DUAL>
-gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob) {
+gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob, int splits) {
   using Kn = Kernel<FA, FB, DUAL>;
-  // Symmetric product (op(A) == op(B)^T as stored, or syr2k): lower triangle of tiles only.
-  const bool lower = a.M == a.N && (DUAL || symmetric_operand(a));
+  const bool lower = splits == 0;
   gbpoly_status st = Kn::prepare(ctx);
   if(st != GBPOLY_OK) return st;
   const int64_t tm = (a.M + kBM - 1) / kBM, tn = (a.N + kBN - 1) / kBN, ktiles = (a.K + kBK - 1) / kBK;
   const int64_t tiles = lower ? tm * (tm + 1) / 2 : tm * tn;
   if(tiles >= (1ll << 31)) return fail(GBPOLY_ERR_UNSUPPORTED, "too many output tiles");
-  int splits = a.ksplit;
-  if(splits <= 0 && (st = split_count(ctx, a.M, a.N, a.K, lower, DUAL, splits)) != GBPOLY_OK) return st;
-  splits = int(std::min<int64_t>(splits, std::max<int64_t>(ktiles, 1)));
+  if(lower && (st = triangle_split(ctx, a.M, a.K, DUAL, splits)) != GBPOLY_OK) return st;
   const int kt_per_split = int((ktiles + splits - 1) / splits);
   CUtensorMap ta = {}, tb = {};
   auto map = [&](CUtensorMap* t, const Operand& o) {
@@ -627,11 +659,11 @@ gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand&
 }
 
 template <Fetch FA>
-gbpoly_status launch_left(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob, Fetch fb) {
+gbpoly_status launch_left(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob, Fetch fb, int splits) {
   switch(fb) {
-  case Fetch::Tma: return launch_sgemm<FA, Fetch::Tma, false>(ctx, a, oa, ob);
-  case Fetch::Rows: return launch_sgemm<FA, Fetch::Rows, false>(ctx, a, oa, ob);
-  default: return launch_sgemm<FA, Fetch::Turn, false>(ctx, a, oa, ob);
+  case Fetch::Tma: return launch_sgemm<FA, Fetch::Tma, false>(ctx, a, oa, ob, splits);
+  case Fetch::Rows: return launch_sgemm<FA, Fetch::Rows, false>(ctx, a, oa, ob, splits);
+  default: return launch_sgemm<FA, Fetch::Turn, false>(ctx, a, oa, ob, splits);
   }
 }
 
@@ -644,8 +676,11 @@ Fetch fetch_of(const Operand& o, bool k_major) {
 
 }  // namespace
 
-gbpoly_status fp32_split_k_count(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, int& splits) {
-  return split_count(ctx, M, N, K, false, false, splits);
+gbpoly_status fp32_split(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, Fp32Split& split) {
+  int cap[kMaxSplit + 1] = {};
+  gbpoly_status st = cluster_capacity(ctx, cap);
+  if(st == GBPOLY_OK) best_regions(cap, (M + kBM - 1) / kBM, (N + kBN - 1) / kBN, (K + kBK - 1) / kBK, split);
+  return st;
 }
 
 size_t fp32_split_k_bytes(int sm_count, int64_t M, int64_t N, int64_t K) {
@@ -679,13 +714,30 @@ gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a) {
                        ((a.lda | a.ldb) & 3) == 0 && K > 0;
   if(!aligned && (a.M + 63) / 64 > 65535)  // the limit of these calls, unchanged
     return fail(GBPOLY_ERR_UNSUPPORTED, "matrix too tall for operands off 16-byte boundaries");
-  if(a.dual) return launch_sgemm<Fetch::Turn, Fetch::Turn, true>(ctx, a, oa, ob);
+  if(a.dual) return launch_sgemm<Fetch::Turn, Fetch::Turn, true>(ctx, a, oa, ob, 0);
   const Fetch fb = fetch_of(ob, b_kmaj);
-  switch(fetch_of(oa, a_kmaj)) {
-  case Fetch::Tma: return launch_left<Fetch::Tma>(ctx, a, oa, ob, fb);
-  case Fetch::Rows: return launch_left<Fetch::Rows>(ctx, a, oa, ob, fb);
-  default: return launch_left<Fetch::Turn>(ctx, a, oa, ob, fb);
-  }
+  auto launch = [&](const GemmF32Args& part, const Operand& left, int splits) {
+    switch(fetch_of(left, a_kmaj)) {
+    case Fetch::Tma: return launch_left<Fetch::Tma>(ctx, part, left, ob, fb, splits);
+    case Fetch::Rows: return launch_left<Fetch::Rows>(ctx, part, left, ob, fb, splits);
+    default: return launch_left<Fetch::Turn>(ctx, part, left, ob, fb, splits);
+    }
+  };
+  if(symmetric_operand(a)) return launch(a, oa, 0);
+  Fp32Split split = a.split;
+  gbpoly_status st = GBPOLY_OK;
+  if(split.rest == 0 && (st = fp32_split(ctx, a.M, a.N, a.K, split)) != GBPOLY_OK) return st;
+  const int m1 = int(std::clamp<int64_t>(split.rows - a.split_row, 0, a.M));  // rows of the first region
+  if(m1 == M) return launch(a, oa, split.first);
+  if(m1 == 0) return launch(a, oa, split.rest);
+  GemmF32Args top = a, below = a;
+  top.M = m1, below.M = M - m1;
+  below.C += m1 * a.ldc;
+  const Operand left_top = a_kmaj ? Operand{a.A, a.lda, m1, K} : Operand{a.A, a.lda, K, m1};
+  const Operand left_below =
+      a_kmaj ? Operand{a.A + m1 * a.lda, a.lda, M - m1, K} : Operand{a.A + m1, a.lda, K, M - m1};
+  if((st = launch(top, left_top, split.first)) != GBPOLY_OK) return st;
+  return launch(below, left_below, split.rest);
 }
 
 }  // namespace gbpoly
