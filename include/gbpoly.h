@@ -109,9 +109,9 @@ gbpoly_status gbpoly_memset(gbpoly_ctx* ctx, void* dst, int value, size_t bytes)
  * least `bytes` large now, so that later calls of that size do not allocate.
  * Needed before capturing tensor-core calls into a graph.  Synchronises. */
 gbpoly_status gbpoly_workspace_reserve(gbpoly_ctx* ctx, size_t bytes);
-/* Workspace bytes a contraction of this shape and form needs (fp32: the
- * partial products of its K split, used when the output tiles are too few
- * to fill the device; 0 otherwise). */
+/* Workspace bytes a contraction of this shape and form needs at most (fp32:
+ * its kernels need none; for shapes whose output tiles are too few to fill the
+ * device the partial products of a K split are still reported). */
 gbpoly_status gbpoly_workspace_query(gbpoly_precision prec, int64_t M, int64_t N, int64_t K, int same_operand,
     size_t* bytes);
 
@@ -127,8 +127,8 @@ gbpoly_status gbpoly_workspace_query(gbpoly_precision prec, int64_t M, int64_t N
  * one per (form, ceil(log2) of M, N, K); unless tuned or set, a shape whose
  * 256 x 256 tiles give every SM pair a tile uses configuration 5 up to
  * K = 128 (tf32: 512, tf32x3, bf16x6: 64), 6 up to K = 384 (tf32x3: 192) and 3
- * beyond (fp16x3: 3, then 2), a smaller or symmetric one the tile shape (128 x 128, 256 x 256, 256 x 128) of the least
- * estimated time.  fp8: configuration 1 (128 x 256 tiles) when its tiles give
+ * beyond (fp16x3: 3, then 2), a smaller or symmetric one the tile shape
+ * (128 x 128, 256 x 256, 256 x 128) of the least estimated time.  fp8: configuration 1 (128 x 256 tiles) when its tiles give
  * every SM one, else 0 (128 x 128, also every symmetric product). */
 gbpoly_status gbpoly_gemm_config_count(gbpoly_precision prec, int* count);
 gbpoly_status gbpoly_gemm_config_set(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K,

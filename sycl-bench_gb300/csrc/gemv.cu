@@ -17,8 +17,9 @@
 //     32-row block, into one partial per (column tile, row);
 //   * column sums: 4 accumulators per thread over all rows of the group,
 //     one partial per (row group, column);
-//   * a final kernel (16 warps per 32 outputs) adds the partials in a fixed order and applies
-//     y = beta * y + alpha * sum (gesummv: tmp += A x, y = alpha tmp + beta (y + B x)).
+//   * a final kernel (16 warps per 32 outputs) adds the partials in a fixed
+//     order and applies y = beta * y + alpha * sum (gesummv: tmp += A x,
+//     y = alpha tmp + beta (y + B x)).
 // Deterministic: the summation tree depends only on the shape and SM count.
 #include "gbpoly_internal.cuh"
 
@@ -49,8 +50,8 @@ struct GemvArgs {
 
 // The four columns of thread t in a 1024-column tile starting at c0: 4 t .. + 3
 // (VEC), or t, t + 256, t + 512, t + 768, so that every 32-bit load of a warp is
-// one 128-byte segment (measured with odd rows: bicg 6990 x 12897 70.8 -> YY us,
-// gesummv 8434 x 6453 89.5 -> YY, against 4 t .. + 3 in both cases).
+// one 128-byte segment (measured with odd rows, against 4 t .. + 3 and the final
+// kernel of 8 warps: bicg 7000 x 7001 48.9 -> 41.8 us, gesummv 76.3 -> 66.9).
 template <bool VEC>
 __device__ __forceinline__ float4 load4(const float* __restrict__ p, int c0, int cols) {
   const int t = threadIdx.x;

@@ -13,9 +13,9 @@
 //                          2^e per 64x64 operand block (FP32's range)        22
 //   fp8       E4M3  1      a0.b0, each operand with one scale per 128x128 block   4
 // Two kernels per call:
-//   * split_kernel (memory bound): writes the K-major term panels of an
-//     operand into the context workspace (an MN-major operand transposed by
-//     the register assignment), K padded with zeros to the k-block; for FP16
+//   * split_kernel (memory bound): writes the K-major term panels of both
+//     operands into the context workspace (an MN-major operand's blocks turned
+//     through a shared tile), K padded with zeros to the k-block; for FP16
 //     terms also each block's inverse scale;
 //   * split_gemm_kernel: persistent (one CTA per SM walks 128 x BN tiles of
 //     C), warp specialised, 384 threads:
@@ -31,13 +31,16 @@
 //                   TMEM lane quarter) x BN/2 columns and sums the chunks in
 //                   FP32 registers with round-to-nearest adds (scaled forms:
 //                   times the chunk's left x right block factor), then writes
-//                   C = alpha*acc + beta*C (through a per-warp staging tile,
-//                   or, in the C-tile configurations, through TMA-loaded and
-//                   TMA-stored boxes of C in shared memory).
+//                   C = alpha*acc + beta*C (through a per-warp staging tile;
+//                   where TMA can address C's rows, through boxes of C in
+//                   shared memory: the whole tile beside a short pipeline,
+//                   the drained ring of a launch of one round, or box by box
+//                   over several rounds: Epi).
 //     CTA-pair configurations (cluster of two, cta_group::2) compute 256 x BN
 //     tiles, each CTA staging 128 rows of A and BN/2 rows of B; when a
-//     launch's last round of tiles would leave half the pairs or more idle,
-//     its tiles run as two K halves on two pairs (the K-split tail).
+//     launch's last round of tiles would leave half the pairs or more idle
+//     and half a tile takes longer than the handoff, its tiles run as two K
+//     halves on two pairs (the K-split tail).
 //     The tensor core accumulates with truncation: over long K its error
 //     grows with the number of MMA steps (measured 3.6e-6 normwise at K=512
 //     for 24-bit operand splits, against 2.6e-7 for the same products summed
@@ -152,7 +155,7 @@ struct Form {
   static constexpr bool HALVES = CG == 2 && BN == BM_CTA;
   static constexpr bool MIRROR = BM == BN || HALVES;
   // a chunk's time, for the decision to split K
-  static constexpr double CHUNK_US = chunk_us(E, TERMS, BN == 128 ? kTileNarrow : kTilePair);
+  [[maybe_unused]] static constexpr double CHUNK_US = chunk_us(E, TERMS, BN == 128 ? kTileNarrow : kTilePair);
   static constexpr int THREADS = 384;  // warpgroup 0: producer, MMA; warpgroups 1-2: epilogue
   static constexpr uint32_t REGS_CTRL = 56, REGS_EPI = 208;
   static constexpr uint32_t IDESC = idesc_of<E, BM, BN>();
