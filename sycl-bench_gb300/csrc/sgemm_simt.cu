@@ -224,7 +224,7 @@ __device__ __forceinline__ void dual_coords(int t, int tiles, int& tile_m, int& 
 template <Fetch FA, Fetch FB, bool DUAL, int STAGES>
 __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constant__ CUtensorMap tmA,
     const __grid_constant__ CUtensorMap tmB, const Operand oa, const Operand ob, int M, int N, int K,
-    float alpha, float beta, float* __restrict__ C, int64_t ldc, int lower, int kt_per_split, int* err) {
+    float alpha, float beta, float* __restrict__ C, int64_t ldc, int lower, int first_tile, int kt_per_split, int* err) {
   constexpr int kTilesPerStage = DUAL ? 4 : 2;
   constexpr int kStageBytes = kTilesPerStage * kTileBytes;
   constexpr int kTmaTiles = DUAL ? 0 : int(FA == Fetch::Tma) + int(FB == Fetch::Tma);
@@ -241,9 +241,9 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
   const int tiles_m = (M + kBM - 1) / kBM, tiles_n = (N + kBN - 1) / kBN;
   int tile_m, tile_n;
   if constexpr(DUAL)
-    dual_coords(blockIdx.x, tiles_m, tile_m, tile_n);
+    dual_coords(first_tile + blockIdx.x, tiles_m, tile_m, tile_n);
   else if(lower)
-    lower_coords(blockIdx.x, tile_m, tile_n);
+    lower_coords(first_tile + blockIdx.x, tile_m, tile_n);
   else
     tile_coords(blockIdx.x, tiles_m, tiles_n, tile_m, tile_n);
   const bool diagonal = DUAL && tile_m == tile_n;
@@ -520,8 +520,15 @@ struct Kernel {
   };
 };
 
-// Clusters of 1 x s CTAs resident at once on the context's device (one CTA
-// per SM in every variant of the kernel, so one query serves them all).
+// Clusters of 1 x s CTAs to count on at once on the context's device (one CTA
+// per SM in every variant of the kernel, so one query serves them all).  GB300
+// reports 152, 76, 46, 36, 28, 23, 15 and 15.  Those of 2, 4 and 8 are reached
+// (36 tiles as clusters of four in one round: syrk 1024 28.7 us); odd ones do
+// not always pack so tightly, the less while the previous launch is ending, and
+// one that finds no place takes a round of its own: 429 x 882 x 768, 28 tiles,
+// 36.9 us as clusters of five, 22.8 of four; syrk 1536 118 us with 46 clusters
+// of three in its first launch, 87 with two.  Hence a sixteenth less for these,
+// though no fewer than of the next power of two.
 gbpoly_status cluster_capacity(gbpoly_ctx* ctx, int (&cap)[kMaxSplit + 1]) {
   using K = Kernel<Fetch::Tma, Fetch::Tma, false>;
   static std::atomic<int> known_cap[32][kMaxSplit + 1];
@@ -540,6 +547,7 @@ gbpoly_status cluster_capacity(gbpoly_ctx* ctx, int (&cap)[kMaxSplit + 1]) {
     GBPOLY_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, K::fn, &l.cfg));
     cap[s] = n;  // 0: no cluster of this size
   }
+  for(int s : {3, 5, 6, 7}) cap[s] = std::max(cap[s] * 15 / 16, cap[s < 4 ? 4 : 8]);
   if(ctx->device >= 0 && ctx->device < 32) {
     for(int s = 1; s <= kMaxSplit; ++s) known_cap[ctx->device][s] = cap[s];
     known.set(ctx->device);
@@ -589,6 +597,10 @@ int best_split(const int (&cap)[kMaxSplit + 1], int64_t tiles, int64_t diagonal,
   return best;
 }
 
+// Two launches for one contraction: the second one's time besides its CTAs',
+// in k tiles' time, and the share of the single launch's time they have to beat.
+constexpr double kSecondLaunch = 0.5, kWorth = 0.96;
+
 // A contraction of a few rounds as two launches, by rows of tiles: the first
 // one full rounds of clusters of one size, the rest split on its own.  The
 // bits of an output depend on its row's split alone, so row panels give the
@@ -599,7 +611,6 @@ int best_split(const int (&cap)[kMaxSplit + 1], int64_t tiles, int64_t diagonal,
 // matters less and the search takes longer.  Products of at most 25 tiles stay
 // one launch: their symmetric form gives their bits (triangle_split).
 void best_regions(const int (&cap)[kMaxSplit + 1], int64_t tm, int64_t tn, int64_t ktiles, Fp32Split& split) {
-  constexpr double kSecondLaunch = 0.5, kWorth = 0.96;
   double best;
   split = Fp32Split{0, 1, best_split(cap, tm * tn, 0, ktiles, false, &best)};
   if(tm * tn <= 25 || tm * tn > 4 * cap[1]) return;
@@ -616,19 +627,37 @@ void best_regions(const int (&cap)[kMaxSplit + 1], int64_t tm, int64_t tn, int64
   }
 }
 
-// The K split of a symmetric FP32 contraction, which launches the lower
-// triangle of tiles; small ones take the full square's split all the same, so
-// that they give the bits of the same product computed in full (with at most
-// 25 tiles the full square's split is 6 to 8, near the limit of 8 in any case).
-gbpoly_status triangle_split(gbpoly_ctx* ctx, int64_t M, int64_t K, bool dual, int& splits) {
+// The same for a symmetric contraction, which launches the lower triangle of
+// tiles (syr2k: those below the diagonal, then the diagonal ones): `first` CTAs
+// for each of the first `rows` tiles of the walk, `rest` for the others (syrk
+// 2304 x 512 84 -> 68 us, 2304 x 2304 261 -> 228, syr2k 2304 x 512 146 -> 115,
+// correlation 3000 x 2300 342 -> 303; none of 36 shapes slower).  Small ones
+// take one split, the full square's, so that they give the bits of the same
+// product computed in full (with at most 25 tiles the full square's split is 6
+// to 8, near the limit of 8 in any case).
+gbpoly_status triangle_split(gbpoly_ctx* ctx, int64_t M, int64_t K, bool dual, Fp32Split& split) {
   int cap[kMaxSplit + 1] = {};
   gbpoly_status st = cluster_capacity(ctx, cap);
   if(st != GBPOLY_OK) return st;
   const int64_t tm = (M + kBM - 1) / kBM, ktiles = (K + kBK - 1) / kBK;
-  if(dual)
-    splits = best_split(cap, tm * (tm - 1) / 2, tm, ktiles, true);
-  else
-    splits = best_split(cap, tm * tm > 25 ? tm * (tm + 1) / 2 : tm * tm, 0, ktiles, false);
+  if(!dual && tm * tm <= 25) {
+    split = Fp32Split{0, 1, best_split(cap, tm * tm, 0, ktiles, false)};
+    return GBPOLY_OK;
+  }
+  const int64_t whole = dual ? tm * (tm - 1) / 2 : tm * (tm + 1) / 2, diagonal = dual ? tm : 0;
+  double best;
+  split = Fp32Split{0, 1, best_split(cap, whole, diagonal, ktiles, dual, &best)};
+  if(whole > 4 * cap[1]) return GBPOLY_OK;
+  best *= kWorth;
+  for(int s = 1; s <= kMaxSplit; ++s) {
+    if(split_time(cap, 1, 0, ktiles, dual, s) < 0) continue;
+    for(int64_t tiles = cap[s]; tiles < whole; tiles += cap[s]) {
+      double rest;
+      const int r = best_split(cap, whole - tiles, diagonal, ktiles, dual, &rest);
+      const double t = split_time(cap, tiles, 0, ktiles, dual, s) + rest + kSecondLaunch;
+      if(t < best) best = t, split = Fp32Split{tiles, s, r};
+    }
+  }
   return GBPOLY_OK;
 }
 
@@ -640,10 +669,10 @@ gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand&
   gbpoly_status st = Kn::prepare(ctx);
   if(st != GBPOLY_OK) return st;
   const int64_t tm = (a.M + kBM - 1) / kBM, tn = (a.N + kBN - 1) / kBN, ktiles = (a.K + kBK - 1) / kBK;
+  Fp32Split split{0, 1, splits};
+  if(lower && (st = triangle_split(ctx, a.M, a.K, DUAL, split)) != GBPOLY_OK) return st;
   const int64_t tiles = lower ? tm * (tm + 1) / 2 : tm * tn;
   if(tiles >= (1ll << 31)) return fail(GBPOLY_ERR_UNSUPPORTED, "too many output tiles");
-  if(lower && (st = triangle_split(ctx, a.M, a.K, DUAL, splits)) != GBPOLY_OK) return st;
-  const int kt_per_split = int((ktiles + splits - 1) / splits);
   CUtensorMap ta = {}, tb = {};
   auto map = [&](CUtensorMap* t, const Operand& o) {
     return make_tmap_2d(ctx, t, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, o.X, o.R, o.Cn, o.ld, kBK, 128,
@@ -651,10 +680,16 @@ gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand&
   };
   if(FA == Fetch::Tma && (st = map(&ta, oa)) != GBPOLY_OK) return st;
   if(FB == Fetch::Tma && (st = map(&tb, ob)) != GBPOLY_OK) return st;
-  ProfileScope prof(ctx, DUAL ? "sgemm_simt_dual" : "sgemm_simt");
-  typename Kn::Launch l(ctx, unsigned(tiles), unsigned(splits));
-  GBPOLY_CUDA_TRY(cudaLaunchKernelEx(&l.cfg, Kn::fn, ta, tb, oa, ob, int(a.M), int(a.N), int(a.K), a.alpha, a.beta, a.C,
-      a.ldc, lower ? 1 : 0, kt_per_split, ctx->err_dev));
+  for(int64_t t0 = 0; t0 < tiles;) {
+    const bool first = t0 < split.rows;
+    const int64_t t1 = first ? split.rows : tiles;
+    const int s = first ? split.first : split.rest;
+    ProfileScope prof(ctx, DUAL ? "sgemm_simt_dual" : "sgemm_simt");
+    typename Kn::Launch l(ctx, unsigned(t1 - t0), unsigned(s));
+    GBPOLY_CUDA_TRY(cudaLaunchKernelEx(&l.cfg, Kn::fn, ta, tb, oa, ob, int(a.M), int(a.N), int(a.K), a.alpha, a.beta,
+        a.C, a.ldc, lower ? 1 : 0, int(t0), int((ktiles + s - 1) / s), ctx->err_dev));
+    t0 = t1;
+  }
   return GBPOLY_OK;
 }
 
