@@ -328,17 +328,18 @@ __global__ void __launch_bounds__(kThreads, atax_ctas(CHUNKS)) atax_kernel(const
       for(int ch = 0; ch < CHUNKS; ++ch) acc[k] += dot4(a[k][ch], xr[ch]);
     }
     const float rs = reduce_rows<R>(acc, lane);
-    if(lane < R) red[it][warp][lane] = rs;
+    // (zero beyond nr, where a zero row times an infinite x is NaN)
+    if(lane < R) red[it][warp][lane] = lane < nr ? rs : 0.f;
     __syncthreads();  // (a set is rewritten two groups later, after the next group's barrier)
 #pragma unroll
     for(int k = 0; k < R; ++k) {
       float sum = 0.f;
 #pragma unroll
       for(int w = 0; w < kThreads / 32; ++w) sum += red[it][w][k];
-      const float t = red[it][kThreads / 32][k] + sum;  // tmp += A x (atax.cpp:78-83)
+      const float t = red[it][kThreads / 32][k] + sum;  // tmp += A x (atax.cpp:78-83); zero beyond nr
       if(tid == 0 && k < nr) tmp[r0 + k] = t;
 #pragma unroll
-      for(int ch = 0; ch < CHUNKS; ++ch) {  // y += A^T tmp (atax.cpp:91-96); a is zero beyond nr
+      for(int ch = 0; ch < CHUNKS; ++ch) {  // y += A^T tmp (atax.cpp:91-96)
         colacc[ch].x = fmaf(a[k][ch].x, t, colacc[ch].x);
         colacc[ch].y = fmaf(a[k][ch].y, t, colacc[ch].y);
         colacc[ch].z = fmaf(a[k][ch].z, t, colacc[ch].z);
