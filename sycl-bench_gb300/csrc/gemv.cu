@@ -304,15 +304,16 @@ __global__ void __launch_bounds__(kThreads, atax_ctas(CHUNKS)) atax_kernel(const
   __shared__ float red[2][kThreads / 32 + 1][R];  // warp sums and the old tmp, alternating sets
   pdl_enter();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int begin = int(int64_t(rows) * blockIdx.x / gridDim.x), end = int(int64_t(rows) * (blockIdx.x + 1) / gridDim.x);
+  const int begin = int(int64_t(rows) * blockIdx.x / gridDim.x);
+  const int count = int(int64_t(rows) * (blockIdx.x + 1) / gridDim.x) - begin;
   float4 xr[CHUNKS], colacc[CHUNKS];
 #pragma unroll
   for(int ch = 0; ch < CHUNKS; ++ch) {
     xr[ch] = load4<VEC>(x, ch * kTileCols, cols);
     colacc[ch] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  for(int r0 = begin, it = 0; r0 < end; r0 += R, it ^= 1) {
-    const int nr = min(R, end - r0);
+  for(int i = 0, it = 0; i < count; i += R, it ^= 1) {  // (begin + i, stepped, could pass the largest row count)
+    const int r0 = begin + i, nr = min(R, count - i);
     float4 a[R][CHUNKS];
 #pragma unroll
     for(int k = 0; k < R; ++k)
@@ -356,7 +357,7 @@ template <int CHUNKS>
 gbpoly_status launch_atax(gbpoly_ctx* ctx, const float* A, int64_t lda, int rows, int cols, const float* x, float* tmp,
     float* y, bool vec) {
   const int ctas = atax_ctas(CHUNKS) * std::max(ctx->sm_count, 1);
-  const int grid = std::max(1, std::min((rows + atax_rows(CHUNKS) - 1) / atax_rows(CHUNKS), ctas));
+  const int grid = std::max(1, std::min((rows - 1) / atax_rows(CHUNKS) + 1, ctas));
   gbpoly_status st = ensure_scratch(ctx, ctx->stats, size_t(grid) * size_t(cols) * 4 + 256, "matrix-vector scratch");
   if(st != GBPOLY_OK) return st;
   float* col_part = static_cast<float*>(ctx->stats.ptr);

@@ -30,3 +30,25 @@ def test_atax_keeps_infinities(ctx, rows, cols, pad):
         ctx.free(b)
     np.testing.assert_array_equal(tmp, np.full(rows, INF))
     np.testing.assert_array_equal(y, np.full(cols, INF))
+
+
+def test_atax_at_the_largest_row_count(ctx):
+    """2^31 - 1 rows, the most a call takes: the row counter of the last group
+    stays inside the matrix (one column, so that A and tmp are 8.6 GB each)."""
+    rows = 2 ** 31 - 1
+    dA, dt = ctx.alloc(rows * 4), ctx.alloc(rows * 4)
+    one = np.ones(1, np.float32)
+    dx, dy = ctx.upload(one), ctx.upload(np.zeros(1, np.float32))
+    ctx.memset(dA, 0, rows * 4)
+    ctx.memset(dt, 0, rows * 4)
+    set_rows = [0, 12345, rows - 17, rows - 16, rows - 2, rows - 1]
+    for r in set_rows:
+        ctx.h2d(dA.ptr + 4 * r, one)
+    ctx.synchronize()
+    ctx.atax(rows, 1, dA, 1, dx, dt, dy)
+    ctx.synchronize()
+    assert ctx.download(dy, (1,))[0] == len(set_rows)
+    for r in set_rows:
+        assert ctx.download(dt.ptr + 4 * r, (1,))[0] == 1
+    for b in (dA, dt, dx, dy):
+        ctx.free(b)
