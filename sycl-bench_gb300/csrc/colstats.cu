@@ -48,12 +48,13 @@ __device__ __forceinline__ float column_chunk_sum(const float* __restrict__ col,
 #pragma unroll
     for(int k = 0; k < kLoads; ++k) {
       const int rk = r + k * kWarps;
-      v[k] = rk < r1 ? col[int64_t(rk) * ldx] : (CENTERED ? m : 0.f);  // beyond the chunk: adds zero
+      v[k] = rk < r1 ? col[int64_t(rk) * ldx] : 0.f;
     }
 #pragma unroll
     for(int k = 0; k < kLoads; ++k) {
       if constexpr(CENTERED) {
-        const float c = v[k] - m;
+        // beyond the chunk nothing is added (m - m would be NaN for an infinite mean)
+        const float c = r + k * kWarps < r1 ? v[k] - m : 0.f;
         a[k % kSums] = fmaf(c, c, a[k % kSums]);
       } else {
         a[k % kSums] += v[k];
