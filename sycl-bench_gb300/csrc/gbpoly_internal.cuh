@@ -341,6 +341,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   return mbar_wait_for(bar, parity, err, code, kWaitTimeoutNs);
 }
 
+// Wait for phase `parity` of `bar` whatever error has been recorded: a CTA may
+// not leave while copies into its shared memory are in flight, and the waits
+// above give up at another thread's error, long before a copy has landed.
+// Bounded as they are (a phase nobody completes).
+__device__ __forceinline__ bool mbar_drain(uint64_t* bar, uint32_t parity, int* err) {
+  if(mbar_try_wait(bar, parity)) return true;
+  const uint64_t t0 = global_timer_ns();
+  while(!mbar_try_wait(bar, parity)) {
+    if(global_timer_ns() - t0 > kWaitTimeoutNs) {
+      atomicCAS(err, 0, kDevErrDrainWait);
+      return false;
+    }
+  }
+  return true;
+}
+
 // Wait until the global counter reaches `target` (other CTAs of the same
 // launch add to it).  Bounded like mbar_wait; ordered before the caller's
 // later loads on success.

@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
       if constexpr(kWords) asm volatile("cp.async.wait_all;" ::: "memory");
       if(kTmaTiles > 0 && tid == 0)
         for(int kt = max(0, issued - STAGES); kt < issued; ++kt)
-          if(!mbar_wait(&full[kt % STAGES], (kt / STAGES) & 1, err, kDevErrDrainWait)) break;
+          if(!mbar_drain(&full[kt % STAGES], (kt / STAGES) & 1, err)) break;
     }
     __syncwarp();
     if(splits > 1) {

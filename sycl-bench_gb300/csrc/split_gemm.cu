@@ -959,7 +959,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
       // second CTA leaves only after the pair's final cluster barrier
       if(rank == 0)
         for(int h = max(0, g - F::STAGES); h < g; ++h)
-          if(!mbar_wait(&full[h % F::STAGES], (h / F::STAGES) & 1, err, kDevErrDrainWait)) break;
+          if(!mbar_drain(&full[h % F::STAGES], (h / F::STAGES) & 1, err)) break;
     } else if(warp == 1 && lane == 0 && rank == 0) {
       // ------------------------------------------------------- MMA issue
       int g = 0, chunk = 0;
@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         umma::commit_pair(drain, 0x1);
       else
         umma::commit(drain);
-      mbar_wait(drain, 0, err, kDevErrDrainWait);
+      mbar_drain(drain, 0, err);
     }
   } else {
     // ------------------------------------------------------------- epilogue
@@ -1091,6 +1091,8 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         }
       };
       if(BOXES && writes && beta != 0.f) load_box(nbase, crow);
+      // the warp's last load of C, the same answer in all lanes (the boxes are written and stored in step)
+      auto c_landed = [&] { return __all_sync(0xffffffffu, mbar_wait(&cbar[warp - 4], (c_loads - 1) & 1, err, kDevErrMmaWait)); };
       // RING: the CTA's only unit.  This warp's HALF / 32 boxes of C live in the
       // pipeline's stages, which no later tile fills.  The loads start while
       // the last chunk's MMAs run: every stage but that chunk's has been read
@@ -1102,12 +1104,14 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         const int at = F::RING_C_EARLY ? (last_chunk + 1) % F::STAGES * F::STAGE : 0;
         ring_box = smem + (at + (warp - 4) * kBoxes * F::C_BOX) % (F::STAGES * F::STAGE);
         if constexpr(RING) {
-          if(beta != 0.f && lane == 0) {
+          if(beta == 0.f) return;
+          if(lane == 0) {
             mbar_arrive_expect_tx(&cbar[warp - 4], kBoxes * F::C_BOX);
 #pragma unroll
             for(int j = 0; j < kBoxes; ++j)
               tma_load_2d(ring_box + j * F::C_BOX, &sched.cmap, &cbar[warp - 4], nbase + 32 * j, crow);
           }
+          ++c_loads;
         }
       };
       // Scaled forms (E4M3, F16): chunk c (stage iteration it0 + c, CH = 1)
@@ -1257,12 +1261,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
           release(b);
         }
       }
-      if(!ok) {
-        // do not leave while C's copies into the stages are in flight
-        if(RING && ring_box != nullptr && beta != 0.f) mbar_wait(&cbar[warp - 4], 0, err, kDevErrDrainWait);
-        if(BOXES && writes && beta != 0.f) mbar_wait(&cbar[warp - 4], (c_loads - 1) & 1, err, kDevErrDrainWait);
-        continue;
-      }
+      if(!ok) continue;
       if constexpr(F::CEPI) {
         // C = alpha acc + beta C in the boxes (lane = row: eight 16-byte
         // chunks, swizzled by row, so each quarter warp covers all banks),
@@ -1319,7 +1318,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
             if(lane == 0) atomicAdd(&sched.flags[slot], 1);  // sums stored: count this warp
             continue;
           }
-          if(!wait_count(&sched.flags[slot], 8 * F::CG, err, kDevErrSplitWait)) {
+          if(!__all_sync(0xffffffffu, wait_count(&sched.flags[slot], 8 * F::CG, err, kDevErrSplitWait))) {
             ok = false;
             continue;
           }
@@ -1339,7 +1338,7 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         // chunks, swizzled by row), each stored by TMA when done (clipped at
         // the matrix edges)
         if(!F::RING_C_EARLY) load_ring(0);
-        if(beta != 0.f && !mbar_wait(&cbar[warp - 4], 0, err, kDevErrMmaWait)) {
+        if(beta != 0.f && !c_landed()) {
           ok = false;
           continue;
         }
@@ -1375,8 +1374,9 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
                 tma_load_2d(ring_box + j * F::C_BOX, &sched.cmap, &cbar[warp - 4], crow, nbase + 32 * j);
             }
           }
+          if(beta != 0.f) ++c_loads;
           __syncwarp();
-          if(beta != 0.f && !mbar_wait(&cbar[warp - 4], 1, err, kDevErrMmaWait)) {
+          if(beta != 0.f && !c_landed()) {
             ok = false;
             continue;
           }
@@ -1403,11 +1403,14 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
         const int boxes = below > 0 ? 2 * kBoxes : kBoxes;
 #pragma unroll
         for(int t = 0; t < (F::MIRROR ? 2 : 1); ++t) {
-          if(t == 1 && below <= 0) break;
+          if(t == 1 && (below <= 0 || !ok)) break;
 #pragma unroll
           for(int j = 0; j < kBoxes; ++j) {
             if(beta != 0.f) {
-              if(!mbar_wait(&cbar[warp - 4], (c_loads - 1) & 1, err, kDevErrMmaWait)) ok = false;
+              if(!c_landed()) {
+                ok = false;
+                break;
+              }
             } else {
               if(lane == 0 && c_stores > 0) bulk_wait_read_all();
               __syncwarp();
@@ -1525,8 +1528,12 @@ __global__ void __launch_bounds__(F::THREADS, 1) split_gemm_kernel(const __grid_
       }
       }  // staged epilogue
     }
-    if constexpr(F::CEPI || EPI != Epi::Staged)
+    if constexpr(F::CEPI || EPI != Epi::Staged) {
+      // whichever wait gave up, C's last load has landed before the CTA leaves
+      // (one is in flight at a time; a load that was waited for is complete)
+      if(!ok && c_loads > 0) mbar_drain(&cbar[warp - 4], (c_loads - 1) & 1, err);
       if(lane == 0 && c_stores > 0) bulk_wait_all();  // C written before the CTA leaves
+    }
   }
 
   umma::fence_before_sync();
