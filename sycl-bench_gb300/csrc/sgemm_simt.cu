@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
-  const int tiles_m = (M + kBM - 1) / kBM, tiles_n = (N + kBN - 1) / kBN;
+  const int tiles_m = (M - 1) / kBM + 1, tiles_n = (N - 1) / kBN + 1;  // (M + kBM could pass 2^31)
   int tile_m, tile_n;
   if constexpr(DUAL)
     dual_coords(first_tile + blockIdx.x, tiles_m, tile_m, tile_n);
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
   const int m0 = tile_m * kBM, n0 = tile_n * kBN;
   const bool mirror = lower && tile_m != tile_n;
   const int splits = int(gridDim.y), split = int(blockIdx.y);  // the cluster is 1 x splits: split == rank
-  const int ktiles = (K + kBK - 1) / kBK;
+  const int ktiles = K / kBK + (K % kBK != 0);
   const int kt0 = split * kt_per_split;
   const int nkt = max(0, min(ktiles, kt0 + kt_per_split) - kt0);
 
@@ -731,7 +731,7 @@ gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a) {
   if(a.M == 0 || a.N == 0) return GBPOLY_OK;
   const bool a_kmaj = a.op_a == GBPOLY_OP_N;
   const bool b_kmaj = a.op_b == GBPOLY_OP_T;
-  if(a.M >= (1ll << 31) - kBM || a.N >= (1ll << 31) - kBN || a.K >= (1ll << 31) - kBK) {
+  if(a.M >= (1ll << 31) || a.N >= (1ll << 31) || a.K >= (1ll << 31)) {
     // beyond the kernel's 32-bit tile coordinates
     TiledOperand<float> oa = a_kmaj ? TiledOperand<float>{a.A, a.lda, 1} : TiledOperand<float>{a.A, 1, a.lda};
     TiledOperand<float> ob = b_kmaj ? TiledOperand<float>{a.B, a.ldb, 1} : TiledOperand<float>{a.B, 1, a.ldb};
