@@ -1805,7 +1805,8 @@ bool same_operand(const GemmF32Args& a) { return symmetric_operand(a); }
 // rows ending on a 16-byte boundary (TMA stores clip the row end at 16-byte
 // granularity: a ragged N would write into the padding of ldc).
 bool c_tile_ok(const GemmF32Args& a) {
-  return (reinterpret_cast<uintptr_t>(a.C) & 15) == 0 && (a.ldc & 3) == 0 && (a.N & 3) == 0;
+  // (a tensor map's row stride ends below 2^40 bytes; one row of C may have any)
+  return (reinterpret_cast<uintptr_t>(a.C) & 15) == 0 && (a.ldc & 3) == 0 && (a.N & 3) == 0 && a.ldc < (1ll << 38);
 }
 
 // C's tensor map for the configurations that move C through TMA.
