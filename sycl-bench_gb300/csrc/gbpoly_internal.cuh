@@ -202,8 +202,8 @@ gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a);
 // shared memory of its clusters and needs none of it; the figure stays for
 // callers that reserve by it.
 size_t fp32_split_k_bytes(int sm_count, int64_t M, int64_t N, int64_t K);
-// The K split gbpoly_gemm_f32 uses for a non-symmetric FP32 contraction of this shape.
-gbpoly_status fp32_split(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, Fp32Split& split);
+// The K split gbpoly_gemm_f32 uses for this FP32 contraction (a's shape and operand layouts).
+gbpoly_status fp32_split(gbpoly_ctx* ctx, const GemmF32Args& a, Fp32Split& split);
 // Tensor-core forms (split_gemm.cu): tf32, bf16x3, tf32x3, bf16x6, fp16x3,
 // fp8.  The split term panels live in the context workspace.
 gbpoly_status launch_gemm_tensor(gbpoly_ctx* ctx, gbpoly_precision prec, const GemmF32Args& a);

@@ -125,7 +125,9 @@ extern "C" gbpoly_status gbpoly_gemm_f32_host(gbpoly_ctx* ctx, gbpoly_precision 
     a.A = pipelined ? dA + r0 * K : dA, a.lda = ac, a.B = dB, a.ldb = bc, a.C = dC + r0 * N, a.ldc = N;
     if(prec == GBPOLY_PREC_FP32) {
       // the K split of the whole call, so the panels give the device-buffer call's bits
-      if((st = fp32_split(ctx, M, N, K, a.split)) != GBPOLY_OK) return st;
+      GemmF32Args whole = a;
+      whole.M = M;
+      if((st = fp32_split(ctx, whole, a.split)) != GBPOLY_OK) return st;
       a.split_row = r0;
       st = launch_gemm_f32_simt(ctx, a);
     }

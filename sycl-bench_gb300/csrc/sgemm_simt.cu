@@ -608,8 +608,8 @@ constexpr double kSecondLaunch = 0.5, kWorth = 0.96;
 // pairs, 24 as clusters of five) 142 -> 130, 2048 cubed 320 -> 295; of 35
 // shapes of 200 to 4000 twelve took two launches, ten of them 1.5 to 31 %
 // faster, two 2 % slower.  Not beyond four rounds of CTAs, where the last one
-// matters less and the search takes longer.  Products of at most 25 tiles stay
-// one launch: their symmetric form gives their bits (triangle_split).
+// matters less and the search takes longer; nor up to 25 tiles, which one round
+// of clusters of five or more holds.
 void best_regions(const int (&cap)[kMaxSplit + 1], int64_t tm, int64_t tn, int64_t ktiles, Fp32Split& split) {
   double best;
   split = Fp32Split{0, 1, best_split(cap, tm * tn, 0, ktiles, false, &best)};
@@ -627,50 +627,67 @@ void best_regions(const int (&cap)[kMaxSplit + 1], int64_t tm, int64_t tn, int64
   }
 }
 
-// The same for a symmetric contraction, which launches the lower triangle of
-// tiles (syr2k: those below the diagonal, then the diagonal ones): `first` CTAs
-// for each of the first `rows` tiles of the walk, `rest` for the others (syrk
-// 2304 x 512 84 -> 68 us, 2304 x 2304 261 -> 228, syr2k 2304 x 512 146 -> 115,
-// correlation 3000 x 2300 342 -> 303; none of 36 shapes slower).  Small ones
-// take one split, the full square's, so that they give the bits of the same
-// product computed in full (with at most 25 tiles the full square's split is 6
-// to 8, near the limit of 8 in any case).
-gbpoly_status triangle_split(gbpoly_ctx* ctx, int64_t M, int64_t K, bool dual, Fp32Split& split) {
-  int cap[kMaxSplit + 1] = {};
-  gbpoly_status st = cluster_capacity(ctx, cap);
-  if(st != GBPOLY_OK) return st;
-  const int64_t tm = (M + kBM - 1) / kBM, ktiles = (K + kBK - 1) / kBK;
-  if(!dual && tm * tm <= 25) {
-    split = Fp32Split{0, 1, best_split(cap, tm * tm, 0, ktiles, false)};
-    return GBPOLY_OK;
-  }
-  const int64_t whole = dual ? tm * (tm - 1) / 2 : tm * (tm + 1) / 2, diagonal = dual ? tm : 0;
+// The same for syr2k, which launches the tiles below the diagonal and then the
+// diagonal ones: `first` CTAs for each of the first `rows` tiles of that walk,
+// `rest` for the others (2304 x 512 146 -> 115 us).
+void dual_regions(const int (&cap)[kMaxSplit + 1], int64_t tm, int64_t ktiles, Fp32Split& split) {
+  const int64_t below = tm * (tm - 1) / 2;
   double best;
-  split = Fp32Split{0, 1, best_split(cap, whole, diagonal, ktiles, dual, &best)};
-  if(whole > 4 * cap[1]) return GBPOLY_OK;
+  split = Fp32Split{0, 1, best_split(cap, below, tm, ktiles, true, &best)};
+  if(below > 4 * cap[1]) return;
   best *= kWorth;
   for(int s = 1; s <= kMaxSplit; ++s) {
-    if(split_time(cap, 1, 0, ktiles, dual, s) < 0) continue;
-    for(int64_t tiles = cap[s]; tiles < whole; tiles += cap[s]) {
+    if(split_time(cap, 1, 0, ktiles, true, s) < 0) continue;
+    for(int64_t tiles = cap[s]; tiles < below; tiles += cap[s]) {
       double rest;
-      const int r = best_split(cap, whole - tiles, diagonal, ktiles, dual, &rest);
-      const double t = split_time(cap, tiles, 0, ktiles, dual, s) + rest + kSecondLaunch;
+      const int r = best_split(cap, below - tiles, tm, ktiles, true, &rest);
+      const double t = split_time(cap, tiles, 0, ktiles, true, s) + rest + kSecondLaunch;
       if(t < best) best = t, split = Fp32Split{tiles, s, r};
     }
   }
-  return GBPOLY_OK;
 }
 
-// splits 0: symmetric product (op(A) == op(B)^T as stored, or syr2k), the lower triangle of tiles only.
+// One split for X X^T and for a product of the same shape and operand layout
+// with another right operand, so that the triangle of tiles of the one gives
+// the bits of the full square of the other (the result does not depend on
+// whether the library sees that the operands are the same, and a host-buffer
+// call, which has two copies, gives the device call's bits).  The two have
+// different best splits, the triangle about half the tiles: the triangle's
+// best one among those that cost the square at most 15 % (us with this rule /
+// each on its own best plan, two launches among them: 1024 cubed N/T 52 / 45,
+// its triangle 28.5 / 28.5; 1536 121 / 121, 125 / 87; 2304 446 / 407, 257 / 225;
+// 3000 x 1000, triangle 182 / 182).
+constexpr double kSquareMost = 1.15;
+
+int square_split(const int (&cap)[kMaxSplit + 1], int64_t tm, int64_t ktiles) {
+  const int64_t square = tm * tm, triangle = tm * (tm + 1) / 2;
+  double most = split_time(cap, square, 0, ktiles, false, 1);
+  for(int s = 2; s <= kMaxSplit; ++s) {
+    const double t = split_time(cap, square, 0, ktiles, false, s);
+    if(t >= 0) most = std::min(most, t);
+  }
+  most *= kSquareMost;
+  int best = 0;
+  double best_t = 0;
+  for(int s = 1; s <= kMaxSplit; ++s) {
+    const double full = split_time(cap, square, 0, ktiles, false, s);
+    if(full < 0 || full > most) continue;
+    const double t = split_time(cap, triangle, 0, ktiles, false, s);
+    if(best == 0 || t < 0.97 * best_t) best = s, best_t = t;
+  }
+  return best;
+}
+
+// lower: symmetric product (op(A) == op(B)^T as stored, or syr2k), the lower
+// triangle of tiles only; split.rows counts tiles of its walk then.  Others
+// are one region: split.rest.
 template <Fetch FA, Fetch FB, bool DUAL>
-gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob, int splits) {
+gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob, bool lower,
+    const Fp32Split& split) {
   using Kn = Kernel<FA, FB, DUAL>;
-  const bool lower = splits == 0;
   gbpoly_status st = Kn::prepare(ctx);
   if(st != GBPOLY_OK) return st;
   const int64_t tm = (a.M + kBM - 1) / kBM, tn = (a.N + kBN - 1) / kBN, ktiles = (a.K + kBK - 1) / kBK;
-  Fp32Split split{0, 1, splits};
-  if(lower && (st = triangle_split(ctx, a.M, a.K, DUAL, split)) != GBPOLY_OK) return st;
   const int64_t tiles = lower ? tm * (tm + 1) / 2 : tm * tn;
   if(tiles >= (1ll << 31)) return fail(GBPOLY_ERR_UNSUPPORTED, "too many output tiles");
   CUtensorMap ta = {}, tb = {};
@@ -694,11 +711,13 @@ gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand&
 }
 
 template <Fetch FA>
-gbpoly_status launch_left(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob, Fetch fb, int splits) {
+gbpoly_status launch_left(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob, Fetch fb,
+    bool lower, int splits) {
+  const Fp32Split split{0, 1, splits};
   switch(fb) {
-  case Fetch::Tma: return launch_sgemm<FA, Fetch::Tma, false>(ctx, a, oa, ob, splits);
-  case Fetch::Rows: return launch_sgemm<FA, Fetch::Rows, false>(ctx, a, oa, ob, splits);
-  default: return launch_sgemm<FA, Fetch::Turn, false>(ctx, a, oa, ob, splits);
+  case Fetch::Tma: return launch_sgemm<FA, Fetch::Tma, false>(ctx, a, oa, ob, lower, split);
+  case Fetch::Rows: return launch_sgemm<FA, Fetch::Rows, false>(ctx, a, oa, ob, lower, split);
+  default: return launch_sgemm<FA, Fetch::Turn, false>(ctx, a, oa, ob, lower, split);
   }
 }
 
@@ -711,11 +730,19 @@ Fetch fetch_of(const Operand& o, bool k_major) {
 
 }  // namespace
 
-gbpoly_status fp32_split(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K, Fp32Split& split) {
+gbpoly_status fp32_split(gbpoly_ctx* ctx, const GemmF32Args& a, Fp32Split& split) {
+  split = Fp32Split{0, 1, 1};
   int cap[kMaxSplit + 1] = {};
   gbpoly_status st = cluster_capacity(ctx, cap);
-  if(st == GBPOLY_OK) best_regions(cap, (M + kBM - 1) / kBM, (N + kBN - 1) / kBN, (K + kBK - 1) / kBK, split);
-  return st;
+  if(st != GBPOLY_OK) return st;
+  const int64_t tm = (a.M + kBM - 1) / kBM, tn = (a.N + kBN - 1) / kBN, ktiles = (a.K + kBK - 1) / kBK;
+  if(a.dual)
+    dual_regions(cap, tm, ktiles, split);
+  else if(a.M == a.N && a.op_a != a.op_b)
+    split.rest = square_split(cap, tm, ktiles);
+  else
+    best_regions(cap, tm, tn, ktiles, split);
+  return GBPOLY_OK;
 }
 
 size_t fp32_split_k_bytes(int sm_count, int64_t M, int64_t N, int64_t K) {
@@ -749,19 +776,19 @@ gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a) {
                        ((a.lda | a.ldb) & 3) == 0 && K > 0;
   if(!aligned && (a.M + 63) / 64 > 65535)  // the limit of these calls, unchanged
     return fail(GBPOLY_ERR_UNSUPPORTED, "matrix too tall for operands off 16-byte boundaries");
-  if(a.dual) return launch_sgemm<Fetch::Turn, Fetch::Turn, true>(ctx, a, oa, ob, 0);
+  const bool symmetric = symmetric_operand(a);
+  Fp32Split split = a.split;
+  gbpoly_status st = GBPOLY_OK;
+  if(split.rest == 0 && (st = fp32_split(ctx, a, split)) != GBPOLY_OK) return st;
+  if(a.dual) return launch_sgemm<Fetch::Turn, Fetch::Turn, true>(ctx, a, oa, ob, true, split);
   const Fetch fb = fetch_of(ob, b_kmaj);
   auto launch = [&](const GemmF32Args& part, const Operand& left, int splits) {
     switch(fetch_of(left, a_kmaj)) {
-    case Fetch::Tma: return launch_left<Fetch::Tma>(ctx, part, left, ob, fb, splits);
-    case Fetch::Rows: return launch_left<Fetch::Rows>(ctx, part, left, ob, fb, splits);
-    default: return launch_left<Fetch::Turn>(ctx, part, left, ob, fb, splits);
+    case Fetch::Tma: return launch_left<Fetch::Tma>(ctx, part, left, ob, fb, symmetric, splits);
+    case Fetch::Rows: return launch_left<Fetch::Rows>(ctx, part, left, ob, fb, symmetric, splits);
+    default: return launch_left<Fetch::Turn>(ctx, part, left, ob, fb, symmetric, splits);
     }
   };
-  if(symmetric_operand(a)) return launch(a, oa, 0);
-  Fp32Split split = a.split;
-  gbpoly_status st = GBPOLY_OK;
-  if(split.rest == 0 && (st = fp32_split(ctx, a.M, a.N, a.K, split)) != GBPOLY_OK) return st;
   const int m1 = int(std::clamp<int64_t>(split.rows - a.split_row, 0, a.M));  // rows of the first region
   if(m1 == M) return launch(a, oa, split.first);
   if(m1 == 0) return launch(a, oa, split.rest);
