@@ -158,12 +158,14 @@ struct RowXform {
   float div = 1.f;
 };
 
-// K split of an FP32 contraction, in CTAs per output tile: `first` in the rows
-// of C before row `rows`, `rest` (1 or more, 0: chosen from the shape) in the
-// others.
+// How an FP32 contraction runs.  Its K split, in CTAs per output tile: `first`
+// in the rows of C before row `rows`, `rest` (1 or more, 0: not chosen yet) in
+// the others; or, tile64, the kernel for short K and any strides, which does
+// not split.
 struct Fp32Split {
   int64_t rows = 0;
   int first = 1, rest = 0;
+  bool tile64 = false;
 };
 
 struct GemmF32Args {
@@ -202,7 +204,7 @@ gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a);
 // shared memory of its clusters and needs none of it; the figure stays for
 // callers that reserve by it.
 size_t fp32_split_k_bytes(int sm_count, int64_t M, int64_t N, int64_t K);
-// The K split gbpoly_gemm_f32 uses for this FP32 contraction (a's shape and operand layouts).
+// How gbpoly_gemm_f32 runs this FP32 contraction (a's shape, operand layouts and alignment).
 gbpoly_status fp32_split(gbpoly_ctx* ctx, const GemmF32Args& a, Fp32Split& split);
 // Tensor-core forms (split_gemm.cu): tf32, bf16x3, tf32x3, bf16x6, fp16x3,
 // fp8.  The split term panels live in the context workspace.

@@ -124,9 +124,9 @@ extern "C" gbpoly_status gbpoly_gemm_f32_host(gbpoly_ctx* ctx, gbpoly_precision 
     a.M = pipelined ? rows : M, a.N = N, a.K = K, a.alpha = alpha, a.beta = beta, a.op_a = op_a, a.op_b = op_b;
     a.A = pipelined ? dA + r0 * K : dA, a.lda = ac, a.B = dB, a.ldb = bc, a.C = dC + r0 * N, a.ldc = N;
     if(prec == GBPOLY_PREC_FP32) {
-      // the K split of the whole call, so the panels give the device-buffer call's bits
+      // the K split of the whole call, so the panels give the bits of a device-buffer call on equally aligned operands
       GemmF32Args whole = a;
-      whole.M = M;
+      whole.M = M, whole.A = A, whole.lda = lda, whole.B = B, whole.ldb = ldb;
       if((st = fp32_split(ctx, whole, a.split)) != GBPOLY_OK) return st;
       a.split_row = r0;
       st = launch_gemm_f32_simt(ctx, a);

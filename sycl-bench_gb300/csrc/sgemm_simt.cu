@@ -11,6 +11,8 @@
 //   * eight consumer warps (256 threads) each keep an 8x8 block of C in
 //     registers and run packed FFMA over 128-bit shared-memory loads;
 //   * the epilogue applies C = alpha*acc + beta*C with bounds checks.
+// Short K on operands off 16-byte boundaries runs on 64x64 tiles instead
+// (use_tile64, below).
 // Grids that would not fill the device split K over the CTAs of a cluster.
 // syr2k's two products (A_i.B_j + B_i.A_j) stream four tiles per stage into
 // the same accumulator.  Symmetric updates (syrk, syr2k, X^T.X) compute only
@@ -29,7 +31,6 @@
 #include <algorithm>
 
 #include "gbpoly_internal.cuh"
-#include "tiled_gemm.cuh"
 #include "umma.cuh"
 
 namespace gbpoly {
@@ -203,6 +204,46 @@ __device__ __forceinline__ void dual_coords(int t, int tiles, int& tile_m, int& 
   }
 }
 
+// C = alpha t + beta C for a warp's 32 x 64 block at (m, n), which lies in shared
+// memory as t[row][column], and for its mirror: rows of C off 16-byte boundaries.
+// The quads' single words would be scattered over a warp's addresses; here a
+// lane is a column (of the mirror: a row) and a warp's access a row segment
+// (us, quads by words / turned: 8192 x 8192 x 32 262 / 210, 3000 x 3000 x 128 65 /
+// 57, syr2k 2000 x 300 67 / 60).  Not inlined: its addresses would cost the
+// kernel's other paths registers.
+constexpr int kTurnPitch = 65;
+__device__ __noinline__ void write_turned(const float* t, int m0, int n0, int M, int N, float alpha, float beta,
+    float* __restrict__ C, int64_t ldc, bool mirror) {
+  const int lane = threadIdx.x & 31;
+  const bool read_c = beta != 0.f;
+#pragma unroll 1
+  for(int r = 0; r < 32; r += 8) {
+    float old[16];
+#pragma unroll
+    for(int e = 0; e < 16; ++e) {
+      const int m = m0 + r + (e >> 1), n = n0 + lane + 32 * (e & 1);
+      old[e] = read_c && m < M && n < N ? C[int64_t(m) * ldc + n] : 0.f;
+    }
+#pragma unroll
+    for(int e = 0; e < 16; ++e) {
+      const int m = m0 + r + (e >> 1), n = n0 + lane + 32 * (e & 1);
+      const float s = t[(r + (e >> 1)) * kTurnPitch + lane + 32 * (e & 1)];
+      if(m < M && n < N) C[int64_t(m) * ldc + n] = fmaf(beta, old[e], alpha * s);
+    }
+  }
+  if(!mirror) return;
+  const int m = m0 + lane;
+#pragma unroll 1
+  for(int c = 0; c < 64; c += 16) {
+    float old[16];
+#pragma unroll
+    for(int e = 0; e < 16; ++e) old[e] = read_c && m < M && n0 + c + e < N ? C[int64_t(n0 + c + e) * ldc + m] : 0.f;
+#pragma unroll
+    for(int e = 0; e < 16; ++e)
+      if(m < M && n0 + c + e < N) C[int64_t(n0 + c + e) * ldc + m] = fmaf(beta, old[e], alpha * t[lane * kTurnPitch + c + e]);
+  }
+}
+
 // FA, FB: how op(A)'s and op(B)'s tiles are fetched.  DUAL: syr2k (both
 // operands K-major), tiles A_i, B_j, B_i, A_j.  On the diagonal the second
 // product is the first one's transpose, S + S^T: half the copies and half the
@@ -221,7 +262,11 @@ __device__ __forceinline__ void dual_coords(int t, int tiles, int& tile_m, int& 
 // (every run gives the same bits), and writes them.  No global scratch, no
 // second launch: a launch stays independent of every other one, on any
 // stream or in any graph.
-template <Fetch FA, Fetch FB, bool DUAL, int STAGES>
+//
+// TURN: unsplit launches on a C whose rows are off 16-byte boundaries, written
+// by write_turned.  An instance of its own: beside the quads' path it cost
+// syr2k's clusters 1 to 2 us (1000 x 100 15.9 -> 17.7).
+template <Fetch FA, Fetch FB, bool DUAL, bool TURN, int STAGES>
 __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constant__ CUtensorMap tmA,
     const __grid_constant__ CUtensorMap tmB, const Operand oa, const Operand ob, int M, int N, int K,
     float alpha, float beta, float* __restrict__ C, int64_t ldc, int lower, int first_tile, int kt_per_split, int* err) {
@@ -231,7 +276,7 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
   constexpr bool kWords = kTmaTiles < 2;
   static_assert(!DUAL || (FA == Fetch::Turn && FB == Fetch::Turn), "syr2k: K-major operands");
   extern __shared__ __align__(1024) char smem_raw[];
-  // 1024-byte aligned (128-byte swizzle atoms); offset arithmetic keeps the pointer in the shared window
+  // 1024-byte aligned; offset arithmetic keeps the pointer in the shared window
   char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * kStageBytes);
   uint64_t* empty = full + STAGES;
@@ -305,7 +350,7 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
           if(!mbar_drain(&full[kt % STAGES], (kt / STAGES) & 1, err)) break;
     }
     __syncwarp();
-    if(splits > 1) {
+    if(!TURN && splits > 1) {
       cluster_sync();  // the cluster's sums are written
       cluster_arrive();
       cluster_wait();  // and read
@@ -421,7 +466,7 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
       acc[f].x += q[0], acc[f].y += q[kPitch], acc[f].z += q[2 * kPitch], acc[f].w += q[3 * kPitch];
     }
   }
-  if(splits > 1) {
+  if(!TURN && splits > 1) {
     // every consumer warp has read its last stage, every copy has landed (each was waited for)
     asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");
     float4* mine = reinterpret_cast<float4*>(smem) + ctid;
@@ -461,6 +506,18 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
     cluster_wait();  // no CTA leaves (or is left) while its sums are being read
     return;
   }
+  if constexpr(TURN) {
+    asm volatile("bar.sync 1, %0;" ::"n"(kConsumers) : "memory");  // the ring is drained, as before the exchange
+    float* t = reinterpret_cast<float*>(smem) + cwarp * 32 * kTurnPitch;
+#pragma unroll
+    for(int f = 0; f < 16; ++f) {
+      float* q = t + owned_row(li, f >> 1) * kTurnPitch + owned_col(lj, 4 * (f & 1));
+      q[0] = acc[f].x, q[1] = acc[f].y, q[2] = acc[f].z, q[3] = acc[f].w;
+    }
+    __syncwarp();
+    if(ok) write_turned(t, m0 + wr, n0 + wc, M, N, alpha, beta, C, ldc, mirror);
+    return;
+  }
   if(!ok) return;
 
   // --------------------------------------------------------------- epilogue
@@ -482,11 +539,11 @@ __global__ void __launch_bounds__(kThreads, 1) sgemm_kernel(const __grid_constan
   }
 }
 
-template <Fetch FA, Fetch FB, bool DUAL>
+template <Fetch FA, Fetch FB, bool DUAL, bool TURN = false>
 struct Kernel {
   static constexpr int kStages = DUAL ? 3 : 4;
   static constexpr int kSmem = kStages * (DUAL ? 4 : 2) * kTileBytes + 1024 + 2 * kStages * 8;
-  static constexpr auto fn = sgemm_kernel<FA, FB, DUAL, kStages>;
+  static constexpr auto fn = sgemm_kernel<FA, FB, DUAL, TURN, kStages>;
 
   // Once per device context: shared-memory opt-in and the register check of
   // the warp split (setmaxnreg draws on the registers of the launch).
@@ -684,9 +741,7 @@ int square_split(const int (&cap)[kMaxSplit + 1], int64_t tm, int64_t ktiles) {
 template <Fetch FA, Fetch FB, bool DUAL>
 gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand& oa, const Operand& ob, bool lower,
     const Fp32Split& split) {
-  using Kn = Kernel<FA, FB, DUAL>;
-  gbpoly_status st = Kn::prepare(ctx);
-  if(st != GBPOLY_OK) return st;
+  gbpoly_status st = GBPOLY_OK;
   const int64_t tm = (a.M + kBM - 1) / kBM, tn = (a.N + kBN - 1) / kBN, ktiles = (a.K + kBK - 1) / kBK;
   const int64_t tiles = lower ? tm * (tm + 1) / 2 : tm * tn;
   if(tiles >= (1ll << 31)) return fail(GBPOLY_ERR_UNSUPPORTED, "too many output tiles");
@@ -697,14 +752,22 @@ gbpoly_status launch_sgemm(gbpoly_ctx* ctx, const GemmF32Args& a, const Operand&
   };
   if(FA == Fetch::Tma && (st = map(&ta, oa)) != GBPOLY_OK) return st;
   if(FB == Fetch::Tma && (st = map(&tb, ob)) != GBPOLY_OK) return st;
-  for(int64_t t0 = 0; t0 < tiles;) {
-    const bool first = t0 < split.rows;
-    const int64_t t1 = first ? split.rows : tiles;
-    const int s = first ? split.first : split.rest;
+  const bool turn = (reinterpret_cast<uintptr_t>(a.C) & 15) != 0 || (a.ldc & 3) != 0;
+  auto launch = [&](auto kernel, int64_t t0, int64_t t1, int s) -> gbpoly_status {
+    using Kn = decltype(kernel);
+    if((st = Kn::prepare(ctx)) != GBPOLY_OK) return st;
     ProfileScope prof(ctx, DUAL ? "sgemm_simt_dual" : "sgemm_simt");
     typename Kn::Launch l(ctx, unsigned(t1 - t0), unsigned(s));
     GBPOLY_CUDA_TRY(cudaLaunchKernelEx(&l.cfg, Kn::fn, ta, tb, oa, ob, int(a.M), int(a.N), int(a.K), a.alpha, a.beta,
         a.C, a.ldc, lower ? 1 : 0, int(t0), int((ktiles + s - 1) / s), ctx->err_dev));
+    return GBPOLY_OK;
+  };
+  for(int64_t t0 = 0; t0 < tiles;) {
+    const bool first = t0 < split.rows;
+    const int64_t t1 = first ? split.rows : tiles;
+    const int s = first ? split.first : split.rest;
+    st = turn && s == 1 ? launch(Kernel<FA, FB, DUAL, true>{}, t0, t1, s) : launch(Kernel<FA, FB, DUAL>{}, t0, t1, s);
+    if(st != GBPOLY_OK) return st;
     t0 = t1;
   }
   return GBPOLY_OK;
@@ -728,10 +791,140 @@ Fetch fetch_of(const Operand& o, bool k_major) {
   return (reinterpret_cast<uintptr_t>(o.X) & 15) == 0 && (o.ld & 3) == 0 && o.R > 0 ? Fetch::Tma : Fetch::Rows;
 }
 
+// ---------------------------------------------------------------- short K, any strides
+// 64 x 64 of C per CTA of 256 threads, 4 x 4 per thread, 16 of K at a time
+// through shared memory: any strides, 64-bit indexes, 64 registers and 8 KB, so
+// that four CTAs of an SM hide one another's start, copies and C.  The same
+// order of K and the same bits as an unsplit sgemm_kernel.
+struct Strided {  // op(X)[r][k] = p[r * s_r + k * s_k]
+  const float* p;
+  int64_t s_r, s_k;
+};
+constexpr int kT64 = 64, kT64K = 16;
+
+__global__ void __launch_bounds__(256) sgemm_tile64_kernel(int64_t M, int64_t N, int64_t K, float alpha, Strided a,
+    Strided b, bool dual, Strided a2, Strided b2, float beta, float* __restrict__ C, int64_t ldc, bool lower) {
+  __shared__ float As[kT64K][kT64 + 1];
+  __shared__ float Bs[kT64K][kT64 + 1];
+  pdl_wait();
+  if(lower && blockIdx.x > blockIdx.y) return;  // strictly above the diagonal: the mirror of another tile
+  const int tid = threadIdx.x;
+  const int tx = tid & 15, ty = tid >> 4;
+  const int64_t m0 = static_cast<int64_t>(blockIdx.y) * kT64, n0 = static_cast<int64_t>(blockIdx.x) * kT64;
+  float acc[4][4];
+#pragma unroll
+  for(int i = 0; i < 4; ++i)
+#pragma unroll
+    for(int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+  const int passes = dual ? 2 : 1;
+  for(int p = 0; p < passes; ++p) {
+    const Strided oa = p ? a2 : a;
+    const Strided ob = p ? b2 : b;
+    for(int64_t k0 = 0; k0 < K; k0 += kT64K) {
+#pragma unroll
+      for(int e = 0; e < 4; ++e) {
+        const int idx = tid + e * 256;
+        // rows fastest when the operand is contiguous along rows, else k fastest
+        const int r = (oa.s_r == 1) ? (idx & 63) : (idx >> 4);
+        const int kk = (oa.s_r == 1) ? (idx >> 6) : (idx & 15);
+        const int64_t gm = m0 + r, gk = k0 + kk;
+        As[kk][r] = (gm < M && gk < K) ? oa.p[gm * oa.s_r + gk * oa.s_k] : 0.f;
+        const int rb = (ob.s_r == 1) ? (idx & 63) : (idx >> 4);
+        const int kb = (ob.s_r == 1) ? (idx >> 6) : (idx & 15);
+        const int64_t gn = n0 + rb, gkb = k0 + kb;
+        Bs[kb][rb] = (gn < N && gkb < K) ? ob.p[gn * ob.s_r + gkb * ob.s_k] : 0.f;
+      }
+      __syncthreads();
+#pragma unroll
+      for(int kk = 0; kk < kT64K; ++kk)
+#pragma unroll
+        for(int i = 0; i < 4; ++i)
+#pragma unroll
+          for(int j = 0; j < 4; ++j) acc[i][j] = fmaf(As[kk][ty * 4 + i], Bs[kk][tx + 16 * j], acc[i][j]);
+      __syncthreads();
+    }
+  }
+  // C values are loaded before the first store (a load cannot move above a
+  // store that may alias it)
+  float cv[4][4];
+#pragma unroll
+  for(int i = 0; i < 4; ++i)
+#pragma unroll
+    for(int j = 0; j < 4; ++j) {
+      const int64_t m = m0 + ty * 4 + i, n = n0 + tx + 16 * j;
+      cv[i][j] = (beta != 0.f && m < M && n < N) ? C[m * ldc + n] : 0.f;
+    }
+#pragma unroll
+  for(int i = 0; i < 4; ++i) {
+    const int64_t m = m0 + ty * 4 + i;
+    if(m >= M) continue;
+#pragma unroll
+    for(int j = 0; j < 4; ++j) {
+      const int64_t n = n0 + tx + 16 * j;
+      if(n < N) C[m * ldc + n] = fmaf(beta, cv[i][j], alpha * acc[i][j]);
+    }
+  }
+  if(lower && blockIdx.x < blockIdx.y) {  // the transposed tile, C[n][m]
+#pragma unroll
+    for(int i = 0; i < 4; ++i)
+#pragma unroll
+      for(int j = 0; j < 4; ++j) {
+        const int64_t m = m0 + ty * 4 + i, n = n0 + tx + 16 * j;
+        cv[i][j] = (beta != 0.f && m < M && n < N) ? C[n * ldc + m] : 0.f;
+      }
+#pragma unroll
+    for(int i = 0; i < 4; ++i) {
+      const int64_t m = m0 + ty * 4 + i;
+      if(m >= M) continue;
+#pragma unroll
+      for(int j = 0; j < 4; ++j) {
+        const int64_t n = n0 + tx + 16 * j;
+        if(n < N) C[n * ldc + m] = fmaf(beta, cv[i][j], alpha * acc[i][j]);
+      }
+    }
+  }
+}
+
+gbpoly_status launch_tile64(gbpoly_ctx* ctx, const GemmF32Args& a, bool lower) {
+  const int64_t gx = (a.N + kT64 - 1) / kT64, gy = (a.M + kT64 - 1) / kT64;
+  if(gy > 65535) return fail(GBPOLY_ERR_UNSUPPORTED, "matrix too tall for the 64 x 64 kernel's grid");
+  const Strided oa = a.op_a == GBPOLY_OP_N ? Strided{a.A, a.lda, 1} : Strided{a.A, 1, a.lda};
+  const Strided ob = a.op_b == GBPOLY_OP_T ? Strided{a.B, a.ldb, 1} : Strided{a.B, 1, a.ldb};
+  ProfileScope prof(ctx, "sgemm_tiled");
+  GBPOLY_CUDA_TRY(launch_pdl(ctx, sgemm_tile64_kernel, dim3(unsigned(gx), unsigned(gy)), 256, 0, a.M, a.N, a.K, a.alpha,
+      oa, ob, a.dual, Strided{a.A2, a.lda2, 1}, Strided{a.B2, a.ldb2, 1}, a.beta, a.C, a.ldc, lower));
+  return GBPOLY_OK;
+}
+
+bool aligned16(const GemmF32Args& a) {
+  return ((reinterpret_cast<uintptr_t>(a.A) | reinterpret_cast<uintptr_t>(a.B)) & 15) == 0 && ((a.lda | a.ldb) & 3) == 0 &&
+         a.K > 0;
+}
+
+// Which calls take 64 x 64 tiles: those beyond the other kernel's 32-bit
+// coordinates, and short K on operands off 16-byte boundaries, where the big
+// kernel's start with 200 KB of shared memory and its word copies cost more
+// than the products: the fewer tiles, the longer K may be, and for all outputs
+// up to K = 16 (us, 128 x 128 / 64 x 64, odd rows: 300 x 300 K = 16 6.9 / 3.2,
+// 500 x 500 K = 32 7.9 / 4.4, 64 9.5 / 6.8; 1000 x 1000 K = 48 9.9 / 8.0, 64 10.0 /
+// 9.8; 2000 x 2000 K = 16 15.2 / 10.8, 32 15.6 / 16.6; 8192 x 8192 K = 16 164 / 132).
+// A mirrored tile is cheaper in the big kernel, which turns it in shared memory
+// (2000 x 2000 symmetric K = 16 13.9 / 20.5; syr2k 500 x 32 16.9 / 9.3, 2000 x 32
+// 17.4 / 25.7).
+bool use_tile64(gbpoly_ctx* ctx, const GemmF32Args& a) {
+  if(a.M >= (1ll << 31) || a.N >= (1ll << 31) || a.K >= (1ll << 31)) return true;
+  if(aligned16(a) || a.K > 80 || (a.M + kT64 - 1) / kT64 > 65535) return false;
+  const int64_t tiles = ((a.M + kBM - 1) / kBM) * ((a.N + kBN - 1) / kBN), sms = std::max(1, ctx->sm_count);
+  if(a.dual) return tiles <= (a.K <= 32 ? sms : (a.K <= 64 ? 16 : 0));
+  if(a.K <= 32) return symmetric_operand(a) ? tiles <= sms : (a.K <= 16 || 2 * tiles <= 3 * sms);
+  return tiles <= (a.K <= 48 ? sms : (a.K <= 64 ? 32 : 16));
+}
+
 }  // namespace
 
 gbpoly_status fp32_split(gbpoly_ctx* ctx, const GemmF32Args& a, Fp32Split& split) {
-  split = Fp32Split{0, 1, 1};
+  split = Fp32Split{0, 1, 1, use_tile64(ctx, a)};
+  if(split.tile64) return GBPOLY_OK;
   int cap[kMaxSplit + 1] = {};
   gbpoly_status st = cluster_capacity(ctx, cap);
   if(st != GBPOLY_OK) return st;
@@ -758,28 +951,19 @@ gbpoly_status launch_gemm_f32_simt(gbpoly_ctx* ctx, const GemmF32Args& a) {
   if(a.M == 0 || a.N == 0) return GBPOLY_OK;
   const bool a_kmaj = a.op_a == GBPOLY_OP_N;
   const bool b_kmaj = a.op_b == GBPOLY_OP_T;
-  if(a.M >= (1ll << 31) || a.N >= (1ll << 31) || a.K >= (1ll << 31)) {
-    // beyond the kernel's 32-bit tile coordinates
-    TiledOperand<float> oa = a_kmaj ? TiledOperand<float>{a.A, a.lda, 1} : TiledOperand<float>{a.A, 1, a.lda};
-    TiledOperand<float> ob = b_kmaj ? TiledOperand<float>{a.B, a.ldb, 1} : TiledOperand<float>{a.B, 1, a.ldb};
-    TiledOperand<float> oa2{a.A2, a.lda2, 1}, ob2{a.B2, a.ldb2, 1};
-    return launch_tiled_gemm<float>(ctx, a.M, a.N, a.K, a.alpha, oa, ob, a.dual, oa2, ob2, a.beta, a.C, a.ldc,
-        a.M == a.N && (a.dual || symmetric_operand(a)));
-  }
+  const bool symmetric = a.M == a.N && (a.dual || symmetric_operand(a));
+  Fp32Split split = a.split;
+  gbpoly_status st = GBPOLY_OK;
+  if(split.rest == 0 && (st = fp32_split(ctx, a, split)) != GBPOLY_OK) return st;
+  if(split.tile64) return launch_tile64(ctx, a, symmetric);
 
   // op(A) is M x K.  Stored as M x K (K-major) for op N, K x M for op T;
   // op(B) is K x N.  Stored as K x N for op N, N x K (K-major) for op T.
   const int M = int(a.M), N = int(a.N), K = int(a.K);
   const Operand oa = a_kmaj ? Operand{a.A, a.lda, M, K} : Operand{a.A, a.lda, K, M};
   const Operand ob = b_kmaj ? Operand{a.B, a.ldb, N, K} : Operand{a.B, a.ldb, K, N};
-  const bool aligned = ((reinterpret_cast<uintptr_t>(a.A) | reinterpret_cast<uintptr_t>(a.B)) & 15) == 0 &&
-                       ((a.lda | a.ldb) & 3) == 0 && K > 0;
-  if(!aligned && (a.M + 63) / 64 > 65535)  // the limit of these calls, unchanged
+  if(!aligned16(a) && (a.M + 63) / 64 > 65535)
     return fail(GBPOLY_ERR_UNSUPPORTED, "matrix too tall for operands off 16-byte boundaries");
-  const bool symmetric = symmetric_operand(a);
-  Fp32Split split = a.split;
-  gbpoly_status st = GBPOLY_OK;
-  if(split.rest == 0 && (st = fp32_split(ctx, a, split)) != GBPOLY_OK) return st;
   if(a.dual) return launch_sgemm<Fetch::Turn, Fetch::Turn, true>(ctx, a, oa, ob, true, split);
   const Fetch fb = fetch_of(ob, b_kmaj);
   auto launch = [&](const GemmF32Args& part, const Operand& left, int splits) {

@@ -1,7 +1,6 @@
 // Simple tiled GEMM over general strides, templated on the element type.
 //
-// The FP64 DGEMM (the FP64 oracle and the double variants of the benchmarks),
-// and FP32 contractions with a dimension beyond 2^31.
+// The FP64 DGEMM (the FP64 oracle and the double variants of the benchmarks).
 //   op(X)[r][k] = X[r * s_r + k * s_k]
 //   C[m][n] = alpha * (sum_k op(A)[m][k] op(B)[k][n]  [+ op(A2) op(B2)]) + beta * C[m][n]
 // 16 x 16 of C per group of 64 threads, BK = 16; persistent CTAs of eight such
@@ -118,7 +117,7 @@ gbpoly_status launch_tiled_gemm(gbpoly_ctx* ctx, int64_t M, int64_t N, int64_t K
   lower = lower && M == N;
   const int64_t tiles = lower ? gy * (gy + 1) / 2 : gx * gy;
   if(tiles >= (1ll << 31)) return fail(GBPOLY_ERR_UNSUPPORTED, "matrix too large for the tiled kernel grid");
-  ProfileScope prof(ctx, sizeof(T) == 8 ? "dgemm_tiled" : "sgemm_tiled");
+  ProfileScope prof(ctx, "dgemm_tiled");
   const unsigned ctas = unsigned(std::min<int64_t>(tiles, std::max(1, ctx->sm_count)));
   GBPOLY_CUDA_TRY(launch_pdl(ctx, tiled_gemm_kernel<T>, ctas, 64 * kTiledGroups, 0, M, N, K, alpha, a, b, dual, a2, b2,
       beta, C, ldc, lower, gx, tiles));
