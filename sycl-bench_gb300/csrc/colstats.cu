@@ -6,26 +6,31 @@
 // sequentially through global memory (covariance.cpp:84-96,
 // correlation.cpp:111-142).  Here a CTA of 8 warps owns 32 adjacent columns and
 // one chunk of rows; lane j of every warp reads column j (a warp reads 128
-// contiguous bytes of a row), each thread keeps sixteen independent loads in
+// contiguous bytes of a row), each thread keeps eight independent loads in
 // flight, and the 8 warps are combined in shared memory into one partial sum
 // per (chunk, column).  Then, in chunk order, the partials are added and the
 // division (and, for standard deviations, the square root and the eps clamp)
 // applied:
-//   * wide or low matrices (the column blocks times eight chunks give every SM
-//     two CTAs, or a chunk has at most 384 rows): the chunks of a column block
-//     are a cluster, whose first CTA reads the others' partials from their
-//     shared memory: one launch;
-//   * high, narrow ones: partials in global memory, a second launch of one
-//     thread per column; about four CTAs per SM stream the matrix.
+//   * up to 4096 x 4096: the (at most eight) chunks of a column block are a
+//     cluster, whose first CTA reads the others' partials from their shared
+//     memory: one launch;
+//   * beyond: partials in global memory, a second launch of one thread per
+//     column; about four CTAs per SM stream the matrix.
 // The result does not depend on the launch beyond that fixed summation tree
 // (same inputs and shape, same bits).  All arithmetic is FP32.
 //
 // Bound: HBM or L2, one read of the matrix (3000 x 2000: 3.5 us at the measured
-// copy rate); the remainder of a chunk's rows is part of the last batch of
-// loads (loaded one by one it cost as much as the batches).  Mean and standard
-// deviation together, us, partials in global memory / clusters: 4000 x 4000
-// 40.8 / 34.6, 3000 x 2000 21.5 / 21.0, 1000 x 1300 13.7 / 10.3, 1000 x 300 9.8 /
-// 6.8, 3000 x 160 14.0 / 9.7; 4096 x 600 12.8 / 19.2.
+// copy rate).  Mean and standard deviation together, us, clusters / partials in
+// global memory: 100 x 100 5.0 / 6.5, 1000 x 1300 7.7 / 11.8, 3000 x 2000 12.9 /
+// 14.3, 4000 x 4000 21 / 25, 4096 x 600 10.4 / 10.4; but 10000 x 1216 22 / 18,
+// 100000 x 1300 270 / 184, 20000 x 8192 236 / 219, 2000 x 30000 105 / 88, 500 x
+// 20000 30 / 17: a cluster's eight chunks are too few CTAs for a high matrix,
+// and more than a wave of them for a wide one.
+//
+// No kernel here triggers the next one early: CTAs of later kernels would be
+// resident, waiting, on whichever SMs had room, and a grid of a wave of CTAs
+// so placed leaves other SMs idle (100000 x 1300, calls queued back to back:
+// 252 us with the early trigger, 185 without).
 #include "gbpoly_internal.cuh"
 
 namespace gbpoly {
@@ -33,45 +38,58 @@ namespace {
 
 constexpr int kColsPerBlock = 32;
 constexpr int kWarps = 8;
+constexpr int64_t kClusterRows = 4096, kClusterCols = 4096;  // largest matrix reduced by clusters
 
 // sum over rows [r0, r1) of f(X[r][j]) for this thread's column j, rows
-// warp, warp + 8, ... of the chunk; sixteen loads in flight.
-template <bool CENTERED>
+// warp, warp + 8, ... of the chunk; eight loads in flight.  What is left after
+// the full batches is loaded together (TAIL: short chunks, where it is a good
+// part of the work) or row by row (long chunks: the tail's predicates cost
+// registers and with them resident CTAs; 2000 x 30000, mean and deviation, 99
+// us against 88).
+template <bool CENTERED, bool TAIL>
 __device__ __forceinline__ float column_chunk_sum(const float* __restrict__ col, int64_t ldx, int r0, int r1, int warp,
     float m) {
-  constexpr int kLoads = 16, kSums = 8;
-  float a[kSums];
+  constexpr int kLoads = 8;
+  float a[kLoads];
 #pragma unroll
-  for(int k = 0; k < kSums; ++k) a[k] = 0.f;
-  for(int r = r0 + warp; r < r1; r += kLoads * kWarps) {
+  for(int k = 0; k < kLoads; ++k) a[k] = 0.f;
+  auto add = [&](float& s, float x) {
+    if constexpr(CENTERED) {
+      const float c = x - m;
+      s = fmaf(c, c, s);
+    } else {
+      s += x;
+    }
+  };
+  int r = r0 + warp;
+  for(; r + (kLoads - 1) * kWarps < r1; r += kLoads * kWarps) {
     float v[kLoads];
 #pragma unroll
-    for(int k = 0; k < kLoads; ++k) {
-      const int rk = r + k * kWarps;
-      v[k] = rk < r1 ? col[int64_t(rk) * ldx] : 0.f;
-    }
+    for(int k = 0; k < kLoads; ++k) v[k] = col[int64_t(r + k * kWarps) * ldx];
 #pragma unroll
-    for(int k = 0; k < kLoads; ++k) {
-      if constexpr(CENTERED) {
-        // beyond the chunk nothing is added (m - m would be NaN for an infinite mean)
-        const float c = r + k * kWarps < r1 ? v[k] - m : 0.f;
-        a[k % kSums] = fmaf(c, c, a[k % kSums]);
-      } else {
-        a[k % kSums] += v[k];
-      }
-    }
+    for(int k = 0; k < kLoads; ++k) add(a[k], v[k]);
+  }
+  if constexpr(TAIL) {
+    float v[kLoads];
+#pragma unroll
+    for(int k = 0; k < kLoads; ++k) v[k] = r + k * kWarps < r1 ? col[int64_t(r + k * kWarps) * ldx] : 0.f;
+#pragma unroll
+    for(int k = 0; k < kLoads; ++k)
+      if(r + k * kWarps < r1) add(a[k], v[k]);  // beyond the chunk nothing: m - m is NaN for an infinite mean
+  } else {
+    for(; r < r1; r += kWarps) add(a[0], col[int64_t(r) * ldx]);
   }
   return ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
 }
 
 // The chunk's sum for column lane of the block, in every lane of warp 0 (all threads call it).
-template <bool CENTERED>
+template <bool CENTERED, bool TAIL>
 __device__ __forceinline__ float block_chunk_sum(const float* __restrict__ X, int64_t ldx, int cols, int r0, int r1, int j,
     const float* __restrict__ mean) {
   __shared__ float red[kWarps][kColsPerBlock + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float s = 0.f;
-  if(j < cols) s = column_chunk_sum<CENTERED>(X + j, ldx, r0, r1, warp, CENTERED ? mean[j] : 0.f);
+  if(j < cols) s = column_chunk_sum<CENTERED, TAIL>(X + j, ldx, r0, r1, warp, CENTERED ? mean[j] : 0.f);
   red[warp][lane] = s;
   __syncthreads();
   float t = red[0][lane];
@@ -95,11 +113,11 @@ template <bool STDDEV>
 __global__ void __launch_bounds__(kWarps * 32) column_cluster_kernel(const float* __restrict__ X, int64_t ldx, int rows,
     int cols, int rows_per_chunk, const float* __restrict__ mean, float divisor, float eps, float* __restrict__ out) {
   __shared__ float part[kColsPerBlock];
-  pdl_enter();
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = blockIdx.x * kColsPerBlock + lane;
   const int r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
-  const float t = block_chunk_sum<STDDEV>(X, ldx, cols, r0, r1, j, mean);
+  const float t = block_chunk_sum<STDDEV, true>(X, ldx, cols, r0, r1, j, mean);
   if(warp == 0) part[lane] = t;
   cluster_sync();
   if(blockIdx.y == 0 && warp == 0) {
@@ -114,11 +132,11 @@ __global__ void __launch_bounds__(kWarps * 32) column_cluster_kernel(const float
 template <bool CENTERED>
 __global__ void __launch_bounds__(kWarps * 32) column_partial_kernel(const float* __restrict__ X, int64_t ldx, int rows,
     int cols, int rows_per_chunk, const float* __restrict__ mean, float* __restrict__ partial) {
-  pdl_enter();
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = blockIdx.x * kColsPerBlock + lane;
   const int r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
-  const float t = block_chunk_sum<CENTERED>(X, ldx, cols, r0, r1, j, mean);
+  const float t = block_chunk_sum<CENTERED, false>(X, ldx, cols, r0, r1, j, mean);
   if(warp == 0 && j < cols) partial[int64_t(blockIdx.y) * cols + j] = t;
 }
 
@@ -127,7 +145,7 @@ __global__ void __launch_bounds__(kWarps * 32) column_partial_kernel(const float
 template <bool STDDEV>
 __global__ void column_final_kernel(const float* __restrict__ partial, int chunks, int cols, float divisor, float eps,
     float* __restrict__ out) {
-  pdl_enter();
+  pdl_wait();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if(j >= cols) return;
   float s = 0.f;
@@ -141,7 +159,7 @@ template <bool SCALED>
 __global__ void __launch_bounds__(256) center_columns_kernel(const float* X, int64_t ldx, int rows, int cols,
     const float* __restrict__ mean, const float* __restrict__ stddev, float scale_div, float* Y, int64_t ldy,
     int rows_per_block) {
-  pdl_enter();
+  pdl_wait();
   const int j = blockIdx.x * 32 + (threadIdx.x & 31);
   if(j >= cols) return;
   const float m = mean[j];
@@ -168,7 +186,7 @@ __global__ void __launch_bounds__(256) center_columns_kernel(const float* X, int
 }
 
 __global__ void set_diagonal_kernel(int64_t n, float value, float* C, int64_t ldc) {
-  pdl_enter();
+  pdl_wait();
   for(int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
     C[i * ldc + i] = value;
 }
@@ -196,7 +214,7 @@ gbpoly_status column_reduce(gbpoly_ctx* ctx, int64_t rows, int64_t cols, const f
   if(cols == 0) return GBPOLY_OK;
   const int col_blocks = int((cols + kColsPerBlock - 1) / kColsPerBlock);
   const int cluster = int(std::max<int64_t>(1, std::min<int64_t>(8, (rows + 63) / 64)));
-  if(int64_t(col_blocks) * 8 >= 2ll * std::max(ctx->sm_count, 1) || rows <= 8 * 384) {
+  if(rows <= kClusterRows && cols <= kClusterCols) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[2];
     cfg.gridDim = dim3(unsigned(col_blocks), unsigned(cluster));
