@@ -11,16 +11,18 @@
 //     t, t + 256, ..., four 32-bit loads of adjacent lanes) and a group of
 //     rows; each row of the tile is one coalesced 4 KB read, 16 rows in flight
 //     per thread (8 per matrix for two);
-//   * row dots: a thread's 4 columns give one term per row; each group of 8
-//     rows in flight is reduced across the warp at once (a halving transpose
+//   * row dots: a thread's 4 columns give one term per row; each group of rows
+//     in flight is reduced across the warp at once (a halving transpose
 //     exchange: 16 shuffles for 16 rows), the 8 warps in shared memory per
 //     32-row block, into one partial per (column tile, row);
 //   * column sums: 4 accumulators per thread over all rows of the group,
 //     one partial per (row group, column);
-//   * a final kernel (16 warps per 32 outputs) adds the partials in a fixed
-//     order and applies y = beta * y + alpha * sum (gesummv: tmp += A x,
-//     y = alpha tmp + beta (y + B x)).
+//   * a final kernel (1 to 16 warps per 32 outputs, by the number of partials)
+//     adds them in a fixed order and applies y = beta * y + alpha * sum
+//     (gesummv: tmp += A x, y = alpha tmp + beta (y + B x)).
 // Deterministic: the summation tree depends only on the shape and SM count.
+// No kernel here triggers the next one early: its waiting CTAs would settle on
+// the SMs that drain first (queued calls 0.5 to 1 us slower).
 #include "gbpoly_internal.cuh"
 
 namespace gbpoly {
@@ -29,6 +31,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kTileCols = 4 * kThreads;  // 1024
 constexpr int kRowBlock = 32;
+constexpr int kRowBatch = 16;  // row groups are multiples of this
 // rows in flight per thread: 16 for one matrix, 8 each for two (gesummv)
 template <bool TWO>
 constexpr int rows_in_flight() {
@@ -109,7 +112,7 @@ __device__ __forceinline__ float reduce_rows(float (&v)[V], int lane) {
 template <int NR, bool NC, bool TWO, bool VEC>
 __global__ void __launch_bounds__(kThreads, 2) gemv_partial_kernel(const GemvArgs g) {
   __shared__ float red[NR > 0 ? NR : 1][kThreads / 32][kRowBlock];
-  pdl_enter();
+  pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tile = blockIdx.x;
   const int c0 = tile * kTileCols;
@@ -180,24 +183,42 @@ __device__ __forceinline__ float apply(const Term& t, float s, int i) {
   return t.beta == 0.f ? t.alpha * s : fmaf(t.alpha, s, t.beta * t.y[i]);
 }
 
-// Final pass, one CTA per 32 outputs: warp w adds the partials with index
-// w, w + 16, ... of output (blockIdx.x * 32 + lane), eight loads in flight; the
-// 16 warp sums are combined in shared memory in warp order.
+// Final pass: the partials of each output added in a fixed order, then
 //   row terms:   y_r[i] = beta y_r[i] + alpha sum over column tiles of row_part[t][.][i]
 //   column term: y_c[j] = beta y_c[j] + alpha sum over row groups of col_part[.][j]
 //   GESUMMV:     tmp += S0, y = alpha tmp + beta (y + S1) (row terms 0, 1)
-constexpr int kFinalWarps = 16;
+// W warps share 32 outputs (lane = output): warp w of them adds the partials
+// w, w + W, ..., eight loads in flight, and their sums are combined in shared
+// memory in warp order.  A CTA of 16 warps holds 16 / W such groups; the first
+// row_blocks CTAs take the row outputs, the others the column outputs, each
+// with the W that final_warps gives for its number of partials.
+//
+// Bound: starting CTAs where outputs are many and their partials few, the
+// latency of the chain of loads where the partials are many, so W follows both
+// (us of the whole call, 16 warps for every 32 outputs / this rule: mvt 1000000
+// x 200 613 / 386, bicg 200 x 1000000 231 / 143, bicg 4096 x 4096 12.3 / 10.2).
+constexpr int kFinalWarps = 16, kFinalLoads = 8;
 
-// Sum over p[g * stride], g = warp, warp + 16, ... < n.
-__device__ __forceinline__ float strided_sum(const float* __restrict__ p, int64_t stride, int n, int warp) {
-  constexpr int kLoads = 8;
-  float s[kLoads];
+// Groups of 32 outputs that share a CTA's warps, as CTAs.
+int64_t final_blocks(int64_t outputs, int w) { return (outputs + 32 * kFinalWarps / w - 1) / (32 * kFinalWarps / w); }
+
+// The least power of two of warps whose loads in flight cover n partials; more,
+// up to one partial each, while the outputs give fewer CTAs than the device has SMs.
+int final_warps(int64_t outputs, int n, int sms) {
+  int w = 1;
+  while(w < kFinalWarps && (n > kFinalLoads * w || (w < n && final_blocks(outputs, w) < sms))) w *= 2;
+  return w;
+}
+
+// Sum over p[g * stride], g = first, first + step, ... < n.
+__device__ __forceinline__ float strided_sum(const float* __restrict__ p, int64_t stride, int n, int first, int step) {
+  float s[kFinalLoads];
 #pragma unroll
-  for(int k = 0; k < kLoads; ++k) s[k] = 0.f;
-  for(int g = warp; g < n; g += kLoads * kFinalWarps) {
+  for(int k = 0; k < kFinalLoads; ++k) s[k] = 0.f;
+  for(int g = first; g < n; g += kFinalLoads * step) {
 #pragma unroll
-    for(int k = 0; k < kLoads; ++k) {
-      const int i = g + k * kFinalWarps;
+    for(int k = 0; k < kFinalLoads; ++k) {
+      const int i = g + k * step;
       s[k] += i < n ? p[int64_t(i) * stride] : 0.f;
     }
   }
@@ -206,36 +227,59 @@ __device__ __forceinline__ float strided_sum(const float* __restrict__ p, int64_
 
 template <int NR, bool NC, bool GESUMMV>
 __global__ void __launch_bounds__(32 * kFinalWarps) gemv_final_kernel(const float* __restrict__ row_part, int col_tiles,
-    int rows, const float* __restrict__ col_part, int row_groups, int cols, Term r0, Term r1, Term cterm) {
-  constexpr int kSums = (NR > 0 ? NR : 0) + (NC ? 1 : 0);
-  __shared__ float red[kSums > 0 ? kSums : 1][kFinalWarps][32];
-  pdl_enter();
+    int rows, int row_warps, int row_blocks, const float* __restrict__ col_part, int row_groups, int cols, int col_warps,
+    Term r0, Term r1, Term cterm) {
+  constexpr int kSums = NR > 1 ? NR : 1;
+  __shared__ float red[kSums][kFinalWarps][32];
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int i = blockIdx.x * 32 + lane;
+  const bool row_side = NR > 0 && (!NC || int(blockIdx.x) < row_blocks);
+  const int W = row_side ? row_warps : col_warps, part = warp & (W - 1);
+  const int block = int(blockIdx.x) - (row_side ? 0 : row_blocks);
+  const int64_t i = ((int64_t(block) * kFinalWarps + warp) >> (31 - __clz(W))) * 32 + lane;
+  if(row_side) {
 #pragma unroll
-  for(int t = 0; t < NR; ++t)
-    red[t][warp][lane] = i < rows ? strided_sum(row_part + int64_t(t) * col_tiles * rows + i, rows, col_tiles, warp) : 0.f;
-  if constexpr(NC) red[kSums - 1][warp][lane] = i < cols ? strided_sum(col_part + i, cols, row_groups, warp) : 0.f;
+    for(int t = 0; t < NR; ++t)
+      red[t][warp][lane] =
+          i < rows ? strided_sum(row_part + int64_t(t) * col_tiles * rows + i, rows, col_tiles, part, W) : 0.f;
+  } else if constexpr(NC) {
+    red[0][warp][lane] = i < cols ? strided_sum(col_part + i, cols, row_groups, part, W) : 0.f;
+  }
   __syncthreads();
-  if(warp != 0) return;
-  float sum[kSums > 0 ? kSums : 1];
+  if(part != 0) return;
+  float sum[kSums];
 #pragma unroll
   for(int t = 0; t < kSums; ++t) {
+    if(t > 0 && !row_side) break;
     sum[t] = 0.f;
-#pragma unroll
-    for(int w = 0; w < kFinalWarps; ++w) sum[t] += red[t][w][lane];
+    for(int w = 0; w < W; ++w) sum[t] += red[t][warp + w][lane];
   }
-  if(NR > 0 && i < rows) {
+  if(row_side) {
+    if(NR == 0 || i >= rows) return;
     if constexpr(GESUMMV) {
       const float tmp = r0.y[i] + sum[0];
       r0.y[i] = tmp;
       r1.y[i] = r1.beta == 0.f ? r1.alpha * tmp : fmaf(r1.alpha, tmp, r1.beta * (r1.y[i] + sum[NR > 1 ? 1 : 0]));
     } else {
       r0.y[i] = apply(r0, sum[0], i);
-      if constexpr(NR > 1) r1.y[i] = apply(r1, sum[NR > 1 ? 1 : 0], i);
+      if constexpr(NR > 1) r1.y[i] = apply(r1, sum[1], i);
     }
+  } else if constexpr(NC) {
+    if(i < cols) cterm.y[i] = apply(cterm, sum[0], i);
   }
-  if(NC && i < cols) cterm.y[i] = apply(cterm, sum[kSums - 1], i);
+}
+
+// The final pass over `rows` row outputs of col_tiles partials and `cols` column outputs of row_groups partials.
+template <int NR, bool NC, bool GESUMMV>
+gbpoly_status launch_final(gbpoly_ctx* ctx, const float* row_part, int col_tiles, int rows, const float* col_part,
+    int row_groups, int cols, Term r0, Term r1, Term ct) {
+  const int rw = final_warps(rows, col_tiles, ctx->sm_count), cw = final_warps(cols, row_groups, ctx->sm_count);
+  const int64_t row_blocks = NR > 0 ? final_blocks(rows, rw) : 0, all = row_blocks + (NC ? final_blocks(cols, cw) : 0);
+  if(all == 0) return GBPOLY_OK;
+  ProfileScope prof(ctx, "gemv_final");
+  GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_final_kernel<NR, NC, GESUMMV>, unsigned(all), 32 * kFinalWarps, 0, row_part,
+      col_tiles, rows, rw, int(row_blocks), col_part, row_groups, cols, cw, r0, r1, ct));
+  return GBPOLY_OK;
 }
 
 template <int NR, bool NC, bool TWO, bool GESUMMV>
@@ -249,7 +293,8 @@ gbpoly_status launch_gemv(gbpoly_ctx* ctx, GemvArgs g, Term r0, Term r1, Term ct
   const int64_t ctas = 2ll * std::max(ctx->sm_count, 1);
   const int64_t two_waves = std::max<int64_t>(1, 2 * ctas / col_tiles), one_wave = std::max<int64_t>(1, ctas / col_tiles);
   const int64_t want_groups = g.rows / two_waves >= (TWO ? 16 : 64) ? two_waves : one_wave;
-  const int rpg = std::max<int>(rows_in_flight<TWO>(), int((g.rows + want_groups - 1) / want_groups));
+  // whole batches of loads: a last one of a few rows takes as long as a full one (bicg 1000000 x 200 370 -> 356 us)
+  const int rpg = int((std::max<int64_t>(1, (g.rows + want_groups - 1) / want_groups) + kRowBatch - 1) / kRowBatch * kRowBatch);
   const int row_groups = std::max(1, (g.rows + rpg - 1) / rpg);
   if(row_groups > 65535) return fail(GBPOLY_ERR_UNSUPPORTED, "too many rows");
   g.col_tiles = col_tiles;
@@ -273,13 +318,9 @@ gbpoly_status launch_gemv(gbpoly_ctx* ctx, GemvArgs g, Term r0, Term r1, Term ct
     else
       GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_partial_kernel<NR, NC, TWO, false>, grid, kThreads, 0, g));
   }
-  const int n = std::max(g.rows, g.cols);
-  if(n == 0) return GBPOLY_OK;
-  ProfileScope prof(ctx, "gemv_final");
   const bool some = g.rows > 0 && g.cols > 0;
-  GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_final_kernel<NR, NC, GESUMMV>, unsigned((n + 31) / 32), 32 * kFinalWarps, 0, g.row_part,
-      some ? col_tiles : 0, g.rows, g.col_part, some ? row_groups : 0, g.cols, r0, r1, ct));
-  return GBPOLY_OK;
+  return launch_final<NR, NC, GESUMMV>(ctx, g.row_part, some ? col_tiles : 0, g.rows, g.col_part, some ? row_groups : 0,
+      g.cols, r0, r1, ct);
 }
 
 // atax in one kernel and one read of A: tmp += A x, then y += A^T tmp.  A CTA
@@ -302,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, atax_ctas(CHUNKS)) atax_kernel(const
     int rows, int cols, const float* __restrict__ x, float* __restrict__ tmp, float* __restrict__ col_part) {
   constexpr int R = atax_rows(CHUNKS);
   __shared__ float red[2][kThreads / 32 + 1][R];  // warp sums and the old tmp, alternating sets
-  pdl_enter();
+  pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int begin = int(int64_t(rows) * blockIdx.x / gridDim.x);
   const int count = int(int64_t(rows) * (blockIdx.x + 1) / gridDim.x) - begin;
@@ -366,10 +407,7 @@ gbpoly_status launch_atax(gbpoly_ctx* ctx, const float* A, int64_t lda, int rows
     GBPOLY_CUDA_TRY(launch_pdl(ctx, vec ? atax_kernel<CHUNKS, true> : atax_kernel<CHUNKS, false>, grid, kThreads, 0, A, lda,
         rows, cols, x, tmp, col_part));
   }
-  ProfileScope prof(ctx, "gemv_final");
-  GBPOLY_CUDA_TRY(launch_pdl(ctx, gemv_final_kernel<0, true, false>, unsigned((cols + 31) / 32), 32 * kFinalWarps, 0,
-      nullptr, 0, rows, col_part, grid, cols, Term{}, Term{}, Term{1.f, 1.f, y}));
-  return GBPOLY_OK;
+  return launch_final<0, true, false>(ctx, nullptr, 0, 0, col_part, grid, cols, Term{}, Term{}, Term{1.f, 1.f, y});
 }
 
 gbpoly_status check_common(gbpoly_ctx* ctx, int64_t rows, int64_t cols, const float* A, int64_t lda) {
