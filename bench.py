@@ -4,7 +4,10 @@
 
 One step = one C = alpha*A*B + beta*C over N x N FP32 matrices (polybench gemm
 initialisation, alpha=32412, beta=2123, N=8192 by default), all operands
-resident in HBM.  Prints one JSON line (rank 0).  Under torchrun every rank
+resident in HBM.  Prints one JSON line on standard output (rank 0) and, on
+standard error, a second record with every form's and every other workload's
+figures: the first stays short enough to be read whole from the end of a
+captured output.  Under torchrun every rank
 runs an independent replica on its own GPU (the contraction has no exchange
 step), so scaling is weak and `value` sums all ranks' work over the slowest
 rank's time.
@@ -1163,6 +1166,19 @@ def cpu_gemm_sample(n: int, target_s: float) -> dict:
             "cores": lib.orc_num_threads()}
 
 
+def output_records(base: dict, res: dict, cpu: dict | None) -> tuple[dict, dict]:
+    """The headline line and the record of details beside it."""
+    line = dict(base, value=res["value"], ms_per_step=res["ms_per_step"], dtype=DTYPE_OF_FORM[res["headline"]],
+                e2e={k: v for k, v in res["e2e"].items() if k != "link"}, roofline=res["roofline"], cpu_baseline=cpu,
+                clocks=res["clocks"], err_vs_fp64=res["err_vs_fp64"], matched_error=res["matched_error"],
+                gpu_launches=res["gpu_launches"], headline_form=res["headline"])
+    details = {"details_of": base["metric"], "e2e_link": res["e2e"].get("link"), "tiers": res["tiers"],
+               "device": {"sm_count": res["device"]["sm_count"], "cc": list(res["device"]["cc"])},
+               "peaks": res["peak_kind"], "grouped": res["grouped"], "family": res["family"],
+               "neighbours": res["neighbours"], "small_k": res["small_k"]}
+    return line, details
+
+
 def main() -> None:
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -1224,14 +1240,8 @@ def main() -> None:
                "sample": f"first {r['rows']} of {n} output rows of the gemm.cpp:82-91 kernel body on the host "
                          f"cores ({r['seconds']:.1f} s), oracle port built -O3 -ffast-math"}
     if dist.rank == 0:
-        line = dict(base, value=res["value"], ms_per_step=res["ms_per_step"],
-                    dtype=DTYPE_OF_FORM[res["headline"]],
-                    e2e=res["e2e"], roofline=res["roofline"], cpu_baseline=cpu, clocks=res["clocks"],
-                    err_vs_fp64=res["err_vs_fp64"], matched_error=res["matched_error"],
-                    gpu_launches=res["gpu_launches"], tiers=res["tiers"], headline_form=res["headline"],
-                    device={"sm_count": res["device"]["sm_count"], "cc": list(res["device"]["cc"])},
-                    peaks=res["peak_kind"], grouped=res["grouped"], family=res["family"],
-                    neighbours=res["neighbours"], small_k=res["small_k"])
+        line, details = output_records(base, res, cpu)
+        print(json.dumps(details), file=sys.stderr)
         print(json.dumps(line))
     dist.close()
 
