@@ -109,27 +109,40 @@ gbpoly_status gbpoly_memset(gbpoly_ctx* ctx, void* dst, int value, size_t bytes)
  * least `bytes` large now, so that later calls of that size do not allocate.
  * Needed before capturing tensor-core calls into a graph.  Synchronises. */
 gbpoly_status gbpoly_workspace_reserve(gbpoly_ctx* ctx, size_t bytes);
-/* Workspace bytes a contraction of this shape and form needs at most (fp32:
- * its kernels need none; for shapes whose output tiles are too few to fill the
- * device the partial products of a K split are still reported). */
+/* Workspace bytes a contraction of this shape and form needs at most.  fp32's
+ * kernels need none; for shapes whose output tiles are too few to fill the
+ * device the figure of a K split in global memory is reported all the same,
+ * an upper bound that callers' sizing has relied on. */
 gbpoly_status gbpoly_workspace_query(gbpoly_precision prec, int64_t M, int64_t N, int64_t K, int same_operand,
     size_t* bytes);
 
 /* -------------------------------------------------------------- autotuner -- */
 
 /* Each tensor-core form has a few compiled tile configurations: tile width,
- * K bytes per pipeline stage, pipeline depth and cluster size (tf32, bf16x3,
- * tf32x3, bf16x6: configurations 3, 4 and 5 run CTA pairs, cta_group::2 MMAs
- * on 256 x 256 tiles; 5 keeps the C tile in shared memory, loaded and stored
- * by TMA, for short K, and runs as 3 for symmetric products or C rows that
- * do not start and end on 16-byte boundaries; 6 runs CTA pairs on 256 x 128
- * tiles.  fp16x3: 2 pairs on 256 x 256, 3 on 256 x 128).  The context keeps
- * one per (form, ceil(log2) of M, N, K); unless tuned or set, a shape whose
- * 256 x 256 tiles give every SM pair a tile uses configuration 5 up to
- * K = 128 (tf32: 512, tf32x3, bf16x6: 64), 6 up to K = 384 (tf32x3: 192) and 3
- * beyond (fp16x3: 3, then 2), a smaller or symmetric one the tile shape
- * (128 x 128, 256 x 256, 256 x 128) of the least estimated time.  fp8: configuration 1 (128 x 256 tiles) when its tiles give
- * every SM one, else 0 (128 x 128, also every symmetric product). */
+ * K bytes per pipeline stage, pipeline depth and cluster size.
+ *
+ *   tf32, bf16x3, tf32x3, bf16x6
+ *     0-2   one CTA per tile (128 x 256 or 128 x 128)
+ *     3, 4  CTA pairs (cta_group::2 MMAs) on 256 x 256 tiles
+ *     5     as 3 with the C tile in shared memory, loaded and stored by TMA,
+ *           for short K; runs as 3 for symmetric products and for C rows that
+ *           do not start and end on 16-byte boundaries
+ *     6     CTA pairs on 256 x 128 tiles
+ *   fp16x3
+ *     0, 1  one CTA per tile (128 x 256, 128 x 128)
+ *     2, 3  CTA pairs on 256 x 256, on 256 x 128
+ *   fp8
+ *     0, 1  one CTA per tile (128 x 128, 128 x 256)
+ *
+ * The context keeps one configuration per (form, ceil(log2) of M, N, K).
+ * Unless tuned or set:
+ *   - a shape whose 256 x 256 tiles give every SM pair a tile uses 5 up to
+ *     K = 128 (tf32: 512; tf32x3, bf16x6: 64), then 6 up to K = 384 (tf32x3:
+ *     192), then 3 (fp16x3: 3 up to K = 384, then 2);
+ *   - a smaller or symmetric one uses the tile shape (128 x 128, 256 x 256,
+ *     256 x 128) of the least estimated time;
+ *   - fp8 uses 1 when its tiles give every SM one, else 0 (also every
+ *     symmetric product). */
 gbpoly_status gbpoly_gemm_config_count(gbpoly_precision prec, int* count);
 gbpoly_status gbpoly_gemm_config_set(gbpoly_ctx* ctx, gbpoly_precision prec, int64_t M, int64_t N, int64_t K,
     int config);
@@ -146,8 +159,8 @@ gbpoly_status gbpoly_autotune_save(gbpoly_ctx* ctx, const char* path);
 gbpoly_status gbpoly_autotune_load(gbpoly_ctx* ctx, const char* path, int* loaded);
 /* K-split tail (CTA-pair configurations, on by default): when the last round
  * of tiles would leave at least half the resident SM pairs idle and half a
- * tile's K takes longer than the handoff (7 to 9 us), each tile of that round
- * runs as two halves of its K range on two pairs;
+ * tile's K takes longer than the handoff (7 us, in a round after others 8),
+ * each tile of that round runs as two halves of its K range on two pairs;
  * the first half adds the second half's partial sums (in a fixed order, so
  * results are the same on every run) and writes C.  The workspace query
  * includes the partial sums. */

@@ -245,10 +245,12 @@ size_t workspace_bytes(gbpoly_precision prec, int64_t M, int64_t N, int64_t K, b
 
 // Launch on the context's stream so that the kernel's CTAs may become resident
 // while the kernel queued before it still runs (programmatic stream
-// serialization).  Every kernel launched this way calls pdl_trigger and then,
-// before it touches global memory, pdl_wait, which returns when all earlier
-// work of the stream has completed: what overlaps is launch latency and the
-// set-up of shared and tensor memory, never data.
+// serialization).  Every kernel launched this way calls pdl_wait before it
+// touches global memory, which returns when all earlier work of the stream has
+// completed: what overlaps is launch latency and the set-up of shared and
+// tensor memory, never data.  A kernel that calls pdl_trigger first lets the
+// next one's CTAs become resident while it runs; without it they do when its
+// own end.
 template <class... Params, class... Args>
 cudaError_t launch_pdl(gbpoly_ctx* ctx, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
