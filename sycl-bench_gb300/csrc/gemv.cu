@@ -15,8 +15,8 @@
 //     in flight is reduced across the warp at once (a halving transpose
 //     exchange: 16 shuffles for 16 rows), the 8 warps in shared memory per
 //     32-row block, into one partial per (column tile, row);
-//   * column sums: 4 accumulators per thread over all rows of the group,
-//     one partial per (row group, column);
+//   * column sums: 4 accumulators per thread over all rows of the group, a
+//     batch of 16 (8) rows at a time, one partial per (row group, column);
 //   * a final kernel (1 to 16 warps per 32 outputs, by the number of partials)
 //     adds them in a fixed order and applies y = beta * y + alpha * sum
 //     (gesummv: tmp += A x, y = alpha tmp + beta (y + B x)).
@@ -107,6 +107,13 @@ __device__ __forceinline__ float reduce_rows(float (&v)[V], int lane) {
   return r;
 }
 
+// v(0) + ... + v(7), the eight warps' sums, in pairs.
+template <class V>
+__device__ __forceinline__ float sum8(V v) {
+  static_assert(kThreads / 32 == 8, "eight warps");
+  return ((v(0) + v(1)) + (v(2) + v(3))) + ((v(4) + v(5)) + (v(6) + v(7)));
+}
+
 // NR row dots (0..2), NC: one column sum, TWO: row dot 1 reads B.
 // VEC: 16-byte aligned rows and columns a multiple of 4 (128-bit loads).
 template <int NR, bool NC, bool TWO, bool VEC>
@@ -147,23 +154,25 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_partial_kernel(const GemvArg
         if(lane < kInFlight) red[t][warp][rr + lane] = rs;
       }
       if constexpr(NC) {
+        // the batch by itself, then onto the group's sum: a chain of 16 terms and
+        // one of batches, not one of all the group's rows
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for(int k = 0; k < kInFlight; ++k) {
           const int r = r0 + rr + k;
           const float w = r < rg1 ? __ldg(g.xc + r) : 0.f;
-          colacc.x = fmaf(a[k].x, w, colacc.x);
-          colacc.y = fmaf(a[k].y, w, colacc.y);
-          colacc.z = fmaf(a[k].z, w, colacc.z);
-          colacc.w = fmaf(a[k].w, w, colacc.w);
+          sum.x = fmaf(a[k].x, w, sum.x);
+          sum.y = fmaf(a[k].y, w, sum.y);
+          sum.z = fmaf(a[k].z, w, sum.z);
+          sum.w = fmaf(a[k].w, w, sum.w);
         }
+        colacc.x += sum.x, colacc.y += sum.y, colacc.z += sum.z, colacc.w += sum.w;
       }
     }
     if constexpr(NR > 0) {
       __syncthreads();
       if(warp < NR) {
-        float s = 0.f;
-#pragma unroll
-        for(int w = 0; w < kThreads / 32; ++w) s += red[warp][w][lane];
+        const float s = sum8([&](int w) { return red[warp][w][lane]; });
         const int r = r0 + lane;
         if(r < rg1) g.row_part[(int64_t(warp) * g.col_tiles + tile) * g.rows + r] = s;
       }
@@ -189,7 +198,7 @@ __device__ __forceinline__ float apply(const Term& t, float s, int i) {
 //   GESUMMV:     tmp += S0, y = alpha tmp + beta (y + S1) (row terms 0, 1)
 // W warps share 32 outputs (lane = output): warp w of them adds the partials
 // w, w + W, ..., eight loads in flight, and their sums are combined in shared
-// memory in warp order.  A CTA of 16 warps holds 16 / W such groups; the first
+// memory in pairs, in warp order.  A CTA of 16 warps holds 16 / W such groups; the first
 // row_blocks CTAs take the row outputs, the others the column outputs, each
 // with the W that final_warps gives for its number of partials.
 //
@@ -202,11 +211,11 @@ constexpr int kFinalWarps = 16, kFinalLoads = 8;
 // Groups of 32 outputs that share a CTA's warps, as CTAs.
 int64_t final_blocks(int64_t outputs, int w) { return (outputs + 32 * kFinalWarps / w - 1) / (32 * kFinalWarps / w); }
 
-// The least power of two of warps whose loads in flight cover n partials; more,
-// up to one partial each, while the outputs give fewer CTAs than the device has SMs.
+// The least power of two of warps whose loads in flight cover n partials; more
+// while the outputs give fewer CTAs than the device has SMs.
 int final_warps(int64_t outputs, int n, int sms) {
   int w = 1;
-  while(w < kFinalWarps && (n > kFinalLoads * w || (w < n && final_blocks(outputs, w) < sms))) w *= 2;
+  while(w < kFinalWarps && (n > kFinalLoads * w || final_blocks(outputs, w) < sms)) w *= 2;
   return w;
 }
 
@@ -251,8 +260,9 @@ __global__ void __launch_bounds__(32 * kFinalWarps) gemv_final_kernel(const floa
 #pragma unroll
   for(int t = 0; t < kSums; ++t) {
     if(t > 0 && !row_side) break;
-    sum[t] = 0.f;
-    for(int w = 0; w < W; ++w) sum[t] += red[t][warp + w][lane];
+    sum[t] = red[t][warp][lane];
+    if(W > 1) sum[t] += red[t][warp + 1][lane];
+    for(int w = 2; w < W; w += 2) sum[t] += red[t][warp + w][lane] + red[t][warp + w + 1][lane];
   }
   if(row_side) {
     if(NR == 0 || i >= rows) return;
@@ -375,9 +385,7 @@ __global__ void __launch_bounds__(kThreads, atax_ctas(CHUNKS)) atax_kernel(const
     __syncthreads();  // (a set is rewritten two groups later, after the next group's barrier)
 #pragma unroll
     for(int k = 0; k < R; ++k) {
-      float sum = 0.f;
-#pragma unroll
-      for(int w = 0; w < kThreads / 32; ++w) sum += red[it][w][k];
+      const float sum = sum8([&](int w) { return red[it][w][k]; });
       const float t = red[it][kThreads / 32][k] + sum;  // tmp += A x (atax.cpp:78-83); zero beyond nr
       if(tid == 0 && k < nr) tmp[r0 + k] = t;
 #pragma unroll
