@@ -15,8 +15,8 @@
 //     in flight is reduced across the warp at once (a halving transpose
 //     exchange: 16 shuffles for 16 rows), the 8 warps in shared memory per
 //     32-row block, into one partial per (column tile, row);
-//   * column sums: 4 accumulators per thread over all rows of the group, a
-//     batch of 16 (8) rows at a time, one partial per (row group, column);
+//   * column sums: 4 accumulators per thread, a batch of 16 (8) rows summed by
+//     itself and added to the group's, one partial per (row group, column);
 //   * a final kernel (1 to 16 warps per 32 outputs, by the number of partials)
 //     adds them in a fixed order and applies y = beta * y + alpha * sum
 //     (gesummv: tmp += A x, y = alpha tmp + beta (y + B x)).
