@@ -21,11 +21,12 @@
 //
 // Bound: HBM or L2, one read of the matrix (3000 x 2000: 3.5 us at the measured
 // copy rate).  Mean and standard deviation together, us, clusters / partials in
-// global memory: 100 x 100 5.0 / 6.5, 1000 x 1300 7.7 / 11.8, 3000 x 2000 12.9 /
-// 14.3, 4000 x 4000 21 / 25, 4096 x 600 10.4 / 10.4; but 10000 x 1216 22 / 18,
-// 100000 x 1300 270 / 184, 20000 x 8192 236 / 219, 2000 x 30000 105 / 88, 500 x
-// 20000 30 / 17: a cluster's eight chunks are too few CTAs for a high matrix,
-// and more than a wave of them for a wide one.
+// global memory: 100 x 100 4.8 / 5.8, 1000 x 1300 6.8 / 10.8, 3000 x 2000 11.0 /
+// 12.6, 4096 x 4096 20.0 / 22.2, 4096 x 600 9.5 / 9.7; but 100000 x 1300 260 /
+// 178, 1000000 x 500 2376 / 667, 20000 x 8192 231 / 214, 5000 x 16384 119 / 108,
+// 2000 x 30000 103 / 85: a cluster's eight chunks are too few CTAs for a high
+// matrix, and more than a wave of them for a wide one.  Between, clusters would
+// still win (8000 x 1300 15.9 / 19.1, 10000 x 1300 18.4 / 21.2).
 //
 // No kernel here triggers the next one early: CTAs of later kernels would be
 // resident, waiting, on whichever SMs had room, and a grid of a wave of CTAs
@@ -45,10 +46,12 @@ constexpr int64_t kClusterRows = 4096, kClusterCols = 4096;  // largest matrix r
 // the full batches is loaded together (TAIL: short chunks, where it is a good
 // part of the work) or row by row (long chunks: the tail's predicates cost
 // registers and with them resident CTAs; 2000 x 30000, mean and deviation, 99
-// us against 88).
+// us against 88).  Rows are unsigned: the end of a chunk and a step past the
+// last row may lie beyond 2^31 (as signed numbers 4096 x 4096, mean, 11.7 us
+// against 9.6).
 template <bool CENTERED, bool TAIL>
-__device__ __forceinline__ float column_chunk_sum(const float* __restrict__ col, int64_t ldx, int r0, int r1, int warp,
-    float m) {
+__device__ __forceinline__ float column_chunk_sum(const float* __restrict__ col, int64_t ldx, unsigned r0, unsigned r1,
+    unsigned warp, float m) {
   constexpr int kLoads = 8;
   float a[kLoads];
 #pragma unroll
@@ -61,7 +64,7 @@ __device__ __forceinline__ float column_chunk_sum(const float* __restrict__ col,
       s += x;
     }
   };
-  int r = r0 + warp;
+  unsigned r = r0 + warp;
   for(; r + (kLoads - 1) * kWarps < r1; r += kLoads * kWarps) {
     float v[kLoads];
 #pragma unroll
@@ -84,8 +87,8 @@ __device__ __forceinline__ float column_chunk_sum(const float* __restrict__ col,
 
 // The chunk's sum for column lane of the block, in every lane of warp 0 (all threads call it).
 template <bool CENTERED, bool TAIL>
-__device__ __forceinline__ float block_chunk_sum(const float* __restrict__ X, int64_t ldx, int cols, int r0, int r1, int j,
-    const float* __restrict__ mean) {
+__device__ __forceinline__ float block_chunk_sum(const float* __restrict__ X, int64_t ldx, int cols, unsigned r0, unsigned r1,
+    int j, const float* __restrict__ mean) {
   __shared__ float red[kWarps][kColsPerBlock + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float s = 0.f;
@@ -129,13 +132,15 @@ __global__ void __launch_bounds__(kWarps * 32) column_cluster_kernel(const float
 }
 
 // partial[chunk][j] = sum over the chunk's rows of X[r][j] (or (X[r][j] - mean[j])^2).
+// Eight CTAs per SM: with six (40 registers) a grid of 938 is two waves (means
+// of 2000 x 30000 56.4 us against 42.6).
 template <bool CENTERED>
-__global__ void __launch_bounds__(kWarps * 32) column_partial_kernel(const float* __restrict__ X, int64_t ldx, int rows,
-    int cols, int rows_per_chunk, const float* __restrict__ mean, float* __restrict__ partial) {
+__global__ void __launch_bounds__(kWarps * 32, 8) column_partial_kernel(const float* __restrict__ X, int64_t ldx,
+    int rows, int cols, int rows_per_chunk, const float* __restrict__ mean, float* __restrict__ partial) {
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = blockIdx.x * kColsPerBlock + lane;
-  const int r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
+  const unsigned r0 = blockIdx.y * unsigned(rows_per_chunk), r1 = min(unsigned(rows), r0 + unsigned(rows_per_chunk));
   const float t = block_chunk_sum<CENTERED, false>(X, ldx, cols, r0, r1, j, mean);
   if(warp == 0 && j < cols) partial[int64_t(blockIdx.y) * cols + j] = t;
 }
